@@ -341,8 +341,8 @@ int vfs_destroy(vfs_ctx *ctx) {
   adjoint_free(c);
   Poisson &P = c->ps;
   cudaFree(P.coef); cudaFree(P.fluid);
-  cudaFree(P.V); cudaFree(P.Z); cudaFree(P.w); cudaFree(P.r); cudaFree(P.t); cudaFree(P.hdev);
-  cudaFree(P.V32); cudaFree(P.Z32); cudaFree(P.w32);
+  cudaFree(P.V); cudaFree(P.V32); cudaFree(P.Z64); cudaFree(P.Z32); cudaFree(P.w); cudaFree(P.r); cudaFree(P.t);
+  cudaFree(P.w32);
   mg_free(P);
   if (c->ev0) cudaEventDestroy(c->ev0);
   if (c->ev1) cudaEventDestroy(c->ev1);

@@ -87,45 +87,78 @@ struct Metrics {
 // (poisson.c:951-969: CP EP WP NP SP TP BP NE SE NW SW TN BN TS BS TE BE TW BW).
 enum { CP = 0, EP, WP, NP, SP, TP, BP, NE, SE, NW, SW, TN, BN, TS, BS, TE, BE, TW, BW, NSLOT };
 
-// One multigrid level in zebra order (see vfs_mg.cu): cells ((k*ny + j)*2 + colour)*hx
-// + i/2 with colour = (i xor k) & 1, hx = ceil(nx/2), n slots in all.
+// One multigrid level in column order (see vfs_mg.cu): the cells of one (i, k) column are
+// contiguous, columns ordered ((k*2 + colour)*hx + i/2) with colour = (i xor k) & 1 and
+// hx = ceil(nx/2).  A column is solved by `ls` lanes of seg consecutive rows each and stored
+// lane-interleaved: row j sits at slot (j % seg)*ls + j/seg of the S slots of its column, so
+// that lanes reading their s-th rows read consecutive slots.  Slots past row ny-1 (and the
+// columns of an odd nx past nx-1) hold zeros; n slots in all, an even number.
 struct ZL {
   int nx, ny, nz, hx, ip, jp, kp;
+  int seg, ls, S;  // rows per lane, lanes and slots of a column
+  int lwl, lw;     // lanes of the group that solves a column: 2^lwl >= ls
+  int serial;      // columns are solved by one thread each (seg = 1)
   long long n;
+};
+__host__ __device__ inline unsigned zrow(const ZL &L, int j) {
+  return (unsigned)j % (unsigned)L.seg * (unsigned)L.ls + (unsigned)j / (unsigned)L.seg;
+}
+// Row of slot pos of a column (ny or more where it holds no cell).
+__host__ __device__ inline int zrow_of(const ZL &L, unsigned pos) {
+  const unsigned s = pos / (unsigned)L.ls;
+  return (int)((pos - s * (unsigned)L.ls) * (unsigned)L.seg + s);
+}
+// First slot of column (i, k).  32-bit index arithmetic: mg_setup refuses levels of 2^31 slots.
+__host__ __device__ inline unsigned zcol(const ZL &L, int i, int k) {
+  return (((unsigned)k * 2u + (unsigned)((i ^ k) & 1)) * (unsigned)L.hx + (unsigned)(i >> 1)) * (unsigned)L.S;
+}
+__host__ __device__ inline long long zidx(const ZL &L, int i, int j, int k) { return (long long)(zcol(L, i, k) + zrow(L, j)); }
+
+// base + (*j + off) * ldv (base when j is null): a Krylov vector whose index the device holds.
+template <typename B>
+struct DynPtrT {
+  B *base;
+  long long ldv;
+  const int *j;
+  int off;
+  __device__ __forceinline__ B *get() const { return j ? base + (long long)(*j + off) * ldv : base; }
 };
 
 struct MGLevel {
   ZL z;
   bool zebra = true;        // two-colour line Gauss-Seidel is race-free on this level
   double *op64 = nullptr;   // 6n: couplings +i, +j, +k, diagonal, Thomas factors cpr, 1/pivot
-  double *pk64 = nullptr;   // 8n: packed operator (two 4-vectors per cell), FP64
+  double *pk64 = nullptr;   // 6n: packed operator (a 4-vector and a 2-vector per cell), FP64
   float *pk32 = nullptr;    // the same in FP32
   uint8_t *act = nullptr;   // n: 1 for an active unknown (non-zero diagonal)
-  double *v64 = nullptr;    // 5n: x, b, previous x (line Jacobi), forward-elimination pairs (2n)
+  unsigned long long *pmask = nullptr;  // n: per cell of a coarse level, active neighbours and children
+  double *v64 = nullptr;    // 3n: x, b, previous x (line Jacobi)
   float *v32 = nullptr;
 };
 
 struct Poisson {
   bool built = false;
-  double *coef = nullptr;   // NSLOT * N doubles (SoA by slot)
+  double *coef = nullptr;   // NSLOT * vec_ld(N) doubles (SoA by slot)
   int nslot = NSLOT;        // 7 when every cross slot is zero (the apply reads slots 0..6)
   uint8_t *fluid = nullptr; // 1 if the cell is a Poisson unknown (gid >= 0)
   long long nfluid = 0;
   double sum_aj = 0;        // sum of aj over fluid cells (Remove_Nullspace_Scale)
   std::vector<MGLevel> lv;  // multigrid levels, finest first
-  // FGMRES workspace (grid layout, N doubles each)
-  int restart = 0;
+  // FGMRES workspace (grid layout, N entries a vector)
   long long ldv = 0;        // distance between basis vectors (N rounded up to 32)
-  double *V = nullptr;      // (restart+1) * ldv
-  double *Z = nullptr;      // restart * ldv
+  int restart = 0;          // vectors allocated of each basis form below
+  int restart32 = 0, restart_z32 = 0, restart_z64 = 0;
+  double *V = nullptr;      // (restart+1) * ldv, FP64 basis (precision 0, 1)
+  float *V32 = nullptr;     // FP32 basis (precision 2)
+  double *Z64 = nullptr;    // preconditioned vectors: the FP64 V-cycle's solutions (precision 1)
+  float *Z32 = nullptr;     // the FP32 V-cycle's solutions (precision 0, 2)
   double *w = nullptr, *r = nullptr, *t = nullptr;
-  // precision 2 (FP32 inner FGMRES): the basis, the preconditioned vectors and w in FP32
-  int restart32 = 0;
-  float *V32 = nullptr, *Z32 = nullptr, *w32 = nullptr;
-  double *hdev = nullptr;   // Gram-Schmidt coefficients on the device (64 doubles)
+  float *w32 = nullptr;     // w of precision 2
   bool transpose = false;   // apply A^T (the adjoint solve)
   bool guess = false;       // VFS_PHI holds the last solution for the current unknowns
 };
+// Distance between the vectors of a set (16-byte pair loads need it even).
+__host__ __device__ inline long long vec_ld(long long n) { return (n + 31) / 32 * 32; }
 
 // One immersed-boundary node of the IB-node list (IBMInfo, variables.h:95-172, as
 // ibm_search_advanced fills it, ibm.c:347-505): the node cell, the nearest surface
@@ -170,9 +203,9 @@ enum DScal {
 constexpr int kKryMax = 31;
 struct KryDev {
   int j, it, jdone, reorth, degen, inner_go, outer_go, conv, fresh, check, maxit, m, cycles;
+  unsigned ticket;  // blocks of the running reduction that have stored their partial sums
   double tol, bnorm, bb, r0, rnorm, rr, hn, scale;
   double inner_rtol, beta;  // precision 2: a cycle ends once its estimate is below inner_rtol * beta
-  double hdev[kKryMax + 3];
   double h[kKryMax + 3], h2[kKryMax + 3], h3[kKryMax + 3];
   double H[(kKryMax + 1) * kKryMax], cs[kKryMax], sn[kKryMax], gv[kKryMax + 1], y[kKryMax];
 };
@@ -342,12 +375,12 @@ int implicit_momentum(Ctx *c, vfs_newton_stats *st);
 int divergence_finish(Ctx *c, double *maxdiv);
 int contra2cart_div(Ctx *c, bool with_divergence);
 
-// multigrid preconditioner (vfs_mg.cu)
+// multigrid preconditioner (vfs_mg.cu): x = M^-1 b, one V-cycle on grid vectors in x's type
 int mg_setup(Ctx *c);
 void mg_free(Poisson &P);
-int mg_precondition(Ctx *c, const double *v, double *z, const vfs_solve_opts &o);
-int mg_precondition_dyn(Ctx *c, const double *V, double *Z, long long ldv, const int *jslot, const vfs_solve_opts &o);
-int mg_precondition_dyn32(Ctx *c, const float *V, float *Z, long long ldv, const int *jslot, const vfs_solve_opts &o);
+int mg_precondition(Ctx *c, DynPtrT<const double> b, DynPtrT<float> x, const vfs_solve_opts &o);
+int mg_precondition(Ctx *c, DynPtrT<const double> b, DynPtrT<double> x, const vfs_solve_opts &o);
+int mg_precondition(Ctx *c, DynPtrT<const float> b, DynPtrT<float> x, const vfs_solve_opts &o);
 int mg_sweep_fine(Ctx *c, int precision);
 
 // reductions (deterministic two-pass); result copied to host

@@ -22,11 +22,24 @@
 //     neighbour giving its weight to the parent.  With these transfers the FGMRES
 //     iteration count stays flat as the grid is refined.
 //
-// Layout: every level stores its cells in "zebra" order, ((k*ny + j)*2 + colour)*hx + i/2
-// with colour = (i xor k) & 1 and hx = ceil(nx/2), so the columns of one colour are
-// contiguous half-rows and each colour pass reads and writes with unit stride.  The
-// finest level is indexed by interior cell (DA index minus one); conversion to and from
-// the solver's DA-layout FP64 vectors happens once per V-cycle.
+// Layout: every level stores its cells column by column (struct ZL): the ny rows of an (i, k)
+// column are contiguous and lane-interleaved, the columns of one colour of a k plane are
+// neighbours.  A group of lw lanes solves a column on its own, every lane seg consecutive
+// rows in registers: all loads of a column are coalesced and in flight together, the two
+// recurrences are a warp scan each, and there is neither shared memory nor a block barrier.
+// The i/k neighbours of a row sit at the same slot of the neighbour column.  The finest level's
+// right-hand side and solution are transposed from and to the solver's grid vectors once per
+// V-cycle through shared memory.
+//
+// The FP32 V-cycle's rounding reaches the solution: a mixed solve stops at its tolerance, and
+// where the operator is nearly singular (channels without bodies) the last digits it leaves
+// (1e-8 of the pressure at rtol 1e-10) follow that rounding.  So the order of the operations
+// of a level is fixed: 32 lanes of ceil(ny/32) rows, levels of at most kSerialCells cells (and
+// coarse line Jacobi) by Thomas' recurrence row by row, no fused multiply-adds.
+//
+// One V-cycle on the B200, the tiled line sweeps with block barriers of before against the
+// columns (us, FP32 / FP64): 256 x 192 x 256 cells 1409 / 2214 -> 830 / 1481 (a colour pass of
+// the finest level 68 -> 42 FP32), 128 x 96 x 128 392 / 486 -> 197 / 297, 64^3 256 / 249 -> 119 / 127.
 //
 // A level with an odd number of cells along a periodic i or k direction cannot be two-
 // coloured; it is smoothed by damped (0.8) line Jacobi instead.
@@ -39,71 +52,50 @@ namespace vfs {
 
 enum { OP_CE = 0, OP_CN, OP_CT, OP_DG, OP_CPR, OP_IDEN, NOP };
 
-// 32-bit index arithmetic: mg_setup refuses levels of 2^31 slots or more.
-__host__ __device__ inline long long zidx(const ZL &L, int i, int j, int k) {
-  return (long long)((((unsigned)k * (unsigned)L.ny + (unsigned)j) * 2u + (unsigned)((i ^ k) & 1)) * (unsigned)L.hx +
-                     (unsigned)(i >> 1));
+// Cell (i, j, k) of slot q of a level; false for a slot that holds no cell.
+__device__ __forceinline__ bool zcell(const ZL &L, unsigned q, int &i, int &j, int &k) {
+  const unsigned col = q / (unsigned)L.S, pos = q - col * (unsigned)L.S;
+  j = zrow_of(L, pos);
+  const unsigned ck = col / (unsigned)L.hx, h = col - ck * (unsigned)L.hx;
+  k = (int)(ck >> 1);
+  i = (int)(2 * h + ((ck & 1) ^ (unsigned)(k & 1)));
+  return j < L.ny && i < L.nx;
 }
 
-// Cell (i, j, k) of a level from its natural index t = (k*ny + j)*nx + i.
-__device__ __forceinline__ void zcell(const ZL &L, long long t, int &i, int &j, int &k) {
-  const unsigned ut = (unsigned)t, nx = (unsigned)L.nx, ny = (unsigned)L.ny;
-  const unsigned r = ut / nx;
-  i = (int)(ut - r * nx);
-  const unsigned kk = r / ny;
-  j = (int)(r - kk * ny);
-  k = (int)kk;
-}
-
-// Programmatic dependent launch along the V-cycle's chain of short kernels: each kernel
-// lets its successor be scheduled as soon as all its own blocks have started, then waits
-// for its predecessor grid to complete (and its writes to be visible) before touching
-// memory, so the launch gap between kernels overlaps the tail of the previous one and
-// the results are those of plain stream order.  Outside such a launch both are no-ops.
-#ifndef VFS_PDL
-#define VFS_PDL 1
-#endif
-__device__ __forceinline__ void pdl_prologue() {
-#if VFS_PDL
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+// Programmatic dependent launch along the V-cycle's chain of short kernels: a kernel may
+// start while its predecessor drains, reads what no kernel of a solve writes (the packed
+// operator), then waits for the predecessor grid to complete (and its writes to be visible)
+// before touching any vector; only then does it let its own successor start, so at most
+// two kernels of the chain are in flight and the results are those of plain stream order.
+// Outside such a launch both are no-ops.
+__device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-#endif
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-// Inside a captured step the chain is launched plainly: captured with programmatic
-// dependent launch (VFS_PDL_CAPTURE 1) the same graph ran 0.5 ms per step slower on the B200
-// (35.9 against 36.4 ms at 256 x 192 x 256).
 #ifndef VFS_PDL_CAPTURE
-#define VFS_PDL_CAPTURE 0
+#define VFS_PDL_CAPTURE 1
 #endif
 // Every launch is counted in the context's launch counter and its status is checked: the
 // return value of cudaLaunchKernelEx, then the sticky launch error.
 template <typename... KArgs, typename... Args>
-static int launch_chain(Ctx *c, const char *what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                        Args... args) {
+static int launch_chain(Ctx *c, const char *what, void (*kernel)(KArgs...), unsigned grid, unsigned block,
+                        size_t smem, Args... args) {
   c->launches++;
-#if VFS_PDL
-  if (c->capturing && !VFS_PDL_CAPTURE) {  // plain launches inside a captured step
-    kernel<<<grid, block, smem, c->stream>>>(static_cast<KArgs>(args)...);
-    return check_launch(c, what);
-  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = c->stream;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = !c->capturing || VFS_PDL_CAPTURE ? 1 : 0;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return set_err(c, VFS_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
   }
-#else
-  kernel<<<grid, block, smem, c->stream>>>(static_cast<KArgs>(args)...);
-#endif
   return check_launch(c, what);
 }
 
@@ -112,14 +104,11 @@ static int launch_chain(Ctx *c, const char *what, void (*kernel)(KArgs...), dim3
 __global__ void k_mg_fine_couplings(Grid g, ZL L, const double *__restrict__ coef, const uint8_t *__restrict__ fluid,
                                     double *__restrict__ op) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long ncell = (long long)L.nx * L.ny * L.nz;
-  if (t >= ncell) return;
-  const int i = (int)(t % L.nx);
-  const long long r = t / L.nx;
-  const int j = (int)(r % L.ny), k = (int)(r / L.ny);
-  const long long N = g.N;
+  int i, j, k;
+  if (t >= L.n || !zcell(L, (unsigned)t, i, j, k)) return;
+  const long long N = vec_ld(g.N);
   const long long p = lidx(g, i + 1, j + 1, k + 1);
-  const long long q = zidx(L, i, j, k);
+  const long long q = t;
   double ce = 0, cn = 0, ct = 0;
   if (fluid[p]) {
     if (i + 1 < L.nx || L.ip) {
@@ -142,12 +131,9 @@ __global__ void k_mg_fine_couplings(Grid g, ZL L, const double *__restrict__ coe
 
 // Coarse couplings: 0.5 x the sum of the four fine couplings across each coarse face.
 __global__ void k_mg_coarse_couplings(ZL F, ZL C, const double *__restrict__ opF, double *__restrict__ opC) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long ncell = (long long)C.nx * C.ny * C.nz;
-  if (t >= ncell) return;
-  const int I = (int)(t % C.nx);
-  const long long r = t / C.nx;
-  const int J = (int)(r % C.ny), K = (int)(r / C.ny);
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  int I, J, K;
+  if (q >= C.n || !zcell(C, (unsigned)q, I, J, K)) return;
   double sx = 0, sy = 0, sz = 0;
   for (int u = 0; u < 2; u++)
     for (int v = 0; v < 2; v++) {
@@ -155,7 +141,6 @@ __global__ void k_mg_coarse_couplings(ZL F, ZL C, const double *__restrict__ opF
       sy += opF[OP_CN * F.n + zidx(F, 2 * I + u, 2 * J + 1, 2 * K + v)];
       sz += opF[OP_CT * F.n + zidx(F, 2 * I + u, 2 * J + v, 2 * K + 1)];
     }
-  const long long q = zidx(C, I, J, K);
   opC[OP_CE * C.n + q] = 0.5 * sx;
   opC[OP_CN * C.n + q] = 0.5 * sy;
   opC[OP_CT * C.n + q] = 0.5 * sz;
@@ -177,13 +162,9 @@ __device__ __forceinline__ ZNb znb(const ZL &L, int i, int j, int k) {
 }
 
 __global__ void k_mg_diag(ZL L, double *__restrict__ op) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long ncell = (long long)L.nx * L.ny * L.nz;
-  if (t >= ncell) return;
-  const int i = (int)(t % L.nx);
-  const long long r = t / L.nx;
-  const int j = (int)(r % L.ny), k = (int)(r / L.ny);
-  const long long q = zidx(L, i, j, k), n = L.n;
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x, n = L.n;
+  int i, j, k;
+  if (q >= n || !zcell(L, (unsigned)q, i, j, k)) return;
   const ZNb b = znb(L, i, j, k);
   double s = op[OP_CE * n + q] + op[OP_CN * n + q] + op[OP_CT * n + q];
   if (b.iw >= 0) s += op[OP_CE * n + zidx(L, b.iw, j, k)];
@@ -222,11 +203,11 @@ __global__ void k_mg_thomas(ZL L, double *__restrict__ op) {
 }
 
 // ------------------------------------------------------------------ packed operator
-// The smoother and the transfers read the operator as two 4-vectors per cell, so a
-// row costs two vector loads: cpl = {ce, cw, ct, cb} (couplings to i+1, i-1, k+1, k-1)
-// and tri = {cs, iden, cpr, dg} (coupling to j-1, Thomas pivot inverse and factor,
-// diagonal).  A missing neighbour has a zero coupling; cs at j = 0 is the periodic
-// wrap coupling when j is periodic, else 0.
+// The smoother and the transfers read the operator as a 4-vector, a 2-vector and two scalars per cell:
+// cpl = {ce, cw, ct, cb} (couplings to i+1, i-1, k+1, k-1) and tri = {cs, iden} (coupling to
+// j-1, Thomas pivot inverse), and the Thomas factor cpr and the diagonal dg apart: a smoothing
+// row reads 28 bytes of operator in FP32, and only the restriction reads the diagonal.  A missing neighbour has a zero coupling; cs at j = 0
+// is the periodic wrap coupling when j is periodic, else 0.
 template <typename T>
 struct __align__(4 * sizeof(T)) Q4 {
   T a, b, c, d;
@@ -237,479 +218,544 @@ struct __align__(2 * sizeof(T)) Q2 {
 };
 
 template <typename T>
-__global__ void k_mg_pack(ZL L, const double *__restrict__ op, Q4<T> *__restrict__ cpl, Q4<T> *__restrict__ tri) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long ncell = (long long)L.nx * L.ny * L.nz;
-  if (t >= ncell) return;
-  const int i = (int)(t % L.nx);
-  const long long r = t / L.nx;
-  const int j = (int)(r % L.ny), k = (int)(r / L.ny);
-  const long long q = zidx(L, i, j, k), n = L.n;
+__global__ void k_mg_pack(ZL L, const double *__restrict__ op, Q4<T> *__restrict__ cpl, Q2<T> *__restrict__ tri,
+                          T *__restrict__ cpr, T *__restrict__ dg) {
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x, n = L.n;
+  int i, j, k;
+  if (q >= n || !zcell(L, (unsigned)q, i, j, k)) return;
   const ZNb nb = znb(L, i, j, k);
-  Q4<T> a, b;
+  Q4<T> a;
+  Q2<T> b;
   a.a = (T)op[OP_CE * n + q];
   a.b = nb.iw >= 0 ? (T)op[OP_CE * n + zidx(L, nb.iw, j, k)] : T(0);
   a.c = (T)op[OP_CT * n + q];
   a.d = nb.kb >= 0 ? (T)op[OP_CT * n + zidx(L, i, j, nb.kb)] : T(0);
   b.a = nb.js >= 0 ? (T)op[OP_CN * n + zidx(L, i, nb.js, k)] : T(0);
   b.b = (T)op[OP_IDEN * n + q];
-  b.c = (T)op[OP_CPR * n + q];
-  b.d = (T)op[OP_DG * n + q];
   cpl[q] = a;
   tri[q] = b;
+  cpr[q] = (T)op[OP_CPR * n + q];
+  dg[q] = (T)op[OP_DG * n + q];
+}
+
+// act[q] = 1 where the level's diagonal is non-zero (an active unknown).
+__global__ void k_mg_active(long long n, const double *__restrict__ op, uint8_t *__restrict__ act) {
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (q < n) act[q] = op[OP_DG * n + q] != 0.0 ? 1 : 0;
+}
+
+// Coarse cell q: bit e (0..26) set where the cell of its 3 x 3 x 3 neighbourhood at
+// (e%3-1, e/3%3-1, e/9-1) exists and is active, bit 27 + ch where its child ch (bits i, j, k) is.
+__device__ __forceinline__ int wrap_or_none(int v, int n, int per) { return (v >= 0 && v < n) ? v : (per ? (v + n) % n : -1); }
+__global__ void k_mg_pmask(ZL F, ZL C, const uint8_t *__restrict__ actF, const uint8_t *__restrict__ actC,
+                           unsigned long long *__restrict__ mask) {
+  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  int I, J, K;
+  if (q >= C.n || !zcell(C, (unsigned)q, I, J, K)) return;
+  unsigned long long m = 0;
+  for (int e = 0; e < 27; e++) {
+    const int i = wrap_or_none(I + e % 3 - 1, C.nx, C.ip), j = wrap_or_none(J + e / 3 % 3 - 1, C.ny, C.jp);
+    const int k = wrap_or_none(K + e / 9 - 1, C.nz, C.kp);
+    if (i >= 0 && j >= 0 && k >= 0 && actC[zidx(C, i, j, k)]) m |= 1ull << e;
+  }
+  for (int ch = 0; ch < 8; ch++)
+    if (actF[zidx(F, 2 * I + (ch & 1), 2 * J + ((ch >> 1) & 1), 2 * K + (ch >> 2))]) m |= 1ull << (27 + ch);
+  mask[q] = m;
 }
 
 // ------------------------------------------------------------------ smoother
-// One colour pass of zebra line Gauss-Seidel (colour 0/1; x read for the other colour,
-// written for this one), or, with colour < 0, one damped line-Jacobi sweep over all
-// columns (neighbours read from xr = the previous iterate, a separate array).
-// x_zero: the neighbours read are known to be zero (first pass from a zero guess).
-// The forward elimination stores (d'_j, cpr_j) in ds; the back substitution writes x.
-// Rows are processed in chunks of CH: every load of a chunk is issued before the
-// recurrence consumes the first one, so a column keeps CH rows of loads in flight.
-template <typename T, int CH>
-__device__ __forceinline__ void zline_column(const ZL &L, const Q4<T> *__restrict__ cpl, const Q4<T> *__restrict__ tri,
-                                             const T *__restrict__ b, const T *__restrict__ xr,
-                                             Q2<T> *__restrict__ ds, T *__restrict__ xw, int colour, T omega,
-                                             int x_zero, long long t) {
-  const int hx = L.hx;
-  int c, h, k;
-  if (colour >= 0) {
-    if (t >= (long long)L.nz * hx) return;
-    h = (int)(t % hx); k = (int)(t / hx); c = colour;
-  } else {
-    if (t >= 2LL * L.nz * hx) return;
-    h = (int)(t % hx); c = (int)((t / hx) & 1); k = (int)(t / (2LL * hx));
+template <typename T>
+__device__ __forceinline__ void scan_compose_up(T &A, T &B, int l, int lw) {
+  // inclusive scan over lanes 0..l of a group of x -> A x + B maps (later lanes applied last)
+#pragma unroll
+  for (int off = 1; off < lw; off <<= 1) {
+    const T pa = __shfl_up_sync(0xffffffffu, A, off, lw), pb = __shfl_up_sync(0xffffffffu, B, off, lw);
+    if (l >= off) { B = A * pb + B; A = A * pa; }
   }
-  const int i = 2 * h + (c ^ (k & 1));
-  if (i >= L.nx) return;
-  const ZNb nb = znb(L, i, 0, k);
-  const long long p0 = zidx(L, i, 0, k);
-  // offsets of the neighbour columns (constant along j).  A missing neighbour (domain
-  // edge, zero coupling) borrows the offset of the opposite one, so every x read is of
-  // the other colour (every level has at least 2 cells along i and k).
-  const long long oe = zidx(L, nb.ie >= 0 ? nb.ie : nb.iw, 0, k) - p0;
-  const long long ow = zidx(L, nb.iw >= 0 ? nb.iw : nb.ie, 0, k) - p0;
-  const long long ot = zidx(L, i, 0, nb.kt >= 0 ? nb.kt : nb.kb) - p0;
-  const long long ob = zidx(L, i, 0, nb.kb >= 0 ? nb.kb : nb.kt) - p0;
-  const long long sj = 2LL * hx;
-  const int ny = L.ny;
-  // periodic j: the wrap coupling and the far end of the own column (old values)
-  T wrap_c = 0, x_first = 0, x_last = 0;
-  if (L.jp && !x_zero) {
-    const T *__restrict__ xs = colour >= 0 ? xw : xr;
-    wrap_c = tri[p0].a;
-    x_first = xs[p0];
-    x_last = xs[p0 + (ny - 1) * sj];
+}
+template <typename T>
+__device__ __forceinline__ void scan_compose_down(T &A, T &B, int l, int lw) {
+  // inclusive scan over lanes l..lw-1 (higher lanes applied first)
+#pragma unroll
+  for (int off = 1; off < lw; off <<= 1) {
+    const T pa = __shfl_down_sync(0xffffffffu, A, off, lw), pb = __shfl_down_sync(0xffffffffu, B, off, lw);
+    if (l + off < lw) { B = A * pb + B; A = A * pa; }
   }
-  T dprev = 0;
+}
+
+// What a pass over the columns of one colour (or, line Jacobi, of both) may assume of x:
+enum { Z_NB_ZERO = 1, Z_OWN_ZERO = 2 };  // the neighbour columns / the own column are zero
+
+// Column t of a pass (colour 0/1: the columns of that colour; < 0: all): its first slot and
+// the slot offsets of its four neighbour columns.  A missing neighbour (domain edge, zero
+// coupling) borrows the opposite one's column, so every x read is of the other colour
+// (every level has at least 2 cells along i and k).
+struct ZCol {
+  unsigned p0;
+  int oe, ow, ot, ob;
+  bool valid;
+};
+__device__ __forceinline__ unsigned zpass_columns(const ZL &L, int colour) {
+  return (unsigned)L.nz * (unsigned)L.hx * (colour >= 0 ? 1u : 2u);
+}
+__device__ __forceinline__ ZCol zcolumn(const ZL &L, int colour, unsigned t) {
+  ZCol r;
+  const unsigned hx = (unsigned)L.hx;
+  r.valid = t < zpass_columns(L, colour);
+  if (!r.valid) t = 0;  // a real column for the addresses; nothing is stored
+  unsigned k = t / hx;
+  const unsigned h = t - k * hx;
+  unsigned c = (unsigned)colour;
+  if (colour < 0) { c = k & 1; k >>= 1; }
+  int i = (int)(2 * h + (c ^ (k & 1)));
+  if (i >= L.nx) { r.valid = false; i -= 2; }
+  const int kk = (int)k;
+  r.p0 = zcol(L, i, kk);
+  int ie = i + 1 < L.nx ? i + 1 : (L.ip ? 0 : -1), iw = i > 0 ? i - 1 : (L.ip ? L.nx - 1 : -1);
+  int kt = kk + 1 < L.nz ? kk + 1 : (L.kp ? 0 : -1), kb = kk > 0 ? kk - 1 : (L.kp ? L.nz - 1 : -1);
+  if (ie < 0) ie = iw;
+  if (iw < 0) iw = ie;
+  if (kt < 0) kt = kb;
+  if (kb < 0) kb = kt;
+  r.oe = (int)(zcol(L, ie, kk) - r.p0);
+  r.ow = (int)(zcol(L, iw, kk) - r.p0);
+  r.ot = (int)(zcol(L, i, kt) - r.p0);
+  r.ob = (int)(zcol(L, i, kb) - r.p0);
+  return r;
+}
+
+// The operator rows of a lane: SEG rows from slot q0, ls apart; none (zeros) for a lane past ls.
+template <typename T, int SEG>
+struct ZRows {
+  Q4<T> cp[SEG];
+  Q2<T> tr[SEG];
+  T cx[SEG];
+};
+template <typename T, int SEG, bool kFull>
+__device__ __forceinline__ void zload(const ZL &L, const Q4<T> *__restrict__ cpl, const Q2<T> *__restrict__ tri,
+                                      const T *__restrict__ cpr, unsigned p0, int l, int flags, ZRows<T, SEG> &R) {
+  const int ls = kFull ? 32 : L.ls;
+  if (!kFull && l >= ls) {
+#pragma unroll
+    for (int s = 0; s < SEG; s++) {
+      R.tr[s] = Q2<T>{T(0), T(0)};
+      R.cx[s] = T(0);
+    }
+    return;
+  }
+#pragma unroll
+  for (int s = 0; s < SEG; s++) {
+    const unsigned q = p0 + (unsigned)(l + s * ls);
+    R.tr[s] = tri[q];
+    R.cx[s] = cpr[q];
+    if (!(flags & Z_NB_ZERO)) R.cp[s] = cpl[q];
+  }
+}
+
+// Solves one column (SEG rows in each of the ls lanes of a group of lw): right-hand side b
+// minus the couplings to the neighbour columns in xr, the forward elimination
+// d_j = r_j / pivot - (cs_j / pivot) d_{j-1} and the back substitution
+// x_j = d_j - cpr_j x_{j+1} as first-order linear recurrences: each lane composes its rows,
+// a shuffle scan combines the lanes, each lane then replays its rows.  Every lane of the
+// warp takes part; `omega` is used by line Jacobi only (kJac: xr is the previous iterate);
+// kFull: all 32 lanes hold rows (ls = 32).
+template <typename T, int SEG, bool kJac, bool kFull>
+__device__ __forceinline__ void zsolve(const ZL &L, const ZCol &z, int l, const ZRows<T, SEG> &R, const T *b,
+                                       const T *xr, T *xw, int flags, T omega) {
+  const unsigned q0 = z.p0 + (unsigned)l;
+  const int ls = kFull ? 32 : L.ls, lw = kFull ? 32 : L.lw;
+  const bool own = kFull || l < ls;
+  T r[SEG], m[SEG];
+#pragma unroll
+  for (int s = 0; s < SEG; s++) r[s] = own ? b[q0 + (unsigned)(s * ls)] : T(0);
+  if (!(flags & Z_NB_ZERO) && own) {
+    T xe[SEG], xv[SEG], xt[SEG], xb[SEG];
+#pragma unroll
+    for (int s = 0; s < SEG; s++) {
+      const int q = (int)(q0 + (unsigned)(s * ls));
+      xe[s] = xr[(unsigned)(q + z.oe)];
+      xv[s] = xr[(unsigned)(q + z.ow)];
+      xt[s] = xr[(unsigned)(q + z.ot)];
+      xb[s] = xr[(unsigned)(q + z.ob)];
+    }
+#pragma unroll
+    for (int s = 0; s < SEG; s++) {
+      r[s] -= R.cp[s].a * xe[s];
+      r[s] -= R.cp[s].b * xv[s];
+      r[s] -= R.cp[s].c * xt[s];
+      r[s] -= R.cp[s].d * xb[s];
+    }
+  }
+  if (L.jp && !(flags & Z_OWN_ZERO)) {
+    // periodic j: the wrap coupling (cs of row 0) and the far end of the own column (old values)
+    const T wrap = __shfl_sync(0xffffffffu, R.tr[0].a, 0, lw);
+    const T first = xr[z.p0], last = xr[z.p0 + zrow(L, L.ny - 1)];
+#pragma unroll
+    for (int s = 0; s < SEG; s++) {
+      const int j = l * SEG + s;
+      if (j == 0) r[s] -= wrap * last;
+      if (j == L.ny - 1) r[s] -= wrap * first;
+    }
+  }
+#pragma unroll
+  for (int s = 0; s < SEG; s++) {
+    r[s] *= R.tr[s].b;
+    m[s] = R.tr[s].a * R.tr[s].b;
+  }
+  if (l == 0) m[0] = 0;
+  T A = 1, B = 0;
+#pragma unroll
+  for (int s = 0; s < SEG; s++) { B = -m[s] * B + r[s]; A = -m[s] * A; }
+  scan_compose_up<T>(A, B, l, lw);
+  T d = __shfl_up_sync(0xffffffffu, B, 1, lw);
+  if (l == 0) d = 0;
+#pragma unroll
+  for (int s = 0; s < SEG; s++) { d = -m[s] * d + r[s]; r[s] = d; }
+  A = 1; B = 0;
+#pragma unroll
+  for (int s = SEG - 1; s >= 0; s--) { B = -R.cx[s] * B + r[s]; A = -R.cx[s] * A; }
+  scan_compose_down<T>(A, B, l, lw);
+  T x = __shfl_down_sync(0xffffffffu, B, 1, lw);
+  if (l == lw - 1) x = 0;
+#pragma unroll
+  for (int s = SEG - 1; s >= 0; s--) { x = -R.cx[s] * x + r[s]; r[s] = x; }
+  if (!z.valid || !own) return;
+#pragma unroll
+  for (int s = 0; s < SEG; s++) {
+    const unsigned q = q0 + (unsigned)(s * ls);
+    if (kJac) {
+      const T xo = (flags & Z_OWN_ZERO) ? T(0) : xr[q];
+      xw[q] = xo + omega * (r[s] - xo);
+    } else {
+      xw[q] = r[s];
+    }
+  }
+}
+
+// The same for columns of more rows per lane than the register forms take: the rows are
+// replayed through the column's own slots of xw, which no other column of the pass reads.
+template <typename T, bool kJac>
+__device__ void zsolve_long(const ZL &L, const ZCol &z, int l, const Q4<T> *__restrict__ cpl,
+                            const Q2<T> *__restrict__ tri, const T *__restrict__ cpr, const T *b, const T *xr, T *xw,
+                            int flags, T omega) {
+  const unsigned q0 = z.p0 + (unsigned)l;
+  const int seg = l < L.ls ? L.seg : 0;
+  const bool st = z.valid;
+  T wrap = 0, first = 0, last = 0;
+  if (L.jp && !(flags & Z_OWN_ZERO)) {
+    wrap = tri[z.p0].a;
+    first = xr[z.p0];
+    last = xr[z.p0 + zrow(L, L.ny - 1)];
+  }
+  __syncwarp();
+  T A = 1, B = 0;
+  for (int s = 0; s < seg; s++) {
+    const unsigned q = q0 + (unsigned)(s * L.ls);
+    const Q2<T> t = tri[q];
+    T r = b[q];
+    if (!(flags & Z_NB_ZERO)) {
+      const Q4<T> c = cpl[q];
+      r -= c.a * xr[(unsigned)((int)q + z.oe)];
+      r -= c.b * xr[(unsigned)((int)q + z.ow)];
+      r -= c.c * xr[(unsigned)((int)q + z.ot)];
+      r -= c.d * xr[(unsigned)((int)q + z.ob)];
+    }
+    const int j = l * seg + s;
+    if (j == 0) r -= wrap * last;
+    if (j == L.ny - 1) r -= wrap * first;
+    r *= t.b;
+    const T m = j > 0 ? t.a * t.b : T(0);
+    if (st) xw[q] = r;
+    B = -m * B + r;
+    A = -m * A;
+  }
+  scan_compose_up<T>(A, B, l, L.lw);
+  T d = __shfl_up_sync(0xffffffffu, B, 1, L.lw);
+  if (l == 0) d = 0;
+  for (int s = 0; s < seg; s++) {
+    const unsigned q = q0 + (unsigned)(s * L.ls);
+    const Q2<T> t = tri[q];
+    const T m = l * seg + s > 0 ? t.a * t.b : T(0);
+    d = -m * d + xw[q];
+    if (st) xw[q] = d;
+  }
+  A = 1; B = 0;
+  for (int s = seg - 1; s >= 0; s--) {
+    const unsigned q = q0 + (unsigned)(s * L.ls);
+    const T c = cpr[q];
+    B = -c * B + xw[q];
+    A = -c * A;
+  }
+  scan_compose_down<T>(A, B, l, L.lw);
+  T x = __shfl_down_sync(0xffffffffu, B, 1, L.lw);
+  if (l == L.lw - 1) x = 0;
+  for (int s = seg - 1; s >= 0; s--) {
+    const unsigned q = q0 + (unsigned)(s * L.ls);
+    x = -cpr[q] * x + xw[q];
+    if (st) {
+      if (kJac) {
+        const T xo = (flags & Z_OWN_ZERO) ? T(0) : xr[q];
+        xw[q] = xo + omega * (x - xo);
+      } else {
+        xw[q] = x;
+      }
+    }
+  }
+}
+
+// Thomas' recurrence of one column by one thread, row by row: r the right-hand sides on entry
+// and the solution on exit, lo the lower couplings (0 at row 0), id the pivots' inverses, cx
+// the forward factors.  Four rows' loads are in flight at a time.
+template <typename T>
+__device__ __forceinline__ void thomas_rows(T *r, const T *lo, const T *id, const T *cx, int ny) {
+  constexpr int CH = 4;
+  T d = 0;
   for (int j0 = 0; j0 < ny; j0 += CH) {
-    T bb[CH], xe[CH], xwv[CH], xt[CH], xb[CH];
-    Q4<T> cp[CH], tr[CH];
+    T rr[CH], ll[CH], ii[CH];
 #pragma unroll
     for (int u = 0; u < CH; u++) {
-      const int j = j0 + u;
-      if (j < ny) {
-        const long long q = p0 + j * sj;
-        bb[u] = b[q];
-        tr[u] = tri[q];
-        if (!x_zero) {
-          cp[u] = cpl[q];
-          xe[u] = xr[q + oe];
-          xwv[u] = xr[q + ow];
-          xt[u] = xr[q + ot];
-          xb[u] = xr[q + ob];
-        }
-      }
+      const int j = min(j0 + u, ny - 1);
+      rr[u] = r[j]; ll[u] = lo[j]; ii[u] = id[j];
     }
 #pragma unroll
     for (int u = 0; u < CH; u++) {
-      const int j = j0 + u;
-      if (j < ny) {
-        T r = bb[u];
-        if (!x_zero) {
-          r -= cp[u].a * xe[u];
-          r -= cp[u].b * xwv[u];
-          r -= cp[u].c * xt[u];
-          r -= cp[u].d * xb[u];
-          if (L.jp) {
-            if (j == 0) r -= wrap_c * x_last;
-            if (j == ny - 1) r -= wrap_c * x_first;
-          }
-        }
-        const T lower = j > 0 ? tr[u].a : T(0);
-        const T d = (r - lower * dprev) * tr[u].b;
-        Q2<T> o;
-        o.a = d; o.b = tr[u].c;
-        ds[p0 + j * sj] = o;
-        dprev = d;
-      }
+      if (j0 + u >= ny) break;
+      d = (rr[u] - ll[u] * d) * ii[u];
+      r[j0 + u] = d;
     }
   }
-  T xnext = 0;
+  T x = 0;
   for (int j1 = ny - 1; j1 >= 0; j1 -= CH) {
-    Q2<T> dd[CH];
-    T xo[CH];
+    T dd[CH], cc[CH];
 #pragma unroll
     for (int u = 0; u < CH; u++) {
-      const int j = j1 - u;
-      if (j >= 0) {
-        dd[u] = ds[p0 + j * sj];
-        if (colour < 0 && !x_zero) xo[u] = xr[p0 + j * sj];
-      }
+      const int j = max(j1 - u, 0);
+      dd[u] = r[j]; cc[u] = cx[j];
     }
 #pragma unroll
     for (int u = 0; u < CH; u++) {
-      const int j = j1 - u;
-      if (j >= 0) {
-        const T v = dd[u].a - dd[u].b * xnext;
-        xnext = v;
-        T out = v;
-        if (colour < 0) out = x_zero ? omega * v : xo[u] + omega * (v - xo[u]);
-        xw[p0 + j * sj] = out;
-      }
+      if (j1 - u < 0) break;
+      x = dd[u] - cc[u] * x;
+      r[j1 - u] = x;
     }
   }
 }
 
-template <typename T> struct ZChunk;
-template <> struct ZChunk<float> { static constexpr int v = 8; };
-template <> struct ZChunk<double> { static constexpr int v = 4; };
-
+// One pass over the columns of one colour.  Bound by the bytes of a row (FP32:
+// operator 28, b 4, the other colour's x 4, x 4); registers set the occupancy.  SEG = 0: columns
+// of more than eight rows a lane.
+template <typename T> struct ZBounds;
+#ifndef VFS_ZCOL_MINB32
+#define VFS_ZCOL_MINB32 5
+#endif
+#ifndef VFS_ZCOL_MINB64
+#define VFS_ZCOL_MINB64 3
+#endif
+template <> struct ZBounds<float> { static constexpr int v = VFS_ZCOL_MINB32; };
+template <> struct ZBounds<double> { static constexpr int v = VFS_ZCOL_MINB64; };
+constexpr int kColThreads = 128;
 template <typename T>
-__global__ void __launch_bounds__(64) k_zline(ZL L, const Q4<T> *__restrict__ cpl, const Q4<T> *__restrict__ tri,
-                                              const T *__restrict__ b, const T *__restrict__ xr,
-                                              Q2<T> *__restrict__ ds, T *__restrict__ xw, int colour, T omega,
-                                              int x_zero) {
-  zline_column<T, ZChunk<T>::v>(L, cpl, tri, b, xr, ds, xw, colour, omega, x_zero,
-                                blockIdx.x * (long long)blockDim.x + threadIdx.x);
-}
-
-// Tiled zebra colour pass for the large levels.  One thread block owns W columns of
-// one colour that are consecutive in memory (same k, half-row positions h0..h0+W-1):
-//   A. all threads load the tile's rows (coalesced across the W columns, many loads in
-//      flight) and form each row's scaled right-hand side r' = r / pivot, the scaled
-//      lower coupling m = lower / pivot and the Thomas factor cpr, in shared memory;
-//   B. each warp solves whole columns: the forward elimination d_j = r'_j - m_j d_{j-1}
-//      and the back substitution x_j = d_j - cpr_j x_{j+1} are first-order linear
-//      recurrences, evaluated as warp scans (each lane composes its run of rows, a
-//      5-step shuffle scan combines the lanes, each lane then replays its rows);
-//   C. all threads write the tile's x back, coalesced.
-// Shared memory: 3 * W * P values of T, P = ny rounded up to odd (conflict-free rows).
-#ifndef VFS_ZTILE_THREADS
-#define VFS_ZTILE_THREADS 256
-#endif
-#ifndef VFS_ZTILE_W32
-#define VFS_ZTILE_W32 16   // columns per tile, FP32
-#endif
-#ifndef VFS_ZTILE_W64
-#define VFS_ZTILE_W64 8    // columns per tile, FP64
-#endif
-#ifndef VFS_ZTILE_U32
-#define VFS_ZTILE_U32 1    // rows each thread loads before using them, FP32
-#endif
-// Measured at 256 x 192 x 256 (V-cycle ms, FP32 / FP64): FP32 rows per thread 1 1.42,
-// 2 1.46, 4 1.78; FP32 columns 8 1.45, 16 1.46, 32 2.02; FP32 blocks per SM 3 1.62, 4 1.48,
-// 5 1.46, 6 1.77; FP64 columns 8 2.20, 16 2.27, 32 2.75.
-#ifndef VFS_ZTILE_MINB
-#define VFS_ZTILE_MINB 5   // resident blocks per SM the register allocation must allow, FP32
-#endif
-#ifndef VFS_ZTILE_MINB64
-#define VFS_ZTILE_MINB64 1  // the same, FP64
-#endif
-constexpr int kTileThreads = VFS_ZTILE_THREADS;
-
-template <typename T>
-__device__ __forceinline__ void scan_compose_up(T &A, T &B, int lane) {
-  // inclusive scan over lanes 0..lane of x -> A x + B maps (later lanes applied last)
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const T pa = __shfl_up_sync(0xffffffffu, A, off), pb = __shfl_up_sync(0xffffffffu, B, off);
-    if (lane >= off) { B = A * pb + B; A = A * pa; }
-  }
-}
-template <typename T>
-__device__ __forceinline__ void scan_compose_down(T &A, T &B, int lane) {
-  // inclusive scan over lanes lane..31 (higher lanes applied first)
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const T pa = __shfl_down_sync(0xffffffffu, A, off), pb = __shfl_down_sync(0xffffffffu, B, off);
-    if (lane + off < 32) { B = A * pb + B; A = A * pa; }
+struct ZOp {
+  const Q4<T> *cpl;
+  const Q2<T> *tri;
+  const T *cpr;
+};
+template <typename T, int SEG, bool kFull>
+__global__ void __launch_bounds__(kColThreads, ZBounds<T>::v) k_zcol(ZL L, ZOp<T> op, const T *b, T *x, int colour,
+                                                                     int flags) {
+  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int lw = kFull ? 32 : L.lw, l = (int)(tid & (unsigned)(lw - 1));
+  const ZCol z = zcolumn(L, colour, kFull ? tid >> 5 : tid >> L.lwl);
+  if constexpr (SEG > 0) {
+    ZRows<T, SEG> R;
+    zload<T, SEG, kFull>(L, op.cpl, op.tri, op.cpr, z.p0, l, flags, R);
+    pdl_wait();
+    zsolve<T, SEG, false, kFull>(L, z, l, R, b, x, x, flags, T(1));
+  } else {
+    pdl_wait();
+    zsolve_long<T, false>(L, z, l, op.cpl, op.tri, op.cpr, b, x, x, flags, T(1));
   }
 }
 
-template <typename T, int W>
-__global__ void __launch_bounds__(kTileThreads, sizeof(T) == 4 ? VFS_ZTILE_MINB : VFS_ZTILE_MINB64) k_zline_tile(ZL L, const Q4<T> *__restrict__ cpl,
-                                                             const Q4<T> *__restrict__ tri, const T *__restrict__ b,
-                                                             const T *__restrict__ xr, T *__restrict__ xw, int colour,
-                                                             int x_zero) {
-  pdl_prologue();
-  extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int hx = L.hx, ny = L.ny;
-  const int P = ny | 1;
-  T *sr = reinterpret_cast<T *>(smem_raw);  // [W][P]: r', then d, then x
-  T *sm = sr + W * P;                        // [W][P]: m
-  T *sc = sm + W * P;                        // [W][P]: cpr
-  const int tiles_per_row = (hx + W - 1) / W;
-  const int k = blockIdx.x / tiles_per_row;
-  const int h0 = (blockIdx.x % tiles_per_row) * W;
-  if (k >= L.nz) return;
-  const long long sj = 2LL * hx;
-  // A: the block size is a multiple of W, so each thread keeps one column and takes
-  // every (blockDim/W)-th row; U rows are loaded before any of them is used.
-  {
-    constexpr int U = sizeof(T) == 4 ? VFS_ZTILE_U32 : 3;
-    const int w = threadIdx.x % W, jstep = blockDim.x / W;
-    const int h = h0 + w;
-    const int i = 2 * h + (colour ^ (k & 1));
-    const bool valid = h < hx && i < L.nx;
-    const int ic = valid ? i : (colour ^ (k & 1));  // a real column for the address arithmetic
-    const ZNb nb = znb(L, ic, 0, k);
-    const long long p0 = zidx(L, ic, 0, k);
-    const long long oe = zidx(L, nb.ie >= 0 ? nb.ie : nb.iw, 0, k) - p0;
-    const long long ow = zidx(L, nb.iw >= 0 ? nb.iw : nb.ie, 0, k) - p0;
-    const long long ot = zidx(L, ic, 0, nb.kt >= 0 ? nb.kt : nb.kb) - p0;
-    const long long ob = zidx(L, ic, 0, nb.kb >= 0 ? nb.kb : nb.kt) - p0;
-    for (int jb = threadIdx.x / W; jb < ny; jb += U * jstep) {
-      T bb[U], xe[U], xwv[U], xt[U], xb[U];
-      Q4<T> tr[U], cp[U];
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int j = jb + u * jstep;
-        if (valid && j < ny) {
-          const long long q = p0 + j * sj;
-          bb[u] = b[q];
-          tr[u] = tri[q];
-          if (!x_zero) {
-            cp[u] = cpl[q];
-            xe[u] = xr[q + oe];
-            xwv[u] = xr[q + ow];
-            xt[u] = xr[q + ot];
-            xb[u] = xr[q + ob];
-          }
-        }
+// A pass over columns too long for the kernel below, by lane groups.
+template <typename T, bool kJac>
+__global__ void __launch_bounds__(kColThreads) k_zlong(ZL L, ZOp<T> op, const T *b, const T *xr, T *xw, int colour,
+                                                       int flags, T omega) {
+  const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
+  pdl_wait();
+  zsolve_long<T, kJac>(L, zcolumn(L, colour, tid >> L.lwl), (int)(tid & (unsigned)(L.lw - 1)), op.cpl, op.tri, op.cpr, b, xr, xw, flags, omega);
+}
+
+// One pass by Thomas' recurrence row by row (small levels, and every line Jacobi sweep: kJac,
+// colour < 0, xr the previous iterate): a block stages the rows of kSerialCols columns in
+// shared memory with coalesced loads, one thread a column solves there, and all write back.
+// (One thread a column straight from global memory took 22 us a pass on 45 x 37 x 53 cells.)
+constexpr int kSerialCols = 16, kSerialThreads = 32 * kSerialCols;
+template <typename T>
+static size_t serial_smem(const ZL &L) { return sizeof(T) * 4 * kSerialCols * ((size_t)L.ny | 1); }
+constexpr size_t kSerialSmem = 200 * 1024;
+template <typename T, bool kJac>
+__global__ void __launch_bounds__(kSerialThreads) k_zserial(ZL L, ZOp<T> op, const T *b, const T *xr, T *xw, int colour,
+                                                            int flags, T omega) {
+  extern __shared__ __align__(16) unsigned char ser_raw[];
+  const int ny = L.ny, ld = ny | 1;
+  T *sr = reinterpret_cast<T *>(ser_raw), *slo = sr + kSerialCols * ld, *sid = slo + kSerialCols * ld,
+    *scx = sid + kSerialCols * ld;
+  const unsigned t0 = blockIdx.x * kSerialCols;
+  const int lane = threadIdx.x & 31, c = threadIdx.x >> 5;  // a warp loads and stores a column
+  const ZCol z = zcolumn(L, colour, t0 + (unsigned)c);
+  pdl_wait();
+  if (z.valid) {
+    T wrap = 0, first = 0, last = 0;
+    if (L.jp && !(flags & Z_OWN_ZERO)) {
+      wrap = op.tri[z.p0].a;
+      first = xr[z.p0];
+      last = xr[z.p0 + zrow(L, ny - 1)];
+    }
+#pragma unroll 2
+    for (int s = lane; s < L.S; s += 32) {
+      const int j = zrow_of(L, (unsigned)s);
+      if (j >= ny) continue;
+      const unsigned q = z.p0 + (unsigned)s;
+      T r = b[q];
+      const Q2<T> t = op.tri[q];
+      if (!(flags & Z_NB_ZERO)) {
+        const Q4<T> cp = op.cpl[q];
+        r -= cp.a * xr[(unsigned)((int)q + z.oe)];
+        r -= cp.b * xr[(unsigned)((int)q + z.ow)];
+        r -= cp.c * xr[(unsigned)((int)q + z.ot)];
+        r -= cp.d * xr[(unsigned)((int)q + z.ob)];
       }
-#pragma unroll
-      for (int u = 0; u < U; u++) {
-        const int j = jb + u * jstep;
-        if (j >= ny) continue;
-        T rr = 0, mm = 0, cc = 0;
-        if (valid) {
-          T r = bb[u];
-          if (!x_zero) {
-            // a missing neighbour has a zero coupling (its offset is the opposite one's)
-            r -= cp[u].a * xe[u];
-            r -= cp[u].b * xwv[u];
-            r -= cp[u].c * xt[u];
-            r -= cp[u].d * xb[u];
-            if (L.jp) {
-              if (j == 0) r -= tr[u].a * xw[p0 + (ny - 1) * sj];
-              if (j == ny - 1) r -= tri[p0].a * xw[p0];
-            }
-          }
-          rr = r * tr[u].b;
-          mm = j > 0 ? tr[u].a * tr[u].b : T(0);
-          cc = tr[u].c;
-        }
-        sr[w * P + j] = rr;
-        sm[w * P + j] = mm;
-        sc[w * P + j] = cc;
-      }
+      if (j == 0) r -= wrap * last;
+      if (j == ny - 1) r -= wrap * first;
+      sr[c * ld + j] = r;
+      slo[c * ld + j] = j > 0 ? t.a : T(0);
+      sid[c * ld + j] = t.b;
+      scx[c * ld + j] = op.cpr[q];
     }
   }
   __syncthreads();
-  // B
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-  const int seg = (ny + 31) >> 5;
-  const int j0 = lane * seg, j1 = min(ny, j0 + seg);
-  for (int w = warp; w < W; w += nwarp) {
-    T *cr = sr + w * P;
-    const T *cm = sm + w * P, *cx = sc + w * P;
-    // forward: d_j = -m_j d_{j-1} + r'_j
-    T A = 1, B = 0;
-    for (int j = j0; j < j1; j++) { const T mj = cm[j]; B = -mj * B + cr[j]; A = -mj * A; }
-    scan_compose_up<T>(A, B, lane);
-    T d = __shfl_up_sync(0xffffffffu, B, 1);
-    if (lane == 0) d = 0;
-    for (int j = j0; j < j1; j++) { d = -cm[j] * d + cr[j]; cr[j] = d; }
-    __syncwarp();
-    // backward: x_j = -cpr_j x_{j+1} + d_j
-    A = 1; B = 0;
-    for (int j = j1 - 1; j >= j0; j--) { const T cj = cx[j]; B = -cj * B + cr[j]; A = -cj * A; }
-    scan_compose_down<T>(A, B, lane);
-    T x = __shfl_down_sync(0xffffffffu, B, 1);
-    if (lane == 31) x = 0;
-    for (int j = j1 - 1; j >= j0; j--) { x = -cx[j] * x + cr[j]; cr[j] = x; }
-    __syncwarp();
+  if (threadIdx.x < kSerialCols && zcolumn(L, colour, t0 + threadIdx.x).valid) {
+    T *r = sr + threadIdx.x * ld;
+    const T *lo = slo + threadIdx.x * ld, *id = sid + threadIdx.x * ld, *cx = scx + threadIdx.x * ld;
+    thomas_rows<T>(r, lo, id, cx, ny);
   }
   __syncthreads();
-  // C
-  for (int e = threadIdx.x; e < ny * W; e += blockDim.x) {
-    const int j = e / W, w = e - (e / W) * W;
-    const int h = h0 + w;
-    const int i = 2 * h + (colour ^ (k & 1));
-    if (h < hx && i < L.nx) xw[zidx(L, i, j, k)] = sr[w * P + j];
+  if (!z.valid) return;
+  for (int s = lane; s < L.S; s += 32) {
+    const int j = zrow_of(L, (unsigned)s);
+    if (j >= ny) continue;
+    const unsigned q = z.p0 + (unsigned)s;
+    const T v = sr[c * ld + j];
+    if (kJac) {
+      const T xo = (flags & Z_OWN_ZERO) ? T(0) : xr[q];
+      xw[q] = (flags & Z_OWN_ZERO) ? omega * v : xo + omega * (v - xo);
+    } else {
+      xw[q] = v;
+    }
   }
 }
 
-template <typename T, int W>
-static size_t tile_smem(int ny) {
-  return (size_t)3 * W * (ny | 1) * sizeof(T);
+// ------------------------------------------------------------------ transfers
+// Coarse right-hand side at slot q of the coarse level: the sum of the residuals b - A x of
+// the cell's active children.  With kColour0 the children of colour 1 ((i xor k) odd) are left
+// out: after a zebra sweep that ends with the colour-1 pass their line equations hold
+// exactly (the j-line solve is exact when j is not periodic), so their residuals are
+// rounding only.  Two rows of a fine column share their loads.
+// Levels of at most this many cells are solved row by row and restricted from all children.
+constexpr long long kSerialCells = 512;
+__host__ __device__ inline bool colour0_restriction(const ZL &F, int zebra) {
+  return zebra && !F.jp && (long long)F.nx * F.ny * F.nz > kSerialCells;
 }
-template <typename T, int W>
-static bool tile_fits(int ny) {
-  return tile_smem<T, W>(ny) <= 200 * 1024;
-}
-
-// Residual b - A x at one cell of a level.
-template <typename T>
-__device__ __forceinline__ T zresid(const ZL &L, const Q4<T> *__restrict__ cpl, const Q4<T> *__restrict__ tri,
-                                    const T *__restrict__ x, const T *__restrict__ b, int i, int j, int k,
-                                    long long q) {
-  const ZNb nb = znb(L, i, j, k);
-  const Q4<T> cp = cpl[q], tr = tri[q];
-  T ax = tr.d * x[q];
-  if (nb.ie >= 0) ax += cp.a * x[zidx(L, nb.ie, j, k)];
-  if (nb.iw >= 0) ax += cp.b * x[zidx(L, nb.iw, j, k)];
-  if (nb.js >= 0) ax += tr.a * x[zidx(L, i, nb.js, k)];
-  if (nb.jn >= 0) { const long long s = zidx(L, i, nb.jn, k); ax += tri[s].a * x[s]; }
-  if (nb.kt >= 0) ax += cp.c * x[zidx(L, i, j, nb.kt)];
-  if (nb.kb >= 0) ax += cp.d * x[zidx(L, i, j, nb.kb)];
-  return b[q] - ax;
-}
-
-// Coarse right-hand side: the sum of the residuals of the (active) children.  With
-// colour0_only the children of colour 1 ((i xor k) odd) are left out: after a zebra sweep
-// that ends with the colour-1 pass their line equations hold exactly (the j-line solve is
-// exact when j is not periodic), so their residuals are rounding only.
-template <typename T>
+template <typename T, bool kColour0>
 __device__ __forceinline__ void zrestrict_cell(const ZL &F, const ZL &C, const Q4<T> *__restrict__ cpl,
-                                              const Q4<T> *__restrict__ tri, const T *__restrict__ x,
-                                              const T *__restrict__ b, T *__restrict__ bc, long long t,
-                                              bool colour0_only = false) {
-  const long long ncell = (long long)C.nx * C.ny * C.nz;
-  if (t >= ncell) return;
+                                               const Q2<T> *__restrict__ tri, const T *__restrict__ dg, const T *x,
+                                               const T *b, T *bc, unsigned q) {
   int I, J, K;
-  zcell(C, t, I, J, K);
-  // every child's residual is formed (all its loads are in range) and an inactive child's
-  // left out by a select, so the loads of all children are in flight together
-  T s = 0;
+  if (q >= (unsigned)C.n || !zcell(C, q, I, J, K)) return;
+  const int j0 = 2 * J, j1 = j0 + 1;
+  const unsigned r0 = zrow(F, j0), r1 = zrow(F, j1);
+  const bool lo = j0 > 0, hi = j1 + 1 < F.ny;
+  const unsigned rm = lo ? zrow(F, j0 - 1) : (F.jp ? zrow(F, F.ny - 1) : r0);
+  const unsigned rp = hi ? zrow(F, j1 + 1) : 0u;  // row 0 (its cs is the wrap coupling, or 0)
+  T res[8];  // of child a + 2 (j & 1) + 4 c
 #pragma unroll
   for (int c = 0; c < 2; c++)
 #pragma unroll
-    for (int bb = 0; bb < 2; bb++)
+    for (int a = 0; a < 2; a++) {
+      if (kColour0 && a != c) continue;
+      const int i = 2 * I + a, k = 2 * K + c;
+      const unsigned p = zcol(F, i, k);
+      const int ie = i + 1 < F.nx ? i + 1 : (F.ip ? 0 : i), iw = i > 0 ? i - 1 : (F.ip ? F.nx - 1 : i);
+      const int kt = k + 1 < F.nz ? k + 1 : (F.kp ? 0 : k), kb = k > 0 ? k - 1 : (F.kp ? F.nz - 1 : k);
+      const unsigned pe = zcol(F, ie, k), pw = zcol(F, iw, k), pt = zcol(F, i, kt), pb = zcol(F, i, kb);
+      const Q4<T> c0 = cpl[p + r0], c1 = cpl[p + r1];
+      const T s0 = tri[p + r0].a, s1 = tri[p + r1].a, s2 = (hi || F.jp) ? tri[p + rp].a : T(0);
+      const T x0 = *(x + p + r0), x1 = *(x + p + r1), xm = *(x + p + rm), xp = *(x + p + rp);
+      const T e0 = *(x + pe + r0), e1 = *(x + pe + r1), w0 = *(x + pw + r0), w1 = *(x + pw + r1);
+      const T t0 = *(x + pt + r0), t1 = *(x + pt + r1), d0 = *(x + pb + r0), d1 = *(x + pb + r1);
+      const T b0 = *(b + p + r0), b1 = *(b + p + r1);
+      const T g0 = dg[p + r0], g1 = dg[p + r1];
+      T a0 = g0 * x0, a1 = g1 * x1;
+      a0 += c0.a * e0; a1 += c1.a * e1;
+      a0 += c0.b * w0; a1 += c1.b * w1;
+      a0 += s0 * xm; a1 += s1 * x0;
+      a0 += s1 * x1; a1 += s2 * xp;
+      a0 += c0.c * t0; a1 += c1.c * t1;
+      a0 += c0.d * d0; a1 += c1.d * d1;
+      res[a + 4 * c] = g0 != T(0) ? b0 - a0 : T(0);
+      res[a + 2 + 4 * c] = g1 != T(0) ? b1 - a1 : T(0);
+    }
+  T sum = 0;
 #pragma unroll
-      for (int a = 0; a < 2; a++) {
-        if (colour0_only && a != c) continue;
-        const int i = 2 * I + a, j = 2 * J + bb, k = 2 * K + c;
-        const long long q = zidx(F, i, j, k);
-        const T r = zresid<T>(F, cpl, tri, x, b, i, j, k, q);
-        if (tri[q].d != T(0)) s += r;
-      }
-  bc[zidx(C, I, J, K)] = s;
+  for (int ch = 0; ch < 8; ch++)
+    if (!kColour0 || (ch & 1) == ch >> 2) sum += res[ch];
+  bc[q] = sum;
 }
 
 template <typename T, bool kColour0>
-__global__ void k_zrestrict(ZL F, ZL C, const Q4<T> *__restrict__ cpl, const Q4<T> *__restrict__ tri,
-                            const T *__restrict__ x, const T *__restrict__ b, T *__restrict__ bc) {
-  pdl_prologue();
-  zrestrict_cell<T>(F, C, cpl, tri, x, b, bc, blockIdx.x * (long long)blockDim.x + threadIdx.x, kColour0);
+__global__ void __launch_bounds__(128) k_zrestrict(ZL F, ZL C, const Q4<T> *__restrict__ cpl,
+                                                   const Q2<T> *__restrict__ tri, const T *__restrict__ dg, const T *x,
+                                                   const T *b, T *bc) {
+  pdl_wait();
+  zrestrict_cell<T, kColour0>(F, C, cpl, tri, dg, x, b, bc, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-// x_fine += P x_coarse (cell-centred trilinear).
-template <typename T>
-__device__ __forceinline__ void zprolong_cell(const ZL &F, const ZL &C, const uint8_t *__restrict__ actF,
-                                             const uint8_t *__restrict__ actC, T *__restrict__ x,
-                                             const T *__restrict__ xc, long long t) {
-  const long long ncell = (long long)F.nx * F.ny * F.nz;
-  if (t >= ncell) return;
-  int i, j, k;
-  zcell(F, t, i, j, k);
-  const long long q = zidx(F, i, j, k);
-  if (!actF[q]) return;
-  const int I = i >> 1, J = j >> 1, K = k >> 1;
-  // the other coarse cell nearest along each direction, or -1
-  int In = I + ((i & 1) ? 1 : -1), Jn = J + ((j & 1) ? 1 : -1), Kn = K + ((k & 1) ? 1 : -1);
-  if (In < 0 || In >= C.nx) In = C.ip ? (In + C.nx) % C.nx : -1;
-  if (Jn < 0 || Jn >= C.ny) Jn = C.jp ? (Jn + C.ny) % C.ny : -1;
-  if (Kn < 0 || Kn >= C.nz) Kn = C.kp ? (Kn + C.nz) % C.nz : -1;
-  const long long own = zidx(C, I, J, K);
-  // every load first (the flag and the value of each coarse neighbour are independent
-  // loads), then the sums in a fixed order: the loads do not wait on the flags
-  T v[8];
-  bool ok[8];
-#pragma unroll
-  for (int n = 1; n < 8; n++) {
-    const int a = n & 1, bb = (n >> 1) & 1, c = n >> 2;
-    const int ii = a ? In : I, jj = bb ? Jn : J, kk = c ? Kn : K;
-    const bool in = ii >= 0 && jj >= 0 && kk >= 0;
-    const long long qc = in ? zidx(C, ii, jj, kk) : own;
-    ok[n] = in && actC[qc];
-    v[n] = xc[qc];
-  }
-  const T xo = xc[own], xq = x[q];
-  T wown = T(27) / T(64);
-  T s = 0;
-#pragma unroll
-  for (int c = 0; c < 2; c++)
-#pragma unroll
-    for (int bb = 0; bb < 2; bb++)
-#pragma unroll
-      for (int a = 0; a < 2; a++) {
-        if (a + bb + c == 0) continue;
-        const T w = (a ? T(1) : T(3)) * (bb ? T(1) : T(3)) * (c ? T(1) : T(3)) / T(64);
-        const int n = a + 2 * bb + 4 * c;
-        if (!ok[n]) { wown += w; continue; }
-        s += w * v[n];
-      }
-  x[q] = xq + (s + wown * xo);
-}
-
-template <typename T>
-__global__ void k_zprolong(ZL F, ZL C, const uint8_t *__restrict__ actF, const uint8_t *__restrict__ actC,
-                           T *__restrict__ x, const T *__restrict__ xc) {
-  pdl_prologue();
-  zprolong_cell<T>(F, C, actF, actC, x, xc, blockIdx.x * (long long)blockDim.x + threadIdx.x);
-}
-
-// The same prolongation from the coarse side: coarse cell t (natural index) loads its
-// 3 x 3 x 3 neighbourhood (values and activity) once and updates its eight children, each
-// child with zprolong_cell's neighbours, weights and order of summation, so the results are
-// the same bits.  Needs a fine level of exactly twice the coarse cells in every direction.
-template <typename T>
-__device__ __forceinline__ void zprolong8_cell(const ZL &F, const ZL &C, const uint8_t *__restrict__ actF,
-                                               const uint8_t *__restrict__ actC, T *__restrict__ x,
-                                               const T *__restrict__ xc, long long t) {
-  const long long nc = (long long)C.nx * C.ny * C.nz;
-  if (t >= nc) return;
+// x_fine += P x_coarse (cell-centred trilinear) for the children of the coarse cell at slot q:
+// its 3 x 3 x 3 neighbourhood is loaded once.  kColour1 leaves out the children of colour 0:
+// the zebra sweep that follows solves their columns from the colour-1 columns alone (when j
+// is not periodic) and never reads their value.
+template <typename T, bool kColour1>
+__device__ __forceinline__ void zprolong_cell(const ZL &F, const ZL &C, const unsigned long long *__restrict__ mask,
+                                              T *x, const T *xc, unsigned q) {
   int I, J, K;
-  zcell(C, t, I, J, K);
-  // neighbour index along one direction, wrapped on a periodic level, -1 beyond an edge
-  auto nb = [](int v, int n, int per) { return (v >= 0 && v < n) ? v : (per ? (v + n) % n : -1); };
-  const int Ii[3] = {nb(I - 1, C.nx, C.ip), I, nb(I + 1, C.nx, C.ip)};
-  const int Jj[3] = {nb(J - 1, C.ny, C.jp), J, nb(J + 1, C.ny, C.jp)};
-  const int Kk[3] = {nb(K - 1, C.nz, C.kp), K, nb(K + 1, C.nz, C.kp)};
-  const long long own = zidx(C, I, J, K);
+  if (q >= (unsigned)C.n || !zcell(C, q, I, J, K)) return;
+  const unsigned long long ok = mask[q];
+  // a neighbour that does not exist is read from the cell itself and masked out
+  auto nb = [](int v, int n, int per, int own) { const int w = wrap_or_none(v, n, per); return w < 0 ? own : w; };
+  const int Ii[3] = {nb(I - 1, C.nx, C.ip, I), I, nb(I + 1, C.nx, C.ip, I)};
+  const int Kk[3] = {nb(K - 1, C.nz, C.kp, K), K, nb(K + 1, C.nz, C.kp, K)};
+  const unsigned rr[3] = {zrow(C, nb(J - 1, C.ny, C.jp, J)), zrow(C, J), zrow(C, nb(J + 1, C.ny, C.jp, J))};
   T v[27];
-  unsigned ok = 0;
 #pragma unroll
-  for (int e = 0; e < 27; e++) {
-    const int a = e % 3, b = (e / 3) % 3, cc = e / 9;
-    const bool in = Ii[a] >= 0 && Jj[b] >= 0 && Kk[cc] >= 0;
-    const long long qc = in ? zidx(C, Ii[a], Jj[b], Kk[cc]) : own;
-    v[e] = xc[qc];
-    if (in && actC[qc]) ok |= 1u << e;
-  }
+  for (int e = 0; e < 27; e++) v[e] = *(xc + zcol(C, Ii[e % 3], Kk[e / 9]) + rr[e / 3 % 3]);
   const T xo = v[13];
+  const unsigned f0 = zrow(F, 2 * J), f1 = zrow(F, 2 * J + 1);
+  unsigned qf[8];
+  T xq[8];
 #pragma unroll
   for (int ch = 0; ch < 8; ch++) {
     const int ai = ch & 1, aj = (ch >> 1) & 1, ak = ch >> 2;
-    const int i = 2 * I + ai, j = 2 * J + aj, k = 2 * K + ak;
-    const long long q = zidx(F, i, j, k);
-    if (!actF[q]) continue;
-    // offset of the other nearest coarse cell: +1 for an odd child index, -1 for an even one
+    if (kColour1 && ai == ak) continue;
+    qf[ch] = zcol(F, 2 * I + ai, 2 * K + ak) + (aj ? f1 : f0);
+    xq[ch] = *(x + qf[ch]);
+  }
+#pragma unroll
+  for (int ch = 0; ch < 8; ch++) {
+    const int ai = ch & 1, aj = (ch >> 1) & 1, ak = ch >> 2;
+    if (kColour1 && ai == ak) continue;
+    // the other nearest coarse cell: the next one for an odd child index, the previous one for an even one
     const int di = ai ? 2 : 0, dj = aj ? 2 : 0, dk = ak ? 2 : 0;
-    const T xq = x[q];
     T wown = T(27) / T(64);
     T s = 0;
 #pragma unroll
@@ -721,50 +767,43 @@ __device__ __forceinline__ void zprolong8_cell(const ZL &F, const ZL &C, const u
           if (a + bb + c == 0) continue;
           const T w = (a ? T(1) : T(3)) * (bb ? T(1) : T(3)) * (c ? T(1) : T(3)) / T(64);
           const int e = (a ? di : 1) + 3 * (bb ? dj : 1) + 9 * (c ? dk : 1);
-          if (!((ok >> e) & 1u)) { wown += w; continue; }
+          if (!((ok >> e) & 1ull)) { wown += w; continue; }
           s += w * v[e];
         }
-    x[q] = xq + (s + wown * xo);
+    if ((ok >> (27 + ch)) & 1ull) x[qf[ch]] = xq[ch] + (s + wown * xo);
   }
 }
 
-template <typename T>
-__global__ void k_zprolong8(ZL F, ZL C, const uint8_t *__restrict__ actF, const uint8_t *__restrict__ actC,
-                            T *__restrict__ x, const T *__restrict__ xc) {
-  pdl_prologue();
-  zprolong8_cell<T>(F, C, actF, actC, x, xc, blockIdx.x * (long long)blockDim.x + threadIdx.x);
-}
-
-// act[q] = 1 where the level's diagonal is non-zero (an active unknown).
-__global__ void k_mg_active(long long n, const double *__restrict__ op, uint8_t *__restrict__ act) {
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (q < n) act[q] = op[OP_DG * n + q] != 0.0 ? 1 : 0;
+template <typename T, bool kColour1>
+__global__ void __launch_bounds__(128) k_zprolong(ZL F, ZL C, const unsigned long long *__restrict__ mask,
+                                                  T *x, const T *xc) {
+  pdl_wait();
+  zprolong_cell<T, kColour1>(F, C, mask, x, xc, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 // ------------------------------------------------------------------ bottom of the V-cycle
-// The coarse levels are too small to fill the GPU, and a launch per colour pass costs
-// more than the work.  From the first level of at most kBottomCells cells down, one thread
-// block runs the rest of the V-cycle (smoothing, restriction, coarsest sweeps,
-// prolongation) with block barriers between the phases; the level data stay in L2.  On the
-// B200 at 256 x 192 x 256 (V-cycle ms, FP32 / FP64): 512 cells (the 8 x 6 x 8 level down)
-// 1.450 / 2.268, 4096 or 8192 1.470 / 2.313, 32768 1.772 / 2.738.
+// The coarse levels are too small to fill the GPU, and a launch per colour pass costs more
+// than the work.  From the first level of at most kSerialCells cells down, one thread block
+// runs the rest of the V-cycle (smoothing, restriction, coarsest sweeps, prolongation), one
+// thread a column, with the vectors and the smoother's operator of all its levels in shared
+// memory and block barriers between the phases: a phase is a chain of shared-memory loads and a barrier, with no trip
+// to L2.  Starting at 4096 cells (lane groups in the same block) took 156 us a V-cycle of
+// 64^3 cells against 133 (FP32); a cluster of eight blocks exchanging through L2 186.
 constexpr int kBottomMaxLevels = 12;
 #ifndef VFS_BOTTOM_THREADS
 #define VFS_BOTTOM_THREADS 512
 #endif
 constexpr int kBottomThreads = VFS_BOTTOM_THREADS;
-#ifndef VFS_BOTTOM_CELLS
-#define VFS_BOTTOM_CELLS 512
-#endif
-constexpr long long kBottomCells = VFS_BOTTOM_CELLS;
+constexpr size_t kBottomSmem = 200 * 1024;
 
 template <typename T>
 struct BLevel {
   ZL z;
-  const uint8_t *act;
-  const Q4<T> *cpl, *tri;
-  T *x, *b, *xo;
-  Q2<T> *ds;
+  const unsigned long long *pmask;  // of the cells of this level, for the prolongation to the finer one
+  const Q4<T> *cpl;
+  const Q2<T> *tri;
+  const T *cpr, *dg;
+  unsigned sm;  // the level's arrays in shared memory, n slots each: x, b, previous x, ce, cw, ct, cb, cs, iden, cpr
   int zebra;
 };
 template <typename T>
@@ -772,104 +811,246 @@ struct Bottom {
   int nl;
   int pre, post, coarse;
   T omega;
+  T *x;        // the top level's vectors
+  const T *b;
   BLevel<T> lv[kBottomMaxLevels];
 };
 
-template <typename T>
-__device__ void blk_smooth(const BLevel<T> &L, int sweeps, bool x_zero, T omega) {
-  const long long half = (long long)L.z.nz * L.z.hx;
-  for (int s = 0; s < sweeps; s++) {
-    const bool z = x_zero && s == 0;
-    if (L.zebra) {
-      for (int col = 0; col < 2; col++) {
-        for (long long t = threadIdx.x; t < half; t += blockDim.x)
-          zline_column<T, 2>(L.z, L.cpl, L.tri, L.b, L.x, L.ds, L.x, col, T(1), (z && col == 0) ? 1 : 0, t);
-        __syncthreads();
+// One column of a bottom level by one thread, everything in shared memory (sm: the level's
+// arrays); the right-hand sides are eliminated in the column's slots of xw.
+template <typename T, bool kJac>
+__device__ __forceinline__ void bot_column(const ZL &L, const ZCol &z, const T *sm, const T *xr, T *xw, int flags, T omega) {
+  if (!z.valid) return;
+  const unsigned n = (unsigned)L.n;
+  const T *b = sm + n + z.p0, *ce = sm + 3 * n + z.p0, *cw = ce + n, *ct = cw + n, *cb = ct + n, *cs = cb + n,
+          *id = cs + n, *cx = id + n;
+  const T *xo = xr + z.p0;
+  T *xv = xw + z.p0;
+  const int ny = L.ny;
+  T wrap = 0, first = 0, last = 0;
+  if (L.jp && !(flags & Z_OWN_ZERO)) { wrap = cs[0]; first = xo[0]; last = xo[ny - 1]; }
+  constexpr int CH = 4;
+  T d = 0;
+  for (int j0 = 0; j0 < ny; j0 += CH) {
+    T r[CH], lo[CH], ii[CH];
+#pragma unroll
+    for (int u = 0; u < CH; u++) {
+      const int j = min(j0 + u, ny - 1);
+      r[u] = b[j]; lo[u] = cs[j]; ii[u] = id[j];
+      if (!(flags & Z_NB_ZERO)) {
+        r[u] -= ce[j] * xo[j + z.oe];
+        r[u] -= cw[j] * xo[j + z.ow];
+        r[u] -= ct[j] * xo[j + z.ot];
+        r[u] -= cb[j] * xo[j + z.ob];
       }
-    } else {
-      if (!z) {
-        for (long long t = threadIdx.x; t < L.z.n; t += blockDim.x) L.xo[t] = L.x[t];
-        __syncthreads();
-      }
-      for (long long t = threadIdx.x; t < 2 * half; t += blockDim.x)
-        zline_column<T, 2>(L.z, L.cpl, L.tri, L.b, L.xo, L.ds, L.x, -1, omega, z ? 1 : 0, t);
-      __syncthreads();
+      if (j == 0) { r[u] -= wrap * last; lo[u] = 0; }
+      if (j == ny - 1) r[u] -= wrap * first;
+    }
+#pragma unroll
+    for (int u = 0; u < CH; u++) {
+      if (j0 + u >= ny) break;
+      d = (r[u] - lo[u] * d) * ii[u];
+      xv[j0 + u] = d;
+    }
+  }
+  T x = 0;
+  for (int j1 = ny - 1; j1 >= 0; j1 -= CH) {
+    T dd[CH], cc[CH], old[CH];
+#pragma unroll
+    for (int u = 0; u < CH; u++) {
+      const int j = max(j1 - u, 0);
+      dd[u] = xv[j]; cc[u] = cx[j];
+      old[u] = kJac && !(flags & Z_OWN_ZERO) ? xo[j] : T(0);
+    }
+#pragma unroll
+    for (int u = 0; u < CH; u++) {
+      if (j1 - u < 0) break;
+      x = dd[u] - cc[u] * x;
+      xv[j1 - u] = kJac ? ((flags & Z_OWN_ZERO) ? omega * x : old[u] + omega * (x - old[u])) : x;
     }
   }
 }
 
+// `sweeps` smoothing sweeps of a bottom level; x ends in x.  At most kSerialCells columns, so
+// every thread has at most one of each colour.
 template <typename T>
-__global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(Bottom<T> B) {
-  pdl_prologue();
+__device__ void bot_smooth(const BLevel<T> &L, T *sm, int sweeps, bool x_zero, T omega) {
+  T *x = sm;
+  if (L.zebra) {
+    const ZCol z[2] = {zcolumn(L.z, 0, threadIdx.x), zcolumn(L.z, 1, threadIdx.x)};
+    for (int s = 0; s < sweeps; s++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) {
+        const bool zero = x_zero && s == 0;
+        bot_column<T, false>(L.z, z[c], sm, x, x, (zero ? Z_OWN_ZERO : 0) | (zero && c == 0 ? Z_NB_ZERO : 0), T(1));
+        __syncthreads();
+      }
+    return;
+  }
+  // line Jacobi
+  T *xo = sm + 2 * L.z.n;
+  T *from = x_zero ? xo : x, *to = x_zero ? x : xo;
+  const ZCol z = zcolumn(L.z, -1, threadIdx.x);
+  for (int s = 0; s < sweeps; s++) {
+    bot_column<T, true>(L.z, z, sm, from, to, x_zero && s == 0 ? Z_NB_ZERO | Z_OWN_ZERO : 0, omega);
+    __syncthreads();
+    T *const t = from; from = to; to = t;
+  }
+  if (from != x) {
+    for (unsigned q = threadIdx.x; q < (unsigned)L.z.n; q += kBottomThreads) x[q] = from[q];
+    __syncthreads();
+  }
+}
+
+template <typename T>
+__global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_constant__ Bottom<T> B) {
+  extern __shared__ __align__(16) unsigned char bot_raw[];
+  T *sm = reinterpret_cast<T *>(bot_raw);
+  // the operators, and zero vectors (slots that hold no cell are read and never written)
+  for (int l = 0; l < B.nl; l++) {
+    const BLevel<T> &L = B.lv[l];
+    const unsigned n = (unsigned)L.z.n;
+    T *s = sm + L.sm;
+    for (unsigned q = threadIdx.x; q < n; q += kBottomThreads) {
+      const Q4<T> c = L.cpl[q];
+      const Q2<T> t = L.tri[q];
+      s[q] = s[n + q] = s[2 * n + q] = T(0);
+      s[3 * n + q] = c.a; s[4 * n + q] = c.b; s[5 * n + q] = c.c; s[6 * n + q] = c.d;
+      s[7 * n + q] = t.a; s[8 * n + q] = t.b; s[9 * n + q] = L.cpr[q];
+    }
+  }
+  __syncthreads();
+  pdl_wait();
+  {
+    const ZL &z = B.lv[0].z;
+    const T *b = B.b;
+    for (unsigned q = threadIdx.x; q < (unsigned)z.n; q += kBottomThreads) sm[z.n + q] = b[q];
+    __syncthreads();
+  }
   for (int l = 0; l < B.nl - 1; l++) {
     const BLevel<T> &F = B.lv[l], &C = B.lv[l + 1];
-    blk_smooth<T>(F, B.pre, true, B.omega);
-    const long long nc = (long long)C.z.nx * C.z.ny * C.z.nz;
-    for (long long t = threadIdx.x; t < nc; t += blockDim.x)
-      zrestrict_cell<T>(F.z, C.z, F.cpl, F.tri, F.x, F.b, C.b, t);
+    T *x = sm + F.sm, *bc = sm + C.sm + C.z.n;
+    bot_smooth<T>(F, x, B.pre, true, B.omega);
+    for (unsigned q = threadIdx.x; q < (unsigned)C.z.n; q += kBottomThreads)
+      zrestrict_cell<T, false>(F.z, C.z, F.cpl, F.tri, F.dg, x, x + F.z.n, bc, q);
     __syncthreads();
   }
-  blk_smooth<T>(B.lv[B.nl - 1], B.coarse, true, B.omega);
+  bot_smooth<T>(B.lv[B.nl - 1], sm + B.lv[B.nl - 1].sm, B.coarse, true, B.omega);
   for (int l = B.nl - 2; l >= 0; l--) {
     const BLevel<T> &F = B.lv[l], &C = B.lv[l + 1];
-    const long long nf = (long long)F.z.nx * F.z.ny * F.z.nz;
-    for (long long t = threadIdx.x; t < nf; t += blockDim.x) zprolong_cell<T>(F.z, C.z, F.act, C.act, F.x, C.x, t);
+    T *x = sm + F.sm;
+    const bool half = F.zebra && !F.z.jp && B.post > 0;
+    for (unsigned q = threadIdx.x; q < (unsigned)C.z.n; q += kBottomThreads) {
+      if (half) zprolong_cell<T, true>(F.z, C.z, C.pmask, x, sm + C.sm, q);
+      else zprolong_cell<T, false>(F.z, C.z, C.pmask, x, sm + C.sm, q);
+    }
     __syncthreads();
-    blk_smooth<T>(F, B.post, false, B.omega);
+    bot_smooth<T>(F, x, B.post, false, B.omega);
+  }
+  T *out = B.x;
+  for (unsigned q = threadIdx.x; q < (unsigned)B.lv[0].z.n; q += kBottomThreads) out[q] = sm[q];
+}
+
+// ------------------------------------------------------------------ grid layout <-> columns
+// A block moves kTileI consecutive i of one k plane and all rows through shared memory, so that
+// both sides are accessed in runs.  Columns too long for that go directly.
+constexpr int kTileI = 16;
+constexpr size_t kTileSmem = 200 * 1024;
+template <typename T>
+__host__ __device__ inline size_t tile_bytes(const ZL &L) { return sizeof(T) * kTileI * ((size_t)L.S | 1); }
+__host__ __device__ inline unsigned tiles_i(const ZL &L) { return (unsigned)(L.nx + kTileI - 1) / kTileI; }
+
+template <typename T, typename VT>
+__global__ void __launch_bounds__(256) k_to_columns(Grid g, ZL L, DynPtrT<const VT> vv, T *__restrict__ b) {
+  extern __shared__ __align__(16) unsigned char tile_raw[];
+  T *sm = reinterpret_cast<T *>(tile_raw);
+  pdl_wait();
+  const VT *__restrict__ v = vv.get();
+  const unsigned ib = tiles_i(L);
+  const int k = (int)(blockIdx.x / ib), i0 = (int)(blockIdx.x % ib) * kTileI, ld = L.S | 1;
+  const int a = threadIdx.x % kTileI;
+  for (int j = threadIdx.x / kTileI; j < L.S; j += 256 / kTileI) {  // rows past ny: the empty slots
+    T t = 0;
+    if (j < L.ny && i0 + a < L.nx) t = (T)v[lidx(g, i0 + a + 1, j + 1, k + 1)];
+    sm[a * ld + (int)zrow(L, j)] = t;
+  }
+  __syncthreads();
+  for (int c = threadIdx.x >> 5; c < kTileI && i0 + c < L.nx; c += 8) {  // a warp a column
+    const unsigned p0 = zcol(L, i0 + c, k);
+    for (int s = threadIdx.x & 31; s < L.S; s += 32) b[p0 + s] = sm[c * ld + s];
   }
 }
-
-// DA-layout vector (FP64, or FP32 in the FP32 inner Krylov) -> finest-level right-hand side.
 template <typename T, typename VT>
-__global__ void k_to_zebra(Grid g, ZL L, const VT *__restrict__ v, const int *__restrict__ jslot, long long ldv,
-                           T *__restrict__ b) {
-  pdl_prologue();
-  if (jslot) v += (long long)(*jslot) * ldv;  // the j-th basis vector of a device-driven solve
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  const long long ncell = (long long)L.nx * L.ny * L.nz;
-  if (t >= ncell) return;
+__global__ void __launch_bounds__(256) k_to_columns_direct(Grid g, ZL L, DynPtrT<const VT> vv, T *__restrict__ b) {
+  pdl_wait();
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
   int i, j, k;
-  zcell(L, t, i, j, k);
-  b[zidx(L, i, j, k)] = (T)v[lidx(g, i + 1, j + 1, k + 1)];
+  if (q >= (unsigned)L.n || !zcell(L, q, i, j, k)) return;
+  b[q] = (T)vv.get()[lidx(g, i + 1, j + 1, k + 1)];
 }
-
-// Finest-level solution -> DA-layout vector (zero off the unknowns).
-template <typename T, typename VT>
-__global__ void k_from_zebra(Grid g, ZL L, const uint8_t *__restrict__ fluid, const T *__restrict__ x,
-                             const int *__restrict__ jslot, long long ldv, VT *__restrict__ z) {
-  pdl_prologue();
-  if (jslot) z += (long long)(*jslot) * ldv;
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  const unsigned up = (unsigned)p, umx = (unsigned)g.mx, umy = (unsigned)g.my;
-  const unsigned r = up / umx, kk = r / umy;
-  const int i = (int)(up - r * umx), j = (int)(r - kk * umy), k = (int)kk;
-  double v = 0;
-  if (fluid[p] && i >= 1 && i <= g.mx - 2 && j >= 1 && j <= g.my - 2 && k >= 1 && k <= g.mz - 2)
-    v = (double)x[zidx(L, i - 1, j - 1, k - 1)];
-  z[p] = (VT)v;
+// The interior points of the grid vector (the V-cycle's solution is zero off the unknowns).
+template <typename T>
+__global__ void __launch_bounds__(256) k_from_columns(Grid g, ZL L, const T *__restrict__ x, DynPtrT<T> zv) {
+  extern __shared__ __align__(16) unsigned char tile_raw[];
+  T *sm = reinterpret_cast<T *>(tile_raw);
+  pdl_wait();
+  T *__restrict__ z = zv.get();
+  const unsigned ib = tiles_i(L);
+  const int k = (int)(blockIdx.x / ib), i0 = (int)(blockIdx.x % ib) * kTileI, ld = L.S | 1;
+  for (int c = threadIdx.x >> 5; c < kTileI && i0 + c < L.nx; c += 8) {  // a warp a column
+    const unsigned p0 = zcol(L, i0 + c, k);
+#pragma unroll 4
+    for (int s = threadIdx.x & 31; s < L.S; s += 32) sm[c * ld + s] = x[p0 + s];
+  }
+  __syncthreads();
+  const int a = threadIdx.x % kTileI;
+  if (i0 + a >= L.nx) return;
+  for (int j = threadIdx.x / kTileI; j < L.ny; j += 256 / kTileI)
+    z[lidx(g, i0 + a + 1, j + 1, k + 1)] = sm[a * ld + (int)zrow(L, j)];
+}
+template <typename T>
+__global__ void __launch_bounds__(256) k_from_columns_direct(Grid g, ZL L, const T *__restrict__ x, DynPtrT<T> zv) {
+  pdl_wait();
+  const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+  int i, j, k;
+  if (q >= (unsigned)L.n || !zcell(L, q, i, j, k)) return;
+  zv.get()[lidx(g, i + 1, j + 1, k + 1)] = x[q];
 }
 
 // ------------------------------------------------------------------ host side
-static ZL make_zl(int nx, int ny, int nz, const Grid &g) {
+// The columns of a level: 32 lanes of ceil(ny/32) rows (fewer lanes for short columns), or one
+// thread a column on small levels and on coarse levels that line Jacobi smooths; their
+// columns have an odd number of slots, free of shared-memory bank conflicts.
+static bool two_colours(const ZL &L) { return !((L.ip && (L.nx & 1)) || (L.kp && (L.nz & 1))); }
+static ZL make_zl(int nx, int ny, int nz, const Grid &g, bool finest) {
   ZL L;
   L.nx = nx; L.ny = ny; L.nz = nz;
   L.hx = (nx + 1) / 2;
   L.ip = g.iper; L.jp = g.jper; L.kp = g.kper;
-  L.n = (long long)nz * ny * 2 * L.hx;
+  L.serial = (long long)nx * ny * nz <= kSerialCells || (!finest && !two_colours(L) && ny <= 256);
+  L.seg = L.serial ? 1 : (ny + 31) / 32;
+  L.ls = L.serial ? ny | 1 : (ny + L.seg - 1) / L.seg;
+  L.S = L.seg * L.ls;
+  L.lwl = 0;
+  while ((1 << L.lwl) < L.ls && L.lwl < 5) L.lwl++;
+  L.lw = 1 << L.lwl;
+  L.n = (long long)nz * 2 * L.hx * L.S;
   return L;
 }
 
+static void level_free(MGLevel &L) {
+  cudaFree(L.op64); cudaFree(L.pk64); cudaFree(L.pk32); cudaFree(L.v64); cudaFree(L.v32); cudaFree(L.act);
+  cudaFree(L.pmask);
+  L.op64 = nullptr;
+}
 void mg_free(Poisson &P) {
-  for (MGLevel &L : P.lv) {
-    cudaFree(L.op64); cudaFree(L.pk64); cudaFree(L.pk32); cudaFree(L.v64); cudaFree(L.v32); cudaFree(L.act);
-  }
+  for (MGLevel &L : P.lv) level_free(L);
   P.lv.clear();
 }
 
 // Per level: raw FP64 couplings and Thomas factors (op64, used to build the next level),
-// the packed FP64 and FP32 operators, and the work vectors x | b | xo | ds (2n).  A rebuild
-// on the same grid (every first time step runs PoissonLHSNew) keeps the levels' buffers.
+// the packed FP64 and FP32 operators, and the work vectors x | b | xo.  A rebuild on the
+// same grid (every first time step runs PoissonLHSNew) keeps the levels' buffers.
 int mg_setup(Ctx *c) {
   Poisson &P = c->ps;
   const Grid &g = c->g;
@@ -884,27 +1065,24 @@ int mg_setup(Ctx *c) {
   };
   while ((int)P.lv.size() < maxlev) {
     MGLevel L;
-    L.z = make_zl(nx, ny, nz, g);
-    L.zebra = !((L.z.ip && (nx & 1)) || (L.z.kp && (nz & 1)));
+    L.z = make_zl(nx, ny, nz, g, P.lv.empty());
+    L.zebra = two_colours(L.z);
     const long long n = L.z.n;
     if (n >= (1LL << 31)) return fail(VFS_ERR_INVALID, "poisson_lhs: grid too large for the multigrid indexing");
     const size_t l = P.lv.size();
     if (l < old.size() && old[l].z.n == n && old[l].op64) {
       L.op64 = old[l].op64; L.pk64 = old[l].pk64; L.pk32 = old[l].pk32;
-      L.v64 = old[l].v64; L.v32 = old[l].v32; L.act = old[l].act;
-      old[l].op64 = nullptr;  // taken
+      L.v64 = old[l].v64; L.v32 = old[l].v32; L.act = old[l].act; L.pmask = old[l].pmask;
+      old[l] = MGLevel();  // taken
     } else {
-      if (l < old.size()) {
-        MGLevel &O = old[l];
-        cudaFree(O.op64); cudaFree(O.pk64); cudaFree(O.pk32); cudaFree(O.v64); cudaFree(O.v32); cudaFree(O.act);
-        O.op64 = nullptr;
-      }
+      if (l < old.size()) { level_free(old[l]); old[l] = MGLevel(); }
       bool ok = cudaMalloc(&L.op64, sizeof(double) * NOP * n) == cudaSuccess;
       ok &= cudaMalloc(&L.pk64, sizeof(double) * 8 * n) == cudaSuccess;
       ok &= cudaMalloc(&L.pk32, sizeof(float) * 8 * n) == cudaSuccess;
-      ok &= cudaMalloc(&L.v64, sizeof(double) * 5 * n) == cudaSuccess;
-      ok &= cudaMalloc(&L.v32, sizeof(float) * 5 * n) == cudaSuccess;
+      ok &= cudaMalloc(&L.v64, sizeof(double) * 3 * n) == cudaSuccess;
+      ok &= cudaMalloc(&L.v32, sizeof(float) * 3 * n) == cudaSuccess;
       ok &= cudaMalloc(&L.act, n) == cudaSuccess;
+      if (l > 0) ok &= cudaMalloc(&L.pmask, sizeof(unsigned long long) * n) == cudaSuccess;
       if (!ok) {
         P.lv.push_back(L);
         return fail(VFS_ERR_CUDA, "poisson_lhs: multigrid allocation failed");
@@ -913,206 +1091,225 @@ int mg_setup(Ctx *c) {
     cudaMemsetAsync(L.op64, 0, sizeof(double) * NOP * n, c->stream);
     cudaMemsetAsync(L.pk64, 0, sizeof(double) * 8 * n, c->stream);
     cudaMemsetAsync(L.pk32, 0, sizeof(float) * 8 * n, c->stream);
-    cudaMemsetAsync(L.v64, 0, sizeof(double) * 5 * n, c->stream);
-    cudaMemsetAsync(L.v32, 0, sizeof(float) * 5 * n, c->stream);
-    const long long ncell = (long long)nx * ny * nz;
+    cudaMemsetAsync(L.v64, 0, sizeof(double) * 3 * n, c->stream);
+    cudaMemsetAsync(L.v32, 0, sizeof(float) * 3 * n, c->stream);
+    const unsigned nb = nblocks(n, 128);
     if (P.lv.empty()) {
-      c->launches++, k_mg_fine_couplings<<<nblocks(ncell, 128), 128, 0, c->stream>>>(g, L.z, P.coef, P.fluid, L.op64);
+      c->launches++, k_mg_fine_couplings<<<nb, 128, 0, c->stream>>>(g, L.z, P.coef, P.fluid, L.op64);
     } else {
       const MGLevel &F = P.lv.back();
-      c->launches++, k_mg_coarse_couplings<<<nblocks(ncell, 128), 128, 0, c->stream>>>(F.z, L.z, F.op64, L.op64);
+      c->launches++, k_mg_coarse_couplings<<<nb, 128, 0, c->stream>>>(F.z, L.z, F.op64, L.op64);
     }
     if ((rc = check_launch(c, "k_mg_couplings"))) { P.lv.push_back(L); return fail(rc, "poisson_lhs: multigrid set-up failed"); }
-    c->launches++, k_mg_diag<<<nblocks(ncell, 128), 128, 0, c->stream>>>(L.z, L.op64);
+    c->launches++, k_mg_diag<<<nb, 128, 0, c->stream>>>(L.z, L.op64);
     c->launches++, k_mg_thomas<<<nblocks((long long)nx * nz, 64), 64, 0, c->stream>>>(L.z, L.op64);
     c->launches++, k_mg_active<<<nblocks(n, 256), 256, 0, c->stream>>>(n, L.op64, L.act);
-    c->launches++, k_mg_pack<double><<<nblocks(ncell, 128), 128, 0, c->stream>>>(L.z, L.op64, (Q4<double> *)L.pk64,
-                                                                 (Q4<double> *)L.pk64 + n);
-    c->launches++, k_mg_pack<float><<<nblocks(ncell, 128), 128, 0, c->stream>>>(L.z, L.op64, (Q4<float> *)L.pk32,
-                                                                (Q4<float> *)L.pk32 + n);
+    c->launches++, k_mg_pack<double><<<nb, 128, 0, c->stream>>>(L.z, L.op64, (Q4<double> *)L.pk64, (Q2<double> *)(L.pk64 + 4 * n), L.pk64 + 6 * n,
+                                                                L.pk64 + 7 * n);
+    c->launches++, k_mg_pack<float><<<nb, 128, 0, c->stream>>>(L.z, L.op64, (Q4<float> *)L.pk32, (Q2<float> *)(L.pk32 + 4 * n), L.pk32 + 6 * n,
+                                                               L.pk32 + 7 * n);
+    if (!P.lv.empty())
+      c->launches++, k_mg_pmask<<<nb, 128, 0, c->stream>>>(P.lv.back().z, L.z, P.lv.back().act, L.act, L.pmask);
     P.lv.push_back(L);
     if ((rc = check_launch(c, "k_mg_setup"))) return fail(rc, "poisson_lhs: multigrid set-up failed");
     if ((nx & 1) || (ny & 1) || (nz & 1) || nx < 4 || ny < 4 || nz < 4) break;
     nx /= 2; ny /= 2; nz /= 2;
   }
-  for (size_t l = P.lv.size(); l < old.size(); l++) {  // levels the new hierarchy does not reach
-    MGLevel &O = old[l];
-    cudaFree(O.op64); cudaFree(O.pk64); cudaFree(O.pk32); cudaFree(O.v64); cudaFree(O.v32); cudaFree(O.act);
-  }
+  for (size_t l = P.lv.size(); l < old.size(); l++) level_free(old[l]);  // levels the new hierarchy does not reach
   return VFS_OK;
 }
 
 // Typed views of a level's packed operator and work vectors.
 template <typename T>
 struct LvT {
-  const Q4<T> *cpl, *tri;
+  const Q4<T> *cpl;
+  const Q2<T> *tri;
+  const T *cpr, *dg;
   T *x, *b, *xo;
-  Q2<T> *ds;
 };
 template <typename T>
-static LvT<T> lvt(const MGLevel &L);
-template <>
-LvT<float> lvt<float>(const MGLevel &L) {
-  const long long n = L.z.n;
-  LvT<float> r;
-  r.cpl = (const Q4<float> *)L.pk32; r.tri = (const Q4<float> *)L.pk32 + n;
-  r.x = L.v32; r.b = L.v32 + n; r.xo = L.v32 + 2 * n; r.ds = (Q2<float> *)(L.v32 + 3 * n);
-  return r;
-}
-template <>
-LvT<double> lvt<double>(const MGLevel &L) {
-  const long long n = L.z.n;
-  LvT<double> r;
-  r.cpl = (const Q4<double> *)L.pk64; r.tri = (const Q4<double> *)L.pk64 + n;
-  r.x = L.v64; r.b = L.v64 + n; r.xo = L.v64 + 2 * n; r.ds = (Q2<double> *)(L.v64 + 3 * n);
-  return r;
-}
+struct VCycle {
+  Ctx *c;
+  vfs_solve_opts o;
+  int nl;
+  LvT<T> lvt(int l) const {
+    const MGLevel &L = c->ps.lv[l];
+    const long long n = L.z.n;
+    T *pk = sizeof(T) == 4 ? (T *)L.pk32 : (T *)L.pk64, *v = sizeof(T) == 4 ? (T *)L.v32 : (T *)L.v64;
+    LvT<T> r;
+    r.cpl = (const Q4<T> *)pk;
+    r.tri = (const Q2<T> *)(pk + 4 * n);
+    r.cpr = pk + 6 * n;
+    r.dg = pk + 7 * n;
+    r.x = v;
+    r.b = v + n;
+    r.xo = v + 2 * n;
+    return r;
+  }
+};
 
 static const double kJacobiOmega = 0.8;
 
-// Launches one tiled colour pass; false when the level's columns do not fit the tile.
-// rc receives the launch status.
-template <typename T, int W>
-static bool launch_tile_w(Ctx *c, const MGLevel &L, const LvT<T> &v, int colour, int x_zero, int &rc) {
-  if (!tile_fits<T, W>(L.z.ny)) return false;
-  const size_t smem = tile_smem<T, W>(L.z.ny);
-  static bool attr_set = false;
-  if (!attr_set) {
-    cudaFuncSetAttribute(k_zline_tile<T, W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
-    attr_set = true;
-  }
-  const int tiles = (L.z.hx + W - 1) / W;
-  rc = launch_chain(c, "k_zline_tile", k_zline_tile<T, W>, dim3(tiles * L.z.nz), dim3(kTileThreads), smem, L.z,
-                    v.cpl, v.tri, v.b, v.x, v.x, colour, x_zero);
-  return true;
-}
 template <typename T>
-static bool launch_zline_tile(Ctx *c, const MGLevel &L, const LvT<T> &v, int colour, int x_zero, int &rc) {
-  if (sizeof(T) == 4)
-    return launch_tile_w<T, VFS_ZTILE_W32>(c, L, v, colour, x_zero, rc) ||
-           launch_tile_w<T, 8>(c, L, v, colour, x_zero, rc);
-  return launch_tile_w<T, VFS_ZTILE_W64>(c, L, v, colour, x_zero, rc) ||
-         launch_tile_w<T, 8>(c, L, v, colour, x_zero, rc);
+static int launch_serial(Ctx *c, const MGLevel &L, const LvT<T> &v, const T *xr, T *xw, int colour, int flags) {
+  const unsigned ncol = (unsigned)L.z.nz * L.z.hx * (colour >= 0 ? 1 : 2), nb = nblocks(ncol, kSerialCols);
+  const size_t smem = serial_smem<T>(L.z);
+  const T om = T(kJacobiOmega);
+  const ZOp<T> op{v.cpl, v.tri, v.cpr};
+  // the shared-memory limit is an attribute of the kernel on a device
+  if (smem > 48 * 1024 &&
+      (cudaFuncSetAttribute(k_zserial<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerialSmem) != cudaSuccess ||
+       cudaFuncSetAttribute(k_zserial<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSerialSmem) != cudaSuccess))
+    return set_err(c, VFS_ERR_CUDA, "multigrid: shared-memory limit");
+  return colour < 0 ? launch_chain(c, "k_zserial", k_zserial<T, true>, nb, kSerialThreads, smem, L.z, op, v.b, xr, xw, colour, flags, om)
+                    : launch_chain(c, "k_zserial", k_zserial<T, false>, nb, kSerialThreads, smem, L.z, op, v.b, xr, xw, colour, flags, om);
+}
+// One colour pass, or with colour < 0 a line Jacobi sweep from xr into xw.
+template <typename T>
+static int launch_pass(Ctx *c, const MGLevel &L, const LvT<T> &v, const T *xr, T *xw, int colour, int flags) {
+  const unsigned ncol = (unsigned)L.z.nz * L.z.hx * (colour >= 0 ? 1 : 2);
+  const ZOp<T> op{v.cpl, v.tri, v.cpr};
+  if ((L.z.serial || colour < 0) && serial_smem<T>(L.z) <= kSerialSmem) return launch_serial<T>(c, L, v, xr, xw, colour, flags);
+  const unsigned nb = nblocks((long long)ncol << L.z.lwl, kColThreads);
+  if (colour < 0 || L.z.serial)  // columns too long for shared memory
+    return launch_chain(c, "k_zlong", colour < 0 ? k_zlong<T, true> : k_zlong<T, false>, nb, kColThreads, 0, L.z, op, v.b,
+                        xr, xw, colour, flags, T(kJacobiOmega));
+#define VFS_PASS(S)                                                                                                \
+  case S:                                                                                                          \
+    return L.z.ls == 32 ? launch_chain(c, "k_zcol", k_zcol<T, S, true>, nb, kColThreads, 0, L.z, op, v.b, xw, colour, flags) \
+                        : launch_chain(c, "k_zcol", k_zcol<T, S, false>, nb, kColThreads, 0, L.z, op, v.b, xw, colour, flags);
+  switch (L.z.seg) {
+    VFS_PASS(1) VFS_PASS(2) VFS_PASS(3) VFS_PASS(4) VFS_PASS(5) VFS_PASS(6) VFS_PASS(7) VFS_PASS(8)
+    default: break;
+  }
+#undef VFS_PASS
+  return launch_chain(c, "k_zcol", k_zcol<T, 0, false>, nb, kColThreads, 0, L.z, op, v.b, xw, colour, flags);
 }
 
 // `sweeps` smoothing sweeps on level l; x_zero: x is taken as zero on entry.
 template <typename T>
-static int mg_smooth(Ctx *c, int l, int sweeps, bool x_zero) {
+static int mg_smooth(const VCycle<T> &V, int l, int sweeps, bool x_zero) {
+  Ctx *c = V.c;
   const MGLevel &L = c->ps.lv[l];
-  const LvT<T> v = lvt<T>(L);
-  const long long half = (long long)L.z.nz * L.z.hx;
+  const LvT<T> v = V.lvt(l);
   int rc = VFS_OK;
-  for (int s = 0; s < sweeps; s++) {
-    const bool z = x_zero && s == 0;
-    if (L.zebra) {
+  if (L.zebra) {
+    for (int s = 0; s < sweeps; s++)
       for (int col = 0; col < 2; col++) {
-        const int xz = (z && col == 0) ? 1 : 0;
-        if (!launch_zline_tile<T>(c, L, v, col, xz, rc)) {
-          c->launches++, k_zline<T><<<nblocks(half, 64), 64, 0, c->stream>>>(L.z, v.cpl, v.tri, v.b, v.x, v.ds, v.x, col, T(1), xz);
-          rc = check_launch(c, "k_zline");
-        }
-        if (rc) return rc;
+        const bool z = x_zero && s == 0;
+        const int flags = (z ? Z_OWN_ZERO : 0) | (z && col == 0 ? Z_NB_ZERO : 0);
+        if ((rc = launch_pass<T>(c, L, v, v.x, v.x, col, flags))) return rc;
       }
-    } else {
-      if (!z) cudaMemcpyAsync(v.xo, v.x, sizeof(T) * L.z.n, cudaMemcpyDeviceToDevice, c->stream);
-      c->launches++, k_zline<T><<<nblocks(2 * half, 64), 64, 0, c->stream>>>(L.z, v.cpl, v.tri, v.b, v.xo, v.ds, v.x, -1,
-                                                               T(kJacobiOmega), z ? 1 : 0);
-      if ((rc = check_launch(c, "k_zline"))) return rc;
-    }
+    return rc;
   }
+  T *from = x_zero ? v.xo : v.x, *to = x_zero ? v.x : v.xo;  // from zero nothing is read
+  for (int s = 0; s < sweeps; s++) {
+    if ((rc = launch_pass<T>(c, L, v, from, to, -1, x_zero && s == 0 ? Z_NB_ZERO | Z_OWN_ZERO : 0))) return rc;
+    std::swap(from, to);
+  }
+  if (from != v.x && cudaMemcpyAsync(v.x, from, sizeof(T) * L.z.n, cudaMemcpyDeviceToDevice, c->stream) != cudaSuccess)
+    return set_err(c, VFS_ERR_CUDA, "multigrid: copy failed");
   return rc;
 }
 
+// Shared memory of the bottom kernel from level l (x, b, the previous x and the operator of every level).
 template <typename T>
-static int mg_bottom(Ctx *c, int l, int nl, const vfs_solve_opts &o) {
+static size_t bottom_smem(const VCycle<T> &V, int l) {
+  long long n = 0;
+  for (int q = l; q < V.nl; q++) n += V.c->ps.lv[q].z.n;
+  return sizeof(T) * 10 * (size_t)n;
+}
+template <typename T>
+static bool bottom_fits(const VCycle<T> &V, int l) {
+  const ZL &z = V.c->ps.lv[l].z;
+  return (long long)z.nx * z.ny * z.nz <= kSerialCells && V.nl - l <= kBottomMaxLevels &&
+         bottom_smem<T>(V, l) <= kBottomSmem;
+}
+template <typename T>
+static int mg_bottom(const VCycle<T> &V, int l) {
+  Ctx *c = V.c;
   Bottom<T> B;
-  B.nl = nl - l;
-  if (B.nl > kBottomMaxLevels) return set_err(c, VFS_ERR_INVALID, "multigrid: too many levels");
-  B.pre = o.pre_smooth; B.post = o.post_smooth; B.coarse = o.coarse_iters;
+  B.nl = V.nl - l;
+  B.pre = V.o.pre_smooth; B.post = V.o.post_smooth; B.coarse = V.o.coarse_iters;
   B.omega = T(kJacobiOmega);
+  const LvT<T> top = V.lvt(l);
+  B.x = top.x;
+  B.b = top.b;
+  unsigned at = 0;
   for (int q = 0; q < B.nl; q++) {
     const MGLevel &L = c->ps.lv[l + q];
-    const LvT<T> v = lvt<T>(L);
+    const LvT<T> v = V.lvt(l + q);
     BLevel<T> &d = B.lv[q];
     d.z = L.z;
-    d.act = L.act;
-    d.cpl = v.cpl; d.tri = v.tri;
-    d.x = v.x; d.b = v.b; d.xo = v.xo; d.ds = v.ds;
+    d.pmask = L.pmask;
+    d.cpl = v.cpl; d.tri = v.tri; d.cpr = v.cpr; d.dg = v.dg;
+    d.sm = at;
+    at += 10u * (unsigned)L.z.n;
     d.zebra = L.zebra ? 1 : 0;
   }
-  return launch_chain(c, "k_mg_bottom", k_mg_bottom<T>, dim3(1), dim3(kBottomThreads), 0, B);
+  const size_t smem = bottom_smem<T>(V, l);
+  // the shared-memory limit is an attribute of the kernel on a device
+  if (smem > 48 * 1024 &&
+      cudaFuncSetAttribute(k_mg_bottom<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBottomSmem) != cudaSuccess)
+    return set_err(c, VFS_ERR_CUDA, "k_mg_bottom: shared-memory limit");
+  return launch_chain(c, "k_mg_bottom", k_mg_bottom<T>, 1, kBottomThreads, smem, B);
 }
 
 // V-cycle from level l (its right-hand side already in place); levels at or below
-// kBottomCells run inside one thread block.
-#ifndef VFS_PROLONG8
-#define VFS_PROLONG8 1
-#endif
+// kSerialCells run inside one thread block.
 template <typename T>
-static int mg_vcycle(Ctx *c, int l, int nl, const vfs_solve_opts &o) {
+static int mg_vcycle(const VCycle<T> &V, int l) {
+  Ctx *c = V.c;
   int rc;
-  const MGLevel &Lv = c->ps.lv[l];
-  if ((long long)Lv.z.nx * Lv.z.ny * Lv.z.nz <= kBottomCells) return mg_bottom<T>(c, l, nl, o);
-  if (l == nl - 1) return mg_smooth<T>(c, l, o.coarse_iters, true);
-  if ((rc = mg_smooth<T>(c, l, o.pre_smooth, true))) return rc;
+  if (bottom_fits<T>(V, l)) return mg_bottom<T>(V, l);
+  if (l == V.nl - 1) return mg_smooth<T>(V, l, V.o.coarse_iters, true);
+  if ((rc = mg_smooth<T>(V, l, V.o.pre_smooth, true))) return rc;
   const MGLevel &F = c->ps.lv[l], &C = c->ps.lv[l + 1];
-  const long long nc = (long long)C.z.nx * C.z.ny * C.z.nz, nf = (long long)F.z.nx * F.z.ny * F.z.nz;
-  const LvT<T> f = lvt<T>(F), cc = lvt<T>(C);
-  // the pre-smoothing ends with a colour-1 pass: on a zebra level without periodic j only
-  // the colour-0 residuals are left
-  if (F.zebra && !F.z.jp)
-    rc = launch_chain(c, "k_zrestrict", k_zrestrict<T, true>, dim3(nblocks(nc, 128)), dim3(128), 0, F.z, C.z, f.cpl,
-                      f.tri, f.x, f.b, cc.b);
-  else
-    rc = launch_chain(c, "k_zrestrict", k_zrestrict<T, false>, dim3(nblocks(nc, 128)), dim3(128), 0, F.z, C.z, f.cpl,
-                      f.tri, f.x, f.b, cc.b);
+  const LvT<T> f = V.lvt(l), cc = V.lvt(l + 1);
+  const unsigned nb = nblocks(C.z.n, 128);
+  // one colour of a zebra level without periodic j is enough for either transfer
+  const bool half = F.zebra && !F.z.jp;
+  rc = colour0_restriction(F.z, F.zebra) ? launch_chain(c, "k_zrestrict", k_zrestrict<T, true>, nb, 128, 0, F.z, C.z, f.cpl, f.tri, f.dg, f.x, f.b, cc.b)
+            : launch_chain(c, "k_zrestrict", k_zrestrict<T, false>, nb, 128, 0, F.z, C.z, f.cpl, f.tri, f.dg, f.x, f.b, cc.b);
   if (rc) return rc;
-  if ((rc = mg_vcycle<T>(c, l + 1, nl, o))) return rc;
-  if (VFS_PROLONG8 && F.z.nx == 2 * C.z.nx && F.z.ny == 2 * C.z.ny && F.z.nz == 2 * C.z.nz)
-    rc = launch_chain(c, "k_zprolong8", k_zprolong8<T>, dim3(nblocks(nc, 128)), dim3(128), 0, F.z, C.z, F.act,
-                      C.act, f.x, cc.x);
-  else
-    rc = launch_chain(c, "k_zprolong", k_zprolong<T>, dim3(nblocks(nf, 256)), dim3(256), 0, F.z, C.z, F.act,
-                      C.act, f.x, cc.x);
+  if ((rc = mg_vcycle<T>(V, l + 1))) return rc;
+  rc = half && V.o.post_smooth > 0
+           ? launch_chain(c, "k_zprolong", k_zprolong<T, true>, nb, 128, 0, F.z, C.z, C.pmask, f.x, cc.x)
+           : launch_chain(c, "k_zprolong", k_zprolong<T, false>, nb, 128, 0, F.z, C.z, C.pmask, f.x, cc.x);
   if (rc) return rc;
-  return mg_smooth<T>(c, l, o.post_smooth, false);
+  return mg_smooth<T>(V, l, V.o.post_smooth, false);
 }
 
-template <typename T, typename VT = double>
-static int mg_apply(Ctx *c, const VT *v, VT *z, const vfs_solve_opts &o, const int *jslot = nullptr,
-                    long long ldv = 0) {
-  Poisson &P = c->ps;
-  const MGLevel &L0 = P.lv[0];
-  const long long ncell = (long long)L0.z.nx * L0.z.ny * L0.z.nz;
-  const LvT<T> l0 = lvt<T>(L0);
+template <typename T, typename VT>
+static int mg_apply(Ctx *c, DynPtrT<const VT> b, DynPtrT<T> x, const vfs_solve_opts &o) {
+  const int nl = o.levels > 0 ? std::min((int)c->ps.lv.size(), o.levels) : (int)c->ps.lv.size();
+  const VCycle<T> V{c, o, nl};
+  const ZL &L = c->ps.lv[0].z;
+  const LvT<T> l0 = V.lvt(0);
+  const size_t smem = tile_bytes<T>(L);
+  const bool tiled = smem <= kTileSmem;
+  const unsigned nt = tiles_i(L) * (unsigned)L.nz, nd = nblocks(L.n, 256);
   int rc;
-  if ((rc = launch_chain(c, "k_to_zebra", k_to_zebra<T, VT>, dim3(nblocks(ncell, 256)), dim3(256), 0, c->g, L0.z, v,
-                         jslot, ldv, l0.b)))
-    return rc;
-  const int nl = o.levels > 0 ? std::min((int)P.lv.size(), o.levels) : (int)P.lv.size();
-  if ((rc = mg_vcycle<T>(c, 0, nl, o))) return rc;
-  return launch_chain(c, "k_from_zebra", k_from_zebra<T, VT>, dim3(nblocks(c->g.N, 256)), dim3(256), 0, c->g, L0.z,
-                      P.fluid, l0.x, jslot, ldv, z);
+  // the shared-memory limit is an attribute of the kernel on a device
+  if (tiled && smem > 48 * 1024 &&
+      (cudaFuncSetAttribute(k_to_columns<T, VT>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem) != cudaSuccess ||
+       cudaFuncSetAttribute(k_from_columns<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem) != cudaSuccess))
+    return set_err(c, VFS_ERR_CUDA, "multigrid: shared-memory limit");
+  rc = tiled ? launch_chain(c, "k_to_columns", k_to_columns<T, VT>, nt, 256, smem, c->g, L, b, l0.b)
+             : launch_chain(c, "k_to_columns", k_to_columns_direct<T, VT>, nd, 256, 0, c->g, L, b, l0.b);
+  if (rc || (rc = mg_vcycle<T>(V, 0))) return rc;
+  return tiled ? launch_chain(c, "k_from_columns", k_from_columns<T>, nt, 256, smem, c->g, L, l0.x, x)
+               : launch_chain(c, "k_from_columns", k_from_columns_direct<T>, nd, 256, 0, c->g, L, l0.x, x);
 }
 
-// z = M^-1 v: one V-cycle in FP32 (precision 0) or FP64.
-int mg_precondition(Ctx *c, const double *v, double *z, const vfs_solve_opts &o) {
-  return o.precision != 1 ? mg_apply<float>(c, v, z, o) : mg_apply<double>(c, v, z, o);
-}
-
-// z_j = M^-1 v_j with v_j = V + j ldv, z_j = Z + j ldv and j read on the device (*jslot).
-int mg_precondition_dyn(Ctx *c, const double *V, double *Z, long long ldv, const int *jslot, const vfs_solve_opts &o) {
-  return o.precision != 1 ? mg_apply<float>(c, V, Z, o, jslot, ldv) : mg_apply<double>(c, V, Z, o, jslot, ldv);
-}
-
-// The same with FP32 vectors (the FP32 inner Krylov of precision 2): an FP32 V-cycle.
-int mg_precondition_dyn32(Ctx *c, const float *V, float *Z, long long ldv, const int *jslot, const vfs_solve_opts &o) {
-  return mg_apply<float, float>(c, V, Z, o, jslot, ldv);
-}
+int mg_precondition(Ctx *c, DynPtrT<const double> b, DynPtrT<float> x, const vfs_solve_opts &o) { return mg_apply<float>(c, b, x, o); }
+int mg_precondition(Ctx *c, DynPtrT<const double> b, DynPtrT<double> x, const vfs_solve_opts &o) { return mg_apply<double>(c, b, x, o); }
+int mg_precondition(Ctx *c, DynPtrT<const float> b, DynPtrT<float> x, const vfs_solve_opts &o) { return mg_apply<float>(c, b, x, o); }
 
 // One smoothing sweep of the finest level (both colours), for timing.
 int mg_sweep_fine(Ctx *c, int precision) {
-  return precision == 0 ? mg_smooth<float>(c, 0, 1, false) : mg_smooth<double>(c, 0, 1, false);
+  const vfs_solve_opts o = {};
+  return precision == 0 ? mg_smooth<float>(VCycle<float>{c, o, 1}, 0, 1, false) : mg_smooth<double>(VCycle<double>{c, o, 1}, 0, 1, false);
 }
 
 }  // namespace vfs

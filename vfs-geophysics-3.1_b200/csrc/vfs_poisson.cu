@@ -124,7 +124,7 @@ __global__ void k_poisson_coef(Grid g, Metrics m, const uint8_t *__restrict__ nv
   const int mx = g.mx, my = g.my, mz = g.mz;
   int i, j, k;
   dijk(g, p, i, j, k);
-  const long long N = g.N;
+  const long long N = vec_ld(g.N);
   const bool interior = !(i == 0 || i == mx - 1 || j == 0 || j == my - 1 || k == 0 || k == mz - 1);
   if (!interior || nv[p] != 0) {
     for (int s = 0; s < NSLOT; s++) coef[s * N + p] = 0;
@@ -204,21 +204,27 @@ __device__ __forceinline__ long long nb_index(const Grid &g, int i, int j, int k
 // (A x)[p] on the grid layout from the first NS stencil slots: NS = 7 when every cross
 // slot of the operator is zero (orthogonal grids), else 19.  A skipped slot is zero, so
 // both forms give the same sums.  Rows of non-unknowns are all zero.
-template <int NS>
+// Every load is issued before the first coefficient is tested (testing first made each x load
+// wait for its coefficient: 237 us an apply at 256 x 192 x 256); an x under a zero coefficient
+// is loaded and left out.
+template <int NS, typename XT>
 __device__ __forceinline__ double apply_row64(const Grid &g, const double *__restrict__ coef,
-                                              const double *__restrict__ x, long long p) {
-  // 32-bit index arithmetic (grids below 2^31 points)
-  const unsigned up = (unsigned)p, umx = (unsigned)g.mx, umy = (unsigned)g.my;
-  const unsigned q = up / umx;
-  const int i = (int)(up - q * umx);
-  const unsigned kk = q / umy;
-  const int j = (int)(q - kk * umy), k = (int)kk;
-  double s = 0;
+                                              const XT *__restrict__ x, long long p) {
+  const long long ld = vec_ld(g.N);
+  int i, j, k;
+  dijk(g, p, i, j, k);
+  if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return 0.0;
+  double cf[NS];
+  XT xv[NS];
 #pragma unroll
   for (int t = 0; t < NS; t++) {
-    const double c = coef[t * g.N + p];
-    if (c != 0.0) s += c * x[nb_index(g, i, j, k, t)];
+    cf[t] = __ldcs(coef + t * ld + p);
+    xv[t] = x[nb_index(g, i, j, k, t)];
   }
+  double s = 0;
+#pragma unroll
+  for (int t = 0; t < NS; t++)
+    if (cf[t] != 0.0) s += cf[t] * (double)xv[t];
   return s;
 }
 
@@ -231,18 +237,33 @@ __global__ void k_apply(Grid g, const double *__restrict__ coef, const double *_
   y[p] = apply_row64<NS>(g, coef, x, p);
 }
 
-// y = A^T x: every stencil entry of row p scattered onto its neighbour (atomics).
-__global__ void k_apply_t(Grid g, int ns, const double *__restrict__ coef, const double *__restrict__ x, double *y) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  const double xp = x[p];
-  if (xp == 0.0) return;
+// The slot that points back: c_off[opposite(t)] = -c_off[t].
+__device__ __forceinline__ constexpr int opposite(int t) {
+  constexpr int o[NSLOT] = {CP, WP, EP, SP, NP, BP, TP, SW, NW, SE, NE, BS, TS, BN, TN, BW, TW, BE, TE};
+  return o[t];
+}
+// (A^T x)[p]: the entry of every neighbour's row that names p (a gather, so the sum is the
+// same in every run; scattering with atomics needed a cleared result and its own pass).
+// Ghost points have no row: their entries are zero.
+template <int NS, typename XT>
+__device__ __forceinline__ double apply_row64_t(const Grid &g, const double *__restrict__ coef,
+                                                const XT *__restrict__ x, long long p) {
+  const long long ld = vec_ld(g.N);
   int i, j, k;
   dijk(g, p, i, j, k);
-  for (int t = 0; t < ns; t++) {
-    const double c = coef[t * g.N + p];
-    if (c != 0.0) atomicAdd(y + nb_index(g, i, j, k, t), c * xp);
+  if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return 0.0;
+  double s = 0;
+#pragma unroll
+  for (int t = 0; t < NS; t++) {
+    const long long q = nb_index(g, i, j, k, t);
+    s += coef[opposite(t) * ld + q] * (double)x[q];
   }
+  return s;
+}
+template <int NS, bool kT, typename XT>
+__device__ __forceinline__ double op_row(const Grid &g, const double *__restrict__ coef, const XT *__restrict__ x,
+                                         long long p) {
+  return kT ? apply_row64_t<NS>(g, coef, x, p) : apply_row64<NS>(g, coef, x, p);
 }
 
 int poisson_set_transpose(Ctx *c, bool on) {
@@ -251,11 +272,6 @@ int poisson_set_transpose(Ctx *c, bool on) {
 }
 
 int poisson_apply_dev(Ctx *c, const double *x, double *y) {
-  if (c->ps.transpose) {
-    cudaMemsetAsync(y, 0, sizeof(double) * c->g.N, c->stream);
-    c->launches++, k_apply_t<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, c->ps.nslot, c->ps.coef, x, y);
-    return check_launch(c, "k_apply_t");
-  }
   if (c->ps.nslot == 7) c->launches++, k_apply<7><<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, c->ps.coef, x, y);
   else c->launches++, k_apply<NSLOT><<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, c->ps.coef, x, y);
   return check_launch(c, "k_apply");
@@ -276,11 +292,11 @@ int poisson_apply_dev(Ctx *c, const double *x, double *y) {
 #endif
 static const int kKryBlocks = 148 * VFS_KRY_BLOCKS_PER_SM;
 // Blocks of the basis passes: a fixed multiple of the SM count, grid-stride (one point
-// pair per thread over the whole vector measured 7 % slower per step on the B200).
-static const int kKryThreads = 256;
+// pair per thread over the whole vector measured 7 % slower per step on the B200), no more
+// than there are pairs.
+static constexpr int kKryThreads = 256;
 static int kry_grid(const Ctx *c) {
-  (void)c;
-  return kKryBlocks;
+  return (int)std::max<long long>(1, std::min<long long>(kKryBlocks, nblocks(c->g.N >> 1, kKryThreads)));
 }
 
 // Block sums of rows 0..nv-1 and of row NV (stored as row nv) of acc into
@@ -306,18 +322,75 @@ __device__ __forceinline__ void block_sums(const double (&acc)[NV + 1], int nv, 
   }
 }
 
+// True in every thread of the block that is the last of the grid to get here: the partial sums
+// stored by all blocks before the call are then visible to it.  Leaves the ticket at zero.
+__device__ __forceinline__ bool last_block(unsigned *ticket) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    if (last) *ticket = 0;
+  }
+  __syncthreads();
+  if (last) __threadfence();
+  return last;
+}
+// out[r] = the sum of the ncols partials of row r for r < nrows, by one block of kKryThreads threads
+// in the order of a strided sum per thread and a tree over the threads; sixteen rows at a time
+// share the barriers of the tree.
+__device__ __forceinline__ void sum_rows(const double *parts, int nrows, int ncols, double *out) {
+  constexpr int R = 16;
+  __shared__ double sh[R][kKryThreads / 2];
+  const int tid = threadIdx.x;
+  for (int r0 = 0; r0 < nrows; r0 += R) {
+    double s[R];
+#pragma unroll
+    for (int u = 0; u < R; u++) s[u] = 0;
+    for (int t = tid; t < ncols; t += kKryThreads)
+#pragma unroll
+      for (int u = 0; u < R; u++)
+        if (r0 + u < nrows) s[u] += __ldcg(parts + (long long)(r0 + u) * ncols + t);
+    // tree over the threads: w = 128, 64, 32 through shared memory, then one warp a row
+#pragma unroll
+    for (int w = kKryThreads / 2; w >= 32; w >>= 1) {
+      if (tid >= w && tid < 2 * w)
+#pragma unroll
+        for (int u = 0; u < R; u++) sh[u][tid - w] = s[u];
+      __syncthreads();
+      if (tid < w)
+#pragma unroll
+        for (int u = 0; u < R; u++) s[u] += sh[u][tid];
+      __syncthreads();
+    }
+    if (tid < 32) {
+#pragma unroll
+      for (int u = 0; u < R; u++) sh[u][tid] = s[u];
+    }
+    __syncthreads();
+    const int lane = tid & 31;
+    for (int u = tid >> 5; u < R; u += kKryThreads / 32) {
+      double v = sh[u][lane];
+#pragma unroll
+      for (int w = 16; w > 0; w >>= 1) v += __shfl_down_sync(0xffffffffu, v, w);
+      if (lane == 0 && r0 + u < nrows) out[r0 + u] = v;
+    }
+    __syncthreads();
+  }
+}
+
 // The Krylov kernels below stream the basis two points at a time (16-byte loads): the
 // basis vectors are stored ldv apart, ldv a multiple of 32, and every other vector is a
 // separate allocation, so pair loads are aligned; an odd last point is done alone.
 
 static const int kRedBlocks = 148 * 2;
 // Number of non-zero cross-derivative slots (7..18) of the operator.
-__global__ void k_count_cross(long long N, const double *__restrict__ coef, double *parts) {
+__global__ void k_count_cross(long long N, long long ld, const double *__restrict__ coef, double *parts) {
   __shared__ double sh[256];
   double s = 0;
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < N; p += stride)
-    for (int t = NE; t < NSLOT; t++) s += coef[t * N + p] != 0.0 ? 1.0 : 0.0;
+    for (int t = NE; t < NSLOT; t++) s += coef[t * ld + p] != 0.0 ? 1.0 : 0.0;
   sh[threadIdx.x] = s;
   __syncthreads();
   for (int w = blockDim.x / 2; w > 0; w >>= 1) {
@@ -349,7 +422,7 @@ int poisson_lhs(Ctx *c) {
   const long long N = g.N;
   int rc;
   if (!P.coef) {
-    bool ok = cudaMalloc(&P.coef, sizeof(double) * NSLOT * N) == cudaSuccess;
+    bool ok = cudaMalloc(&P.coef, sizeof(double) * NSLOT * vec_ld(N)) == cudaSuccess;
     ok &= cudaMalloc(&P.fluid, N) == cudaSuccess;
     ok &= cudaMalloc(&P.w, sizeof(double) * N) == cudaSuccess;
     ok &= cudaMalloc(&P.r, sizeof(double) * N) == cudaSuccess;
@@ -371,7 +444,7 @@ int poisson_lhs(Ctx *c) {
   P.nfluid = (long long)llround(cnt);
   P.sum_aj = saj;
   // the apply reads only slots CP..BP when no row has a cross-derivative entry
-  c->launches++, k_count_cross<<<kRedBlocks, 256, 0, c->stream>>>(N, P.coef, c->red);
+  c->launches++, k_count_cross<<<kRedBlocks, 256, 0, c->stream>>>(N, vec_ld(N), P.coef, c->red);
   if ((rc = check_launch(c, "k_count_cross"))) return rc;
   double ncross = 0;
   if ((rc = reduce_sum(c, c->red, kRedBlocks, &ncross))) return rc;
@@ -539,17 +612,6 @@ struct Guard {
 __device__ __forceinline__ bool guard_off(const Guard &q) { return q.flag && ((*q.flag != 0) != (q.want != 0)); }
 static Guard always() { return Guard{nullptr, 0}; }
 
-// base + (*j + off) * ldv (base when j is null).
-template <typename B>
-struct DynPtrT {
-  B *base;
-  long long ldv;
-  const int *j;
-  int off;
-  __device__ __forceinline__ B *get() const { return j ? base + (long long)(*j + off) * ldv : base; }
-};
-using DynPtr = DynPtrT<double>;
-
 // Two consecutive basis entries as FP64 (the FP32 basis of precision 2 is widened on load
 // and rounded on store; every sum and product is FP64).
 __device__ __forceinline__ double2 ld2(const double *__restrict__ p, long long i) {
@@ -571,54 +633,120 @@ __device__ __forceinline__ void set_cond(unsigned long long h, int use, int v) {
   if (use) cudaGraphSetConditional((cudaGraphConditionalHandle)h, v ? 1u : 0u);
 }
 
-template <int NS>
-__global__ void k_apply_dyn(Grid g, const double *__restrict__ coef, DynPtr x, double *__restrict__ y) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  y[p] = apply_row64<NS>(g, coef, x.get(), p);
-}
-// The inner operator of precision 2: FP32 vectors, the FP64 coefficients, FP64 products and
-// sum, the result rounded to FP32 (FP32 coefficients measured 20-40 % more iterations:
-// iterative refinement converges at the rate of the inner operator's error).
-template <int NS>
-__global__ void k_apply32_dyn(Grid g, const double *__restrict__ coef, DynPtrT<float> xp, float *__restrict__ y) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  const float *__restrict__ x = xp.get();
-  const unsigned up = (unsigned)p, umx = (unsigned)g.mx, umy = (unsigned)g.my;
-  const unsigned q = up / umx;
-  const int i = (int)(up - q * umx);
-  const unsigned kk = q / umy;
-  const int j = (int)(q - kk * umy), k = (int)kk;
-  double s = 0.0;
-#pragma unroll
-  for (int t = 0; t < NS; t++) {
-    const double c = coef[t * g.N + p];
-    if (c != 0.0) s += c * (double)x[nb_index(g, i, j, k, t)];
+// ---- control steps (the first warp of the last block of a pass).  The column and the rotations
+// are staged in shared memory by the lanes; the sums and the recurrence, whose order is
+// fixed, run in lane 0 (reading them from global memory between its stores cost a round trip
+// to L2 per entry: 12 us a Hessenberg column at 15 columns on average).
+// After h = V^T w and h[nv] = <w, w>: one Gram-Schmidt pass, or re-orthogonalise.
+__device__ __forceinline__ void kry_ctl_a(KryDev *kd) {
+  __shared__ double sh[kKryMax + 3];
+  __shared__ int again;
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x, j = kd->j, nv = j + 1, m = kd->m;
+  for (int t = lane; t <= nv; t += 32) sh[t] = kd->h[t];
+  __syncwarp();
+  if (lane == 0) {
+    double proj0 = 0;
+    for (int t = 0; t < nv; t++) proj0 += sh[t] * sh[t];
+    const double hn2_0 = sh[nv] - proj0;  // |w - V h|^2 for orthonormal V
+    const bool one = hn2_0 > 0.5 * sh[nv];
+    kd->degen = 0;
+    kd->reorth = one ? 0 : 1;
+    if (one) {
+      const double hn = sqrt(hn2_0);
+      kd->hn = hn;
+      kd->scale = 1.0 / hn;
+    }
+    again = one ? 0 : 1;
   }
-  y[p] = (float)s;
+  __syncwarp();
+  if (!again)
+    for (int t = lane; t < nv; t += 32) kd->H[t * m + j] = sh[t];
 }
-__global__ void k_apply_t_dyn(Grid g, int ns, const double *__restrict__ coef, DynPtr x, double *y, Guard q) {
-  if (guard_off(q)) return;
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  const double xp = x.get()[p];
-  if (xp == 0.0) return;
-  int i, j, k;
-  dijk(g, p, i, j, k);
-  for (int t = 0; t < ns; t++) {
-    const double c = coef[t * g.N + p];
-    if (c != 0.0) atomicAdd(y + nb_index(g, i, j, k, t), c * xp);
+// After w -= V h and h2 = V^T w: the second pass.
+__device__ __forceinline__ void kry_ctl_b(KryDev *kd) {
+  __shared__ double sh[kKryMax + 3];
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x, j = kd->j, nv = j + 1, m = kd->m;
+  for (int t = lane; t <= nv; t += 32) sh[t] = kd->h2[t];
+  for (int t = lane; t < nv; t += 32) kd->H[t * m + j] = kd->h[t] + kd->h2[t];
+  __syncwarp();
+  if (lane == 0) {
+    const double ww = sh[nv];
+    double proj = 0;
+    for (int t = 0; t < nv; t++) proj += sh[t] * sh[t];
+    const double hn2 = ww - proj;  // |w - V h2|^2 for orthonormal V
+    const bool ok = hn2 > 1e-4 * ww;
+    kd->degen = ok ? 0 : 1;  // w nearly in span(V): form w - V h2 and take its norm
+    if (ok) {
+      const double hn = sqrt(hn2);
+      kd->hn = hn;
+      kd->scale = 1.0 / hn;
+    }
   }
 }
-__global__ void k_zero_g(long long n, double *y, Guard q) {
-  if (guard_off(q)) return;
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p < n) y[p] = 0.0;
+// After the explicit w -= V h2 (degenerate case).
+__device__ __forceinline__ void kry_ctl_c(KryDev *kd) {
+  if (threadIdx.x == 0) {
+    const int nv = kd->j + 1;
+    kd->hn = sqrt(fmax(kd->h3[nv], 0.0));
+    kd->scale = kd->hn > 0 ? 1.0 / kd->hn : 0.0;
+  }
+  __syncwarp();
+}
+// Hessenberg column j: Givens rotations, residual estimate, loop control.
+__device__ __forceinline__ void kry_givens(KryDev *kd, unsigned long long h_inner, int use_graph) {
+  __shared__ double col[kKryMax + 1], cs[kKryMax], sn[kKryMax];
+  if (threadIdx.x >= 32) return;
+  const int lane = threadIdx.x, j = kd->j, m = kd->m;
+  for (int t = lane; t <= j; t += 32) col[t] = kd->H[t * m + j];
+  for (int t = lane; t < j; t += 32) { cs[t] = kd->cs[t]; sn[t] = kd->sn[t]; }
+  const double hn = kd->hn, g = kd->gv[j], tol = kd->tol, inner_tol = kd->inner_rtol * kd->beta;
+  const int it = kd->it + 1, maxit = kd->maxit;
+  __syncwarp();
+  if (lane == 0) {
+    double a = col[0];
+    for (int t = 0; t < j; t++) {
+      const double bb = col[t + 1];
+      col[t] = cs[t] * a + sn[t] * bb;
+      a = -sn[t] * a + cs[t] * bb;
+    }
+    const double den = sqrt(a * a + hn * hn);
+    const double c = den > 0 ? a / den : 1.0, s = den > 0 ? hn / den : 0.0;
+    col[j] = den;
+    const double g1 = -s * g, rnorm = fabs(g1);
+    kd->cs[j] = c;
+    kd->sn[j] = s;
+    kd->gv[j + 1] = g1;
+    kd->gv[j] = c * g;
+    kd->it = it;
+    kd->jdone = j + 1;
+    kd->rnorm = rnorm;
+    // precision 2 also ends the cycle (an iterative-refinement sweep) once the FP32 Arnoldi
+    // estimate has fallen by inner_rtol; the next cycle restarts from the FP64 residual
+    const bool stop = rnorm <= tol || hn == 0 || rnorm <= inner_tol;
+    const int go = !stop && j + 1 < m && it < maxit;
+    kd->j = j + 1;
+    kd->inner_go = go;
+    set_cond(h_inner, use_graph, go);
+  }
+  __syncwarp();
+  for (int t = lane; t <= j; t += 32) kd->H[t * m + j] = col[t];
 }
 
-// <V_t, w> (t < nv) and <w, w> with nv = j + 1 from the device state (B: the basis type,
-// FP64, or FP32 for precision 2; the sums are FP64).
+// w = A z_j.  The rows are FP64 sums of FP64 coefficients whatever the vectors' types (precision
+// 2: FP32 coefficients measured 20-40 % more iterations, since iterative refinement converges
+// at the rate of the inner operator's error), rounded to w's type.
+template <int NS, bool kT, typename B, typename ZT>
+__global__ void __launch_bounds__(256) k_apply_dyn(Grid g, long long ldv, const double *__restrict__ coef,
+                                                   const ZT *__restrict__ Z, const KryDev *__restrict__ kd,
+                                                   B *__restrict__ w) {
+  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (p >= g.N) return;
+  w[p] = (B)op_row<NS, kT>(g, coef, Z + (long long)kd->j * ldv, p);
+}
+
+// h_t = <V_t, w> (t <= j) and <w, w>, and the first Gram-Schmidt decision.
 template <int NV, typename B>
 __device__ __forceinline__ void multidot_body(long long N, long long ldv, const B *__restrict__ V, int nv,
                                               const B *__restrict__ w, double *__restrict__ parts) {
@@ -649,19 +777,20 @@ __device__ __forceinline__ void multidot_body(long long N, long long ldv, const 
   block_sums<NV>(acc, nv, parts);
 }
 template <typename B>
-__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_multidot_dyn(long long N, long long ldv,
-                                                                             const B *__restrict__ V,
-                                                                             const KryDev *__restrict__ kd,
-                                                                             const B *__restrict__ w,
-                                                                             double *__restrict__ parts) {
+__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_multidot(long long N, long long ldv,
+                                                                         const B *__restrict__ V, KryDev *kd,
+                                                                         const B *__restrict__ w, double *parts) {
   const int nv = kd->j + 1;
   if (nv <= 4) multidot_body<4>(N, ldv, V, nv, w, parts);
   else if (nv <= 8) multidot_body<8>(N, ldv, V, nv, w, parts);
   else if (nv <= 16) multidot_body<16>(N, ldv, V, nv, w, parts);
   else multidot_body<32>(N, ldv, V, nv, w, parts);
+  if (!last_block(&kd->ticket)) return;
+  sum_rows(parts, nv + 1, gridDim.x, kd->h);
+  kry_ctl_a(kd);
 }
 
-// w -= sum_t h_t V_t (h = kd->hdev), with <V_t, w> and <w, w> of the result.
+// w -= sum_t h_t V_t, with <V_t, w> and <w, w> of the result.
 template <int NV, typename B>
 __device__ __forceinline__ void update_dots_body(long long N, long long ldv, const B *__restrict__ V, int nv,
                                                  const double *__restrict__ h, B *__restrict__ w,
@@ -702,20 +831,48 @@ __device__ __forceinline__ void update_dots_body(long long N, long long ldv, con
   block_sums<NV>(acc, nv, parts);
 }
 template <typename B>
-__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_update_dots_dyn(long long N, long long ldv,
-                                                                                const B *__restrict__ V,
-                                                                                const KryDev *__restrict__ kd,
-                                                                                B *__restrict__ w,
-                                                                                double *__restrict__ parts, Guard q) {
-  if (guard_off(q)) return;
+__device__ __forceinline__ void update_dots(long long n, long long ldv, const B *__restrict__ V, int nv,
+                                            const double *__restrict__ h, B *__restrict__ w, double *__restrict__ parts) {
+  if (nv <= 4) update_dots_body<4>(n, ldv, V, nv, h, w, parts);
+  else if (nv <= 8) update_dots_body<8>(n, ldv, V, nv, h, w, parts);
+  else if (nv <= 16) update_dots_body<16>(n, ldv, V, nv, h, w, parts);
+  else update_dots_body<32>(n, ldv, V, nv, h, w, parts);
+}
+// The second Gram-Schmidt pass where the first asked for it.
+template <typename B>
+__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_reorth(long long n, long long ldv,
+                                                                       const B *__restrict__ V, KryDev *kd,
+                                                                       B *__restrict__ w, double *parts) {
+  if (!kd->reorth) return;
   const int nv = kd->j + 1;
-  if (nv <= 4) update_dots_body<4>(N, ldv, V, nv, kd->hdev, w, parts);
-  else if (nv <= 8) update_dots_body<8>(N, ldv, V, nv, kd->hdev, w, parts);
-  else if (nv <= 16) update_dots_body<16>(N, ldv, V, nv, kd->hdev, w, parts);
-  else update_dots_body<32>(N, ldv, V, nv, kd->hdev, w, parts);
+  update_dots<B>(n, ldv, V, nv, kd->h, w, parts);
+  if (!last_block(&kd->ticket)) return;
+  sum_rows(parts, nv + 1, gridDim.x, kd->h2);
+  kry_ctl_b(kd);
+}
+// The explicit w - V h2 of the degenerate case, and the Hessenberg column.
+template <typename B>
+__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_hessenberg(long long n, long long ldv,
+                                                                           const B *__restrict__ V, KryDev *kd,
+                                                                           B *__restrict__ w, double *parts,
+                                                                           unsigned long long h_inner, int use_graph) {
+  if (kd->reorth && kd->degen) {
+    const int nv = kd->j + 1;
+    update_dots<B>(n, ldv, V, nv, kd->h2, w, parts);
+    if (!last_block(&kd->ticket)) return;
+    sum_rows(parts, nv + 1, gridDim.x, kd->h3);
+    if (threadIdx.x < 32) {
+      kry_ctl_c(kd);
+      kry_givens(kd, h_inner, use_graph);
+    }
+  } else if (blockIdx.x == 0) {
+    kry_givens(kd, h_inner, use_graph);
+  }
 }
 
-// out = (w - sum_t h_t V_t) * scale (h = kd->hdev, scale = kd->scale).
+// V_{j+1} = (w - sum_t h_t V_t) * scale, with h of the last pass (none in the degenerate case,
+// whose w has been orthogonalised in place), after the Hessenberg step (kd->jdone = j + 1).
+// Not needed when the cycle ends there.
 template <int NV, typename B>
 __device__ __forceinline__ void update_scale_body(long long N, long long ldv, const B *__restrict__ V, int nv,
                                                   const double *__restrict__ h, const B *__restrict__ w,
@@ -745,36 +902,18 @@ __device__ __forceinline__ void update_scale_body(long long N, long long ldv, co
   }
 }
 template <typename B>
-__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_update_scale_dyn(long long N, long long ldv,
-                                                                                 const B *__restrict__ V,
-                                                                                 const KryDev *__restrict__ kd,
-                                                                                 const B *__restrict__ w,
-                                                                                 DynPtrT<B> out, Guard q) {
-  if (guard_off(q)) return;
-  const int nv = kd->j + 1;
-  B *o = out.get();
-  if (nv <= 4) update_scale_body<4>(N, ldv, V, nv, kd->hdev, w, kd->scale, o);
-  else if (nv <= 8) update_scale_body<8>(N, ldv, V, nv, kd->hdev, w, kd->scale, o);
-  else if (nv <= 16) update_scale_body<16>(N, ldv, V, nv, kd->hdev, w, kd->scale, o);
-  else update_scale_body<32>(N, ldv, V, nv, kd->hdev, w, kd->scale, o);
-}
-
-// Rows 0..nrows-1 of the block partials summed in a fixed order; nrows = j + 2 (the nv
-// dot products and the norm) from the device state.
-__global__ void k_sum_rows_dyn(const double *parts, const KryDev *kd, int ncols, double *out, Guard q) {
-  if (guard_off(q)) return;
-  const int r = blockIdx.x;
-  if (r >= kd->j + 2) return;
-  __shared__ double sh[256];
-  double s = 0;
-  for (int t = threadIdx.x; t < ncols; t += blockDim.x) s += parts[(long long)r * ncols + t];
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[r] = sh[0];
+__global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_next_vector(long long N, long long ldv, B *V,
+                                                                            const KryDev *__restrict__ kd,
+                                                                            const B *__restrict__ w) {
+  if (!kd->inner_go) return;
+  const int jd = kd->jdone;
+  B *o = V + (long long)jd * ldv;
+  const int nv = kd->reorth && kd->degen ? 0 : jd;
+  const double *h = kd->reorth ? kd->h2 : kd->h;
+  if (nv <= 4) update_scale_body<4>(N, ldv, V, nv, h, w, kd->scale, o);
+  else if (nv <= 8) update_scale_body<8>(N, ldv, V, nv, h, w, kd->scale, o);
+  else if (nv <= 16) update_scale_body<16>(N, ldv, V, nv, h, w, kd->scale, o);
+  else update_scale_body<32>(N, ldv, V, nv, h, w, kd->scale, o);
 }
 
 // Sum of n partials (one block, fixed order, as k_sum_parts) into out, guarded.
@@ -802,7 +941,7 @@ __global__ void __launch_bounds__(1024) k_sum_parts_g(const double *parts, int n
 }
 
 // r = b - A x with the block sums of <r, r>, guarded.
-template <int NS>
+template <int NS, bool kT>
 __global__ void __launch_bounds__(256) k_residual_g(Grid g, const double *__restrict__ coef,
                                                     const double *__restrict__ b, const double *__restrict__ x,
                                                     double *__restrict__ r, double *__restrict__ parts, Guard q) {
@@ -811,7 +950,7 @@ __global__ void __launch_bounds__(256) k_residual_g(Grid g, const double *__rest
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   double v2 = 0;
   if (p < g.N) {
-    const double v = b[p] - apply_row64<NS>(g, coef, x, p);
+    const double v = b[p] - op_row<NS, kT>(g, coef, x, p);
     r[p] = v;
     v2 = v * v;
   }
@@ -825,25 +964,6 @@ __global__ void __launch_bounds__(256) k_residual_g(Grid g, const double *__rest
     parts[blockIdx.x] = s;
   }
 }
-// r = b - r (r holding A x) and the partial sums of <r, r>, guarded (grid-stride).
-__global__ void k_sub_norm_g(long long n, const double *__restrict__ b, double *r, double *parts, Guard q) {
-  if (guard_off(q)) return;
-  __shared__ double sh[256];
-  double s = 0;
-  for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
-    const double v = b[p] - r[p];
-    r[p] = v;
-    s += v * v;
-  }
-  sh[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) parts[blockIdx.x] = sh[0];
-}
-
 // dst = src * (*scale), guarded (FP64 arithmetic, stored in dst's type).
 template <typename S, typename D>
 __global__ void k_scale_copy_dyn(long long n, const S *__restrict__ src, const double *__restrict__ scale,
@@ -914,87 +1034,23 @@ __global__ void k_kry_cycle(KryDev *kd, unsigned long long h_inner, int use_grap
   }
   set_cond(h_inner, use_graph, kd->inner_go);
 }
-// After h = V^T w and h[nv] = <w, w>: one Gram-Schmidt pass, or re-orthogonalise.
-__global__ void k_kry_ctl_a(KryDev *kd) {
-  const int j = kd->j, nv = j + 1, m = kd->m;
-  double proj0 = 0;
-  for (int t = 0; t < nv; t++) proj0 += kd->h[t] * kd->h[t];
-  const double hn2_0 = kd->h[nv] - proj0;  // |w - V h|^2 for orthonormal V
-  for (int t = 0; t < nv; t++) kd->hdev[t] = kd->h[t];
-  kd->degen = 0;
-  if (hn2_0 > 0.5 * kd->h[nv]) {
-    for (int t = 0; t < nv; t++) kd->H[t * m + j] = kd->h[t];
-    kd->hn = sqrt(hn2_0);
-    kd->scale = 1.0 / kd->hn;
-    kd->reorth = 0;
-  } else {
-    kd->reorth = 1;
-  }
-}
-// After w -= V h and h2 = V^T w: the second pass.
-__global__ void k_kry_ctl_b(KryDev *kd) {
-  if (!kd->reorth) return;
-  const int j = kd->j, nv = j + 1, m = kd->m;
-  const double ww = kd->h2[nv];
-  double proj = 0;
-  for (int t = 0; t < nv; t++) proj += kd->h2[t] * kd->h2[t];
-  const double hn2 = ww - proj;  // |w - V h2|^2 for orthonormal V
-  for (int t = 0; t < nv; t++) {
-    kd->hdev[t] = kd->h2[t];
-    kd->H[t * m + j] = kd->h[t] + kd->h2[t];
-  }
-  if (hn2 > 1e-4 * ww) {
-    kd->hn = sqrt(hn2);
-    kd->scale = 1.0 / kd->hn;
-    kd->degen = 0;
-  } else {
-    kd->degen = 1;  // w nearly in span(V): form w - V h2 and take its norm
-  }
-}
-// After the explicit w -= V h2 (degenerate case).
-__global__ void k_kry_ctl_c(KryDev *kd) {
-  if (!kd->degen) return;
-  const int nv = kd->j + 1;
-  kd->hn = sqrt(fmax(kd->h3[nv], 0.0));
-  kd->scale = kd->hn > 0 ? 1.0 / kd->hn : 0.0;
-}
-// Hessenberg column j: Givens rotations, residual estimate, loop control.
-__global__ void k_kry_givens(KryDev *kd, unsigned long long h_inner, int use_graph) {
-  const int j = kd->j, m = kd->m;
-  double *H = kd->H;
-  H[(j + 1) * m + j] = kd->hn;
-  for (int t = 0; t < j; t++) {
-    const double a = H[t * m + j], bb = H[(t + 1) * m + j];
-    H[t * m + j] = kd->cs[t] * a + kd->sn[t] * bb;
-    H[(t + 1) * m + j] = -kd->sn[t] * a + kd->cs[t] * bb;
-  }
-  const double a = H[j * m + j], bb = H[(j + 1) * m + j];
-  const double den = sqrt(a * a + bb * bb);
-  kd->cs[j] = den > 0 ? a / den : 1.0;
-  kd->sn[j] = den > 0 ? bb / den : 0.0;
-  H[j * m + j] = den;
-  H[(j + 1) * m + j] = 0;
-  kd->gv[j + 1] = -kd->sn[j] * kd->gv[j];
-  kd->gv[j] = kd->cs[j] * kd->gv[j];
-  kd->it++;
-  kd->jdone = j + 1;
-  kd->rnorm = fabs(kd->gv[j + 1]);
-  // precision 2 also ends the cycle (an iterative-refinement sweep) once the FP32 Arnoldi
-  // estimate has fallen by inner_rtol; the next cycle restarts from the FP64 residual
-  const bool stop = kd->rnorm <= kd->tol || kd->hn == 0 || kd->rnorm <= kd->inner_rtol * kd->beta;
-  kd->j = j + 1;
-  kd->inner_go = !stop && kd->j < m && kd->it < kd->maxit;
-  set_cond(h_inner, use_graph, kd->inner_go);
-}
-// Back substitution (y into hdev for the update) and the test for the true residual.
-__global__ void k_kry_backsub(KryDev *kd) {
+// Back substitution (kd->y) and the test for the true residual; the triangle staged in shared memory.
+__global__ void __launch_bounds__(256) k_kry_backsub(KryDev *kd) {
+  __shared__ double H[kKryMax * kKryMax], g[kKryMax], y[kKryMax];
   const int jd = kd->jdone, m = kd->m;
-  for (int t = jd - 1; t >= 0; t--) {
-    double sum = kd->gv[t];
-    for (int u = t + 1; u < jd; u++) sum -= kd->H[t * m + u] * kd->y[u];
-    kd->y[t] = sum / kd->H[t * m + t];
+  for (int t = threadIdx.x; t < jd * m; t += 256) H[t] = kd->H[t];
+  for (int t = threadIdx.x; t < jd; t += 256) g[t] = kd->gv[t];
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int t = jd - 1; t >= 0; t--) {
+      double sum = g[t];
+      for (int u = t + 1; u < jd; u++) sum -= H[t * m + u] * y[u];
+      y[t] = sum / H[t * m + t];
+    }
+    kd->check = (jd > 0 && kd->rnorm <= kd->tol) ? 1 : 0;
   }
-  kd->check = (jd > 0 && kd->rnorm <= kd->tol) ? 1 : 0;
+  __syncthreads();
+  for (int t = threadIdx.x; t < jd; t += 256) kd->y[t] = y[t];
 }
 // After the confirming residual (when kd->check): convergence and the outer loop.
 __global__ void k_kry_confirm(KryDev *kd, unsigned long long h_outer, int use_graph) {
@@ -1008,100 +1064,58 @@ __global__ void k_kry_confirm(KryDev *kd, unsigned long long h_outer, int use_gr
 }
 
 // ---- host side
-static DynPtr dyn(double *base, long long ldv, const int *j, int off) { return DynPtr{base, ldv, j, off}; }
-
 // r = b - A x and <r, r> into *rr, under guard q.
 static int residual_dev(Ctx *c, const double *b, double *x, double *r, double *rr, Guard q) {
   Poisson &P = c->ps;
   const long long N = c->g.N;
   int rc;
-  if (P.transpose) {
-    c->launches++, k_zero_g<<<nblocks(N, 256), 256, 0, c->stream>>>(N, r, q);
-    c->launches++, k_apply_t_dyn<<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.nslot, P.coef, dyn(x, 0, nullptr, 0), r, q);
-    c->launches++, k_sub_norm_g<<<kKryBlocks, 256, 0, c->stream>>>(N, b, r, c->red, q);
-    if ((rc = check_launch(c, "residual (transposed)"))) return rc;
-    c->launches++, k_sum_parts_g<<<1, 1024, 0, c->stream>>>(c->red, kKryBlocks, rr, q);
-    return check_launch(c, "k_sum_parts_g");
-  }
   const int nb = (int)nblocks(N, 256);
-  if (P.nslot == 7)
-    c->launches++, k_residual_g<7><<<nb, 256, 0, c->stream>>>(c->g, P.coef, b, x, r, c->red, q);
-  else
-    c->launches++, k_residual_g<NSLOT><<<nb, 256, 0, c->stream>>>(c->g, P.coef, b, x, r, c->red, q);
+#define VFS_RESIDUAL(NS, T) c->launches++, k_residual_g<NS, T><<<nb, 256, 0, c->stream>>>(c->g, P.coef, b, x, r, c->red, q)
+  if (P.transpose) {
+    if (P.nslot == 7) VFS_RESIDUAL(7, true); else VFS_RESIDUAL(NSLOT, true);
+  } else {
+    if (P.nslot == 7) VFS_RESIDUAL(7, false); else VFS_RESIDUAL(NSLOT, false);
+  }
+#undef VFS_RESIDUAL
   if ((rc = check_launch(c, "k_residual_g"))) return rc;
   c->launches++, k_sum_parts_g<<<1, 1024, 0, c->stream>>>(c->red, nb, rr, q);
   return check_launch(c, "k_sum_parts_g");
 }
 
-// w = A z_j (z_j = Z + j ldv with j from the device state).
-static int apply_dyn(Ctx *c, double *Z, double *w) {
-  Poisson &P = c->ps;
-  const long long N = c->g.N;
-  KryDev *kd = c->kd;
-  if (P.transpose) {
-    c->launches++, k_zero_g<<<nblocks(N, 256), 256, 0, c->stream>>>(N, w, always());
-    c->launches++, k_apply_t_dyn<<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.nslot, P.coef,
-                                                                          dyn(Z, P.ldv, &kd->j, 0), w, always());
-    return check_launch(c, "k_apply_t_dyn");
-  }
-  if (P.nslot == 7)
-    c->launches++, k_apply_dyn<7><<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.coef, dyn(Z, P.ldv, &kd->j, 0), w);
-  else
-    c->launches++, k_apply_dyn<NSLOT><<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.coef, dyn(Z, P.ldv, &kd->j, 0), w);
-  return check_launch(c, "k_apply_dyn");
-}
-static int apply32_dyn(Ctx *c, float *Z, float *w) {
-  Poisson &P = c->ps;
-  const long long N = c->g.N;
-  const DynPtrT<float> z{Z, P.ldv, &c->kd->j, 0};
-  if (P.nslot == 7)
-    c->launches++, k_apply32_dyn<7><<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.coef, z, w);
-  else
-    c->launches++, k_apply32_dyn<NSLOT><<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.coef, z, w);
-  return check_launch(c, "k_apply32_dyn");
-}
-
-// One Arnoldi step of the device-driven FGMRES (body of the inner loop), on the basis of
-// type B (FP64; FP32 for precision 2, whose preconditioner and operator apply are FP32).
-template <typename B>
-static int kry_body_t(Ctx *c, const vfs_solve_opts &o, unsigned long long h_inner, int use_graph, B *V, B *Z, B *w) {
+// One Arnoldi step of the device-driven FGMRES (body of the inner loop) on a basis of type B
+// with preconditioned vectors of type ZT (the V-cycle's type): FP64/FP32 for precision 0,
+// FP64/FP64 for 1, FP32/FP32 for 2.  An FP32 V-cycle's z_j is kept in FP32, the values it has.
+template <typename B, typename ZT>
+static int kry_body_t(Ctx *c, const vfs_solve_opts &o, unsigned long long h_inner, int use_graph, B *V, ZT *Z, B *w) {
   Poisson &P = c->ps;
   KryDev *kd = c->kd;
   const long long N = c->g.N;
   const int kg = kry_grid(c);
   int rc;
-  if (sizeof(B) == 4) {
-    if ((rc = mg_precondition_dyn32(c, (const float *)V, (float *)Z, P.ldv, &kd->j, o))) return rc;  // z_j = M^-1 v_j
-    if ((rc = apply32_dyn(c, (float *)Z, (float *)w))) return rc;                                     // w = A z_j
+  if ((rc = mg_precondition(c, DynPtrT<const B>{V, P.ldv, &kd->j, 0}, DynPtrT<ZT>{Z, P.ldv, &kd->j, 0}, o)))
+    return rc;  // z_j = M^-1 v_j
+#define VFS_APPLY(NS, T) c->launches++, k_apply_dyn<NS, T><<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.ldv, P.coef, Z, kd, w)
+  if (P.transpose) {
+    if (P.nslot == 7) VFS_APPLY(7, true); else VFS_APPLY(NSLOT, true);
   } else {
-    if ((rc = mg_precondition_dyn(c, (const double *)V, (double *)Z, P.ldv, &kd->j, o))) return rc;
-    if ((rc = apply_dyn(c, (double *)Z, (double *)w))) return rc;
+    if (P.nslot == 7) VFS_APPLY(7, false); else VFS_APPLY(NSLOT, false);
   }
-  c->launches++, k_multidot_dyn<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red);
-  c->launches++, k_sum_rows_dyn<<<kKryMax + 2, 256, 0, c->stream>>>(c->red, kd, kg, kd->h, always());
-  c->launches++, k_kry_ctl_a<<<1, 1, 0, c->stream>>>(kd);
-  if ((rc = check_launch(c, "FGMRES Gram-Schmidt"))) return rc;
-  const Guard reorth{&kd->reorth, 1}, degen{&kd->degen, 1}, plain{&kd->degen, 0};
-  c->launches++, k_update_dots_dyn<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red, reorth);
-  c->launches++, k_sum_rows_dyn<<<kKryMax + 2, 256, 0, c->stream>>>(c->red, kd, kg, kd->h2, reorth);
-  c->launches++, k_kry_ctl_b<<<1, 1, 0, c->stream>>>(kd);
-  c->launches++, k_update_dots_dyn<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red, degen);
-  c->launches++, k_sum_rows_dyn<<<kKryMax + 2, 256, 0, c->stream>>>(c->red, kd, kg, kd->h3, degen);
-  c->launches++, k_kry_ctl_c<<<1, 1, 0, c->stream>>>(kd);
-  if ((rc = check_launch(c, "FGMRES re-orthogonalisation"))) return rc;
-  const DynPtrT<B> next{V, P.ldv, &kd->j, 1};
-  c->launches++, k_update_scale_dyn<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, next, plain);
-  c->launches++, k_scale_copy_dyn<B, B><<<nblocks(N, 256), 256, 0, c->stream>>>(N, w, &kd->scale, next, degen);
-  c->launches++, k_kry_givens<<<1, 1, 0, c->stream>>>(kd, h_inner, use_graph);
-  return check_launch(c, "FGMRES Givens");
+#undef VFS_APPLY
+  if ((rc = check_launch(c, "k_apply_dyn"))) return rc;
+  c->launches++, k_multidot<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red);
+  c->launches++, k_reorth<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red);
+  c->launches++, k_hessenberg<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red, h_inner, use_graph);
+  c->launches++, k_next_vector<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w);
+  return check_launch(c, "FGMRES Arnoldi step");
 }
 
 static bool fp32_inner(const vfs_solve_opts &o) { return o.precision == 2; }
 
 static int kry_body(Ctx *c, const vfs_solve_opts &o, unsigned long long h_inner, int use_graph) {
   Poisson &P = c->ps;
-  return fp32_inner(o) ? kry_body_t<float>(c, o, h_inner, use_graph, P.V32, P.Z32, P.w32)
-                       : kry_body_t<double>(c, o, h_inner, use_graph, P.V, P.Z, P.w);
+  if (o.precision == 2) return kry_body_t<float, float>(c, o, h_inner, use_graph, P.V32, P.Z32, P.w32);
+  if (o.precision == 1) return kry_body_t<double, double>(c, o, h_inner, use_graph, P.V, P.Z64, P.w);
+  return kry_body_t<double, float>(c, o, h_inner, use_graph, P.V, P.Z32, P.w);
 }
 
 static int kry_cycle_start(Ctx *c, const vfs_solve_opts &o, const double *b, double *x, unsigned long long h_inner,
@@ -1117,7 +1131,7 @@ static int kry_cycle_start(Ctx *c, const vfs_solve_opts &o, const double *b, dou
         N, P.r, &kd->scale, DynPtrT<float>{P.V32, P.ldv, nullptr, 0}, Guard{&kd->inner_go, 1});
   else
     c->launches++, k_scale_copy_dyn<double, double><<<nblocks(N, 256), 256, 0, c->stream>>>(
-        N, P.r, &kd->scale, dyn(P.V, P.ldv, nullptr, 0), Guard{&kd->inner_go, 1});
+        N, P.r, &kd->scale, DynPtrT<double>{P.V, P.ldv, nullptr, 0}, Guard{&kd->inner_go, 1});
   return check_launch(c, "FGMRES cycle start");
 }
 
@@ -1127,11 +1141,11 @@ static int kry_cycle_end(Ctx *c, const vfs_solve_opts &o, const double *b, doubl
   KryDev *kd = c->kd;
   const long long N = c->g.N;
   int rc;
-  c->launches++, k_kry_backsub<<<1, 1, 0, c->stream>>>(kd);
-  if (fp32_inner(o))
-    c->launches++, k_lincomb_add_dyn<float><<<nblocks(N, 256), 256, 0, c->stream>>>(N, P.ldv, P.Z32, kd, x);
+  c->launches++, k_kry_backsub<<<1, 256, 0, c->stream>>>(kd);
+  if (o.precision == 1)
+    c->launches++, k_lincomb_add_dyn<double><<<nblocks(N, 256), 256, 0, c->stream>>>(N, P.ldv, P.Z64, kd, x);
   else
-    c->launches++, k_lincomb_add_dyn<double><<<nblocks(N, 256), 256, 0, c->stream>>>(N, P.ldv, P.Z, kd, x);
+    c->launches++, k_lincomb_add_dyn<float><<<nblocks(N, 256), 256, 0, c->stream>>>(N, P.ldv, P.Z32, kd, x);
   if ((rc = check_launch(c, "FGMRES update"))) return rc;
   if ((rc = residual_dev(c, b, x, P.r, &kd->rr, Guard{&kd->check, 1}))) return rc;
   c->launches++, k_kry_confirm<<<1, 1, 0, c->stream>>>(kd, h_outer, use_graph);
@@ -1240,37 +1254,40 @@ static vfs_solve_opts solve_opts(const Ctx *c, const vfs_solve_opts *oin) {
 // most this factor before the FP64 residual is formed again (FP32 keeps about 7 digits).
 static const double kInnerRtol = 1e-5;
 
-// Allocates the solver's workspace for options o (the Krylov basis, and for precision 2
-// its FP32 form); outside a stream capture.
+// Allocates the solver's workspace for options o (the Krylov basis and the preconditioned
+// vectors in the types of its precision); outside a stream capture.
 int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   const vfs_solve_opts o = solve_opts(c, oin);
   Poisson &P = c->ps;
-  const long long N = c->g.N;
-  const bool f32 = o.precision == 2;
-  if (P.restart >= o.restart && (!f32 || P.restart32 >= o.restart)) return VFS_OK;
+  const long long ldv = vec_ld(c->g.N);
+  const int m = o.restart;
+  const bool f64 = o.precision != 2, z64 = o.precision == 1;
+  if ((!f64 || P.restart >= m) && (f64 || P.restart32 >= m) && (!z64 || P.restart_z64 >= m) &&
+      (z64 || P.restart_z32 >= m))
+    return VFS_OK;
   if (c->capturing) return set_err(c, VFS_ERR_STATE, "poisson_solve: Krylov basis not allocated before capture");
   c->setup_epoch++;  // a captured step graph holds the old buffers
-  P.ldv = (N + 31) / 32 * 32;
-  if (P.restart < o.restart) {
-    cudaFree(P.V); cudaFree(P.Z);
-    P.V = P.Z = nullptr;
-    P.restart = 0;
-    if (cudaMalloc(&P.V, sizeof(double) * P.ldv * (o.restart + 1)) != cudaSuccess ||
-        cudaMalloc(&P.Z, sizeof(double) * P.ldv * o.restart) != cudaSuccess)
-      return set_err(c, VFS_ERR_CUDA, "poisson_solve: Krylov basis allocation failed");
-    P.restart = o.restart;
-  }
-  if (!f32) return VFS_OK;
-  if (P.restart32 < o.restart) {
-    cudaFree(P.V32); cudaFree(P.Z32); cudaFree(P.w32);
-    P.V32 = P.Z32 = P.w32 = nullptr;
-    P.restart32 = 0;
-    if (cudaMalloc(&P.V32, sizeof(float) * P.ldv * (o.restart + 1)) != cudaSuccess ||
-        cudaMalloc(&P.Z32, sizeof(float) * P.ldv * o.restart) != cudaSuccess ||
-        cudaMalloc(&P.w32, sizeof(float) * P.ldv) != cudaSuccess)
-      return set_err(c, VFS_ERR_CUDA, "poisson_solve: FP32 Krylov basis allocation failed");
-    P.restart32 = o.restart;
-  }
+  if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "poisson_solve: failed");
+  P.ldv = ldv;
+  bool ok = true;
+  // the ghost points of the preconditioned vectors are never written: zero from the start
+  auto grow = [&](auto **v, int &have, int extra) {
+    if (!ok || have >= m) return;
+    const size_t bytes = sizeof(**v) * (size_t)ldv * (m + extra);
+    cudaFree(*v);
+    *v = nullptr;
+    have = 0;
+    ok = cudaMalloc(v, bytes) == cudaSuccess;
+    if (!ok) return;
+    cudaMemsetAsync(*v, 0, bytes, c->stream);
+    have = m;
+  };
+  if (f64) grow(&P.V, P.restart, 1);
+  else grow(&P.V32, P.restart32, 1);
+  if (z64) grow(&P.Z64, P.restart_z64, 0);
+  else grow(&P.Z32, P.restart_z32, 0);
+  if (!f64 && ok && !P.w32) ok = cudaMalloc(&P.w32, sizeof(float) * (size_t)ldv) == cudaSuccess;
+  if (!ok) return set_err(c, VFS_ERR_CUDA, "poisson_solve: Krylov basis allocation failed");
   return VFS_OK;
 }
 
@@ -1636,8 +1653,11 @@ int run_kernel(Ctx *c, int which, int reps) {
         vfs_solve_opts o;
         memset(&o, 0, sizeof(o));
         o.precision = which == 9 ? 0 : 1;
-        o.pre_smooth = 3; o.post_smooth = 3; o.coarse_iters = 4;
-        rc = mg_precondition(c, c->f[VFS_B][0], P.t, o);
+        o = solve_opts(c, &o);
+        if ((rc = poisson_prepare(c, &o))) return rc;
+        const DynPtrT<const double> b{c->f[VFS_B][0], 0, nullptr, 0};
+        rc = o.precision == 0 ? mg_precondition(c, b, DynPtrT<float>{P.Z32, 0, nullptr, 0}, o)
+                              : mg_precondition(c, b, DynPtrT<double>{P.Z64, 0, nullptr, 0}, o);
         if (rc) return rc;
         break;
       }
