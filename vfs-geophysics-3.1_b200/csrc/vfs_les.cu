@@ -2,20 +2,22 @@
 // (les.c:67-1133) and Compute_eddy_viscosity_LES (les.c:1135-1252), default options
 // (3-D box test filter, testfilter_ik = 0, clark = 0, no homogeneous-direction averaging).
 //
-// Six kernels, FP64 throughout, each pointwise expression in the reference's order:
+// FP64 throughout:
 //   k_les_prep    every DA point: contravariant centre velocity U,V,W and test-filter
 //                 weight of the point itself;
-//   k_les_image   every DA point: at the point's periodic image the strain products
-//                 S_ab*|S| and the test-filtered velocity (les.c:191-298);
-//   k_les_lm      interior cells, 3-D tile with a one-cell halo staged in shared memory:
-//                 the Germano identity contractions L_ij M_ij G and M_ij M_ij G
-//                 (les.c:300-661);
-//   k_les_cs      every DA point: filtered LM/MM, Cs = max(0, LM/(2(MM+eps))), wall floor
-//                 and [0, max_cs] clipping, periodic ghosts from their images (les.c:708-1048);
+//   k_les_image   interior cells: the strain products S_ab*|S| and the test-filtered
+//                 velocity (les.c:191-298); k_les_ghosts gives ghost points their image's;
+//   k_les_lm      interior cells: the Germano identity contractions L_ij M_ij G and
+//                 M_ij M_ij G (les.c:300-661);
+//   k_les_cs      interior cells: filtered LM/MM, Cs = max(0, LM/(2(MM+eps))), wall floor
+//                 and [0, max_cs] clipping (les.c:708-1048), ghosts as above;
 //   k_les_refilter  second test filtering of Cs over fluid cells (les.c:1051-1120);
 //   k_les_nut     nu_t = Cs * Delta^2 * |S| and its periodic ghosts (les.c:1174-1243).
-// The 3x3x3 test filter is integrate_testfilter (rhs2.c:412-455): eight 2x2x2 sub-cubes,
-// each summed in the reference's order, over the same sums of weights.
+// The 3x3x3 test filter is integrate_testfilter (rhs2.c:412-455): the weighted sums of eight
+// overlapping 2x2x2 sub-cubes over the sums of their weights.  A cell's own point lies in
+// all eight, a face neighbour in four, an edge neighbour in two, a corner in one, so the
+// sum is the (1 2 1) x (1 2 1) x (1 2 1) sum of value x weight: three one-dimensional
+// passes instead of 64 products (the same sum in another order).
 #include <cmath>
 
 #include "vfs_internal.cuh"
@@ -76,36 +78,102 @@ __device__ __forceinline__ double strain(const double o[9], double s[6]) {
                      s[2] * s[2] + s[4] * s[4] + s[5] * s[5]));
 }
 
-// Neighbour n = R*9 + Q*3 + P (R, Q, P = k, j, i offsets + 1) of the m-th point of the
-// s-th 2x2x2 sub-cube, in the order integrate_testfilter sums them (rhs2.c:433-455).
-__host__ __device__ constexpr int tf_base(int s) { return (s & 1) * 9 + ((s >> 2) & 1) * 3 + ((s >> 1) & 1); }
-__host__ __device__ constexpr int tf_off(int m) { return (m & 1) * 9 + ((m >> 2) & 1) * 3 + ((m >> 1) & 1); }
+// ------------------------------------------------------------------ test filter
+// A block of FTX x FTY interior cells marches through `kz` planes along k.  Every plane of
+// the tile and its one-cell rim is formed once (load: value x weight of NQ quantities at a
+// point), filtered along i and j through shared memory and along k in two running sums per
+// quantity and cell; emit gets the filtered sums of each cell.  15 quantities from 13
+// fields: bound by shared-memory traffic (six 8-byte accesses per quantity and cell, where
+// summing the sub-cubes as written took about ninety).
+constexpr int FTX = 32, FTY = 8, FRX = FTX + 2, FRY = FTY + 2;
+constexpr int kFilterThreads = FTX * FTY;
+template <int NQ>
+constexpr size_t filter_smem() { return sizeof(double) * NQ * (FRX * FRY + FTX * FRY); }
 
-// Sum of the sub-cube weight sums (the common denominator w1 + ... + w8).
-__device__ __forceinline__ double tf_wsum(const double w[27]) {
-  double tot = 0;
+template <int NQ, class Load, class Emit>
+__device__ __forceinline__ void box_filter(const Grid &g, int kz, const Load &load, const Emit &emit) {
+  extern __shared__ __align__(16) double les_sm[];
+  double *raw = les_sm, *fi = les_sm + NQ * FRX * FRY;  // the plane, and the plane filtered along i
+  const int i0 = 1 + blockIdx.x * FTX, j0 = 1 + blockIdx.y * FTY;
+  const int k0 = 1 + blockIdx.z * kz, k1 = min(k0 + kz, g.mz - 1);  // cells k0 .. k1-1
+  const int tx = threadIdx.x % FTX, ty = threadIdx.x / FTX;
+  const int i = i0 + tx, j = j0 + ty;
+  const bool cell = i <= g.mx - 2 && j <= g.my - 2;
+  double a[NQ], b[NQ];
 #pragma unroll
-  for (int s = 0; s < 8; s++) {
-    double ws = w[tf_base(s) + tf_off(0)];
+  for (int q = 0; q < NQ; q++) a[q] = b[q] = 0;
+  for (int k = k0 - 1; k <= k1; k++) {
+    for (int t = threadIdx.x; t < FRX * FRY; t += kFilterThreads) {
+      const int pi = i0 - 1 + t % FRX, pj = j0 - 1 + t / FRX;
+      double v[NQ];
 #pragma unroll
-    for (int m = 1; m < 8; m++) ws += w[tf_base(s) + tf_off(m)];
-    tot = (s == 0) ? ws : tot + ws;
+      for (int q = 0; q < NQ; q++) v[q] = 0;
+      if (pi < g.mx && pj < g.my) load(pi, pj, k, lidx(g, pi, pj, k), v);
+#pragma unroll
+      for (int q = 0; q < NQ; q++) raw[q * (FRX * FRY) + t] = v[q];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < FTX * FRY; t += kFilterThreads) {
+      const int c = (t / FTX) * FRX + t % FTX + 1;
+#pragma unroll
+      for (int q = 0; q < NQ; q++) {
+        const double *r = raw + q * (FRX * FRY) + c;
+        fi[q * (FTX * FRY) + t] = r[-1] + 2.0 * r[0] + r[1];
+      }
+    }
+    __syncthreads();  // also orders the next plane's writes of raw after this plane's reads
+    double f[NQ];
+#pragma unroll
+    for (int q = 0; q < NQ; q++) {
+      const double *r = fi + q * (FTX * FRY) + (ty + 1) * FTX + tx;
+      const double v = r[-FTX] + 2.0 * r[0] + r[FTX];
+      f[q] = a[q] + v;
+      a[q] = b[q] + 2.0 * v;
+      b[q] = v;
+    }
+    if (k > k0 && cell) emit(i, j, k - 1, lidx(g, i, j, k - 1), f);
   }
-  return tot;
+}
+// Planes a block marches through: as many as leave two blocks per SM, at most 16.
+static dim3 filter_grid(const Grid &g, int &kz) {
+  const unsigned bx = (g.mx - 2 + FTX - 1) / FTX, by = (g.my - 2 + FTY - 1) / FTY;
+  kz = 16;
+  while (kz > 2 && (unsigned long long)bx * by * ((g.mz - 2 + kz - 1) / kz) < 2 * 148) kz /= 2;
+  return dim3(bx, by, (g.mz - 2 + kz - 1) / kz);
 }
 
-// integrate_testfilter of one 27-point quantity given as val[n].
-__device__ __forceinline__ double tf_apply(const double val[27], const double w[27], double wsum) {
-  double tot = 0;
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    const int b = tf_base(s);
-    double vs = val[b + tf_off(0)] * w[b + tf_off(0)];
-#pragma unroll
-    for (int m = 1; m < 8; m++) vs += val[b + tf_off(m)] * w[b + tf_off(m)];
-    tot = (s == 0) ? vs : tot + vs;
+// Ghost points of n arrays: the value of the periodic image where that is an interior cell,
+// 0 elsewhere.
+struct LesArrays {
+  int n;
+  double *a[9];
+};
+__global__ void __launch_bounds__(256) k_les_ghosts(Grid g, LesArrays o) {
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long ni = 2LL * g.my * g.mz, nj = 2LL * g.mx * g.mz, nk = 2LL * g.mx * g.my;
+  int i, j, k;
+  if (t < ni) {
+    const long long r = t >> 1;
+    i = (t & 1) ? g.mx - 1 : 0; j = (int)(r % g.my); k = (int)(r / g.my);
+  } else if ((t -= ni) < nj) {
+    const long long r = t >> 1;
+    j = (t & 1) ? g.my - 1 : 0; i = (int)(r % g.mx); k = (int)(r / g.mx);
+  } else if ((t -= nj) < nk) {
+    const long long r = t >> 1;
+    k = (t & 1) ? g.mz - 1 : 0; i = (int)(r % g.mx); j = (int)(r / g.mx);
+  } else {
+    return;
   }
-  return tot / wsum;
+  const int ii = wrapi(g, i), jj = wrapj(g, j), kk = wrapk(g, k);
+  const long long p = lidx(g, i, j, k), s = lidx(g, ii, jj, kk);
+  const bool in = les_interior(g, ii, jj, kk);
+  for (int q = 0; q < o.n; q++) o.a[q][p] = in ? o.a[q][s] : 0.0;
+}
+static int les_ghosts(Ctx *c, const LesArrays &o) {
+  const Grid &g = c->g;
+  const long long n = 2LL * g.my * g.mz + 2LL * g.mx * g.mz + 2LL * g.mx * g.my;
+  c->launches++, k_les_ghosts<<<nblocks(n, 256), 256, 0, c->stream>>>(g, o);
+  return check_launch(c, "k_les_ghosts");
 }
 
 struct LesPrep {
@@ -128,61 +196,38 @@ __global__ void k_les_prep(Grid g, CV3 u, CV3 csi, CV3 eta, CV3 zet, const doubl
   o.wgt[p] = (nv[p] > 1) ? 0.0 : 1. / aj[p];  // get_weight, les.c:31-32
 }
 
-// Strain products S_ab |S| and the test-filtered velocity at every DA point's periodic
-// image (computed at interior fluid cells, les.c:191-238, and copied to periodic ghosts,
-// les.c:267-298); zero where the image is solid or a boundary point.
-__global__ void k_les_image(Grid g, CV3 u, CV3 csi, CV3 eta, CV3 zet, const double *__restrict__ aj,
-                            const uint8_t *__restrict__ nv, LesPrep o) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  int i, j, k;
-  dijk(g, p, i, j, k);
-  const int a = wrapi(g, i), b = wrapj(g, j), c = wrapk(g, k);
-  const long long q = lidx(g, a, b, c);
-  double ss[6] = {0, 0, 0, 0, 0, 0}, uf[3] = {0, 0, 0};
-  if (les_interior(g, a, b, c) && nv[q] <= 1) {
-    double d[9], gr[9], st[6];
-    du_center(g, u, nv, q, a, b, c, d);
-    const double cc[3] = {csi.x[q], csi.y[q], csi.z[q]};
-    const double ee[3] = {eta.x[q], eta.y[q], eta.z[q]};
-    const double zz[3] = {zet.x[q], zet.y[q], zet.z[q]};
-    du_dxyz(cc, ee, zz, aj[q], d, gr);
-    const double sabs = strain(gr, st);
+// Strain products S_ab |S| and the test-filtered velocity of the interior cells (les.c:191-238);
+// zero at solid cells.
+__global__ void __launch_bounds__(kFilterThreads, 2) k_les_image(Grid g, int kz, CV3 u, CV3 csi, CV3 eta, CV3 zet,
+                                                                 const double *__restrict__ aj,
+                                                                 const uint8_t *__restrict__ nv, LesPrep o) {
+  box_filter<4>(
+      g, kz,
+      [&](int, int, int, long long p, double *v) {
+        const double w = o.wgt[p];
+        v[0] = w; v[1] = u.x[p] * w; v[2] = u.y[p] * w; v[3] = u.z[p] * w;
+      },
+      [&](int i, int j, int k, long long p, const double *f) {
+        double ss[6] = {0, 0, 0, 0, 0, 0}, uf[3] = {0, 0, 0};
+        if (nv[p] <= 1) {
+          double d[9], gr[9], st[6];
+          du_center(g, u, nv, p, i, j, k, d);
+          const double cc[3] = {csi.x[p], csi.y[p], csi.z[p]};
+          const double ee[3] = {eta.x[p], eta.y[p], eta.z[p]};
+          const double zz[3] = {zet.x[p], zet.y[p], zet.z[p]};
+          du_dxyz(cc, ee, zz, aj[p], d, gr);
+          const double sabs = strain(gr, st);
 #pragma unroll
-    for (int t = 0; t < 6; t++) ss[t] = st[t] * sabs;
-    // integrate_testfilter of u, v, w with the get_weight weights (les.c:219-237)
-    const long long sy = g.mx, sz = (long long)g.mx * g.my;
-    double wt = 0, t0 = 0, t1 = 0, t2 = 0;
-#pragma unroll 1
-    for (int s = 0; s < 8; s++) {
-      double ws = 0, v0 = 0, v1 = 0, v2 = 0;
+          for (int t = 0; t < 6; t++) ss[t] = st[t] * sabs;
+          uf[0] = f[1] / f[0]; uf[1] = f[2] / f[0]; uf[2] = f[3] / f[0];
+        }
 #pragma unroll
-      for (int m = 0; m < 8; m++) {
-        const int n = tf_base(s) + tf_off(m);
-        const long long qq = q + (n / 9 - 1) * sz + ((n / 3) % 3 - 1) * sy + (n % 3 - 1);
-        const double wn = o.wgt[qq];
-        if (m == 0) { ws = wn; v0 = u.x[qq] * wn; v1 = u.y[qq] * wn; v2 = u.z[qq] * wn; }
-        else { ws += wn; v0 += u.x[qq] * wn; v1 += u.y[qq] * wn; v2 += u.z[qq] * wn; }
-      }
-      if (s == 0) { wt = ws; t0 = v0; t1 = v1; t2 = v2; }
-      else { wt += ws; t0 += v0; t1 += v1; t2 += v2; }
-    }
-    uf[0] = t0 / wt; uf[1] = t1 / wt; uf[2] = t2 / wt;
-  }
-#pragma unroll
-  for (int t = 0; t < 6; t++) o.ss[t][p] = ss[t];
-  o.uf[0][p] = uf[0]; o.uf[1][p] = uf[1]; o.uf[2][p] = uf[2];
+        for (int t = 0; t < 6; t++) o.ss[t][p] = ss[t];
+        o.uf[0][p] = uf[0]; o.uf[1][p] = uf[1]; o.uf[2][p] = uf[2];
+      });
 }
 
 // ------------------------------------------------------------------ k_les_lm
-constexpr int LTX = 32, LTY = 4, LTZ = 2;
-constexpr int LHX = LTX + 2, LHY = LTY + 2, LHZ = LTZ + 2, LHN = LHX * LHY * LHZ;
-constexpr int kLesLmThreads = LTX * LTY * LTZ;
-constexpr int kLesVals = 13;  // u v w U V W weight SS11 SS12 SS13 SS22 SS23 SS33
-struct LesLmSmem {
-  double v[kLesVals][LHN];
-};
-
 struct LesLmIn {
   CV3 u;
   const double *U, *V, *W, *wgt, *ss[6];
@@ -200,126 +245,17 @@ __device__ __forceinline__ void covariant(const double a[3][3], double G[3][3]) 
   G[2][0] = (a32 * a21 - a31 * a22) / det; G[2][1] = -(a32 * a11 - a31 * a12) / det; G[2][2] = (a22 * a11 - a21 * a12) / det;
 }
 
-// Tile index of neighbour n (R*9 + Q*3 + P) of the cell at tile index c0.
-__device__ __forceinline__ int les_nb(int c0, int n) {
-  return c0 + (n / 9 - 1) * LHX * LHY + ((n / 3) % 3 - 1) * LHX + (n % 3 - 1);
-}
-
-// Quantity q at tile point h: q < 9 the product (U,V,W)[q/3] * (u,v,w)[q%3] (les.c:381-391),
-// q >= 9 the strain product S_ab |S| number q-9 (les.c:428-430).
-template <int q>
-__device__ __forceinline__ double les_quantity(const LesLmSmem &S, int h) {
-  if (q < 9) return S.v[3 + q / 3][h] * S.v[q % 3][h];
-  return S.v[7 + (q - 9)][h];
-}
-
-// integrate_testfilter of quantities Q0 .. Q0+NQ-1 (rhs2.c:412-455) into F[].
-template <int Q0, int NQ>
-__device__ __forceinline__ void les_filter_pass(const LesLmSmem &S, int c0, double wsum, double *F) {
-  double tot[NQ], vs[NQ];
-#pragma unroll 1
-  for (int s = 0; s < 8; s++) {
-#pragma unroll
-    for (int m = 0; m < 8; m++) {
-      const int h = les_nb(c0, tf_base(s) + tf_off(m));
-      const double wn = S.v[6][h];
-      double x[NQ];
-#pragma unroll
-      for (int q = 0; q < NQ; q++) {
-        switch (Q0 + q) {
-          case 0: x[q] = les_quantity<0>(S, h); break;
-          case 1: x[q] = les_quantity<1>(S, h); break;
-          case 2: x[q] = les_quantity<2>(S, h); break;
-          case 3: x[q] = les_quantity<3>(S, h); break;
-          case 4: x[q] = les_quantity<4>(S, h); break;
-          case 5: x[q] = les_quantity<5>(S, h); break;
-          case 6: x[q] = les_quantity<6>(S, h); break;
-          case 7: x[q] = les_quantity<7>(S, h); break;
-          case 8: x[q] = les_quantity<8>(S, h); break;
-          case 9: x[q] = les_quantity<9>(S, h); break;
-          case 10: x[q] = les_quantity<10>(S, h); break;
-          case 11: x[q] = les_quantity<11>(S, h); break;
-          case 12: x[q] = les_quantity<12>(S, h); break;
-          case 13: x[q] = les_quantity<13>(S, h); break;
-          default: x[q] = les_quantity<14>(S, h); break;
-        }
-      }
-#pragma unroll
-      for (int q = 0; q < NQ; q++) vs[q] = (m == 0) ? x[q] * wn : vs[q] + x[q] * wn;
-    }
-#pragma unroll
-    for (int q = 0; q < NQ; q++) tot[q] = (s == 0) ? vs[q] : tot[q] + vs[q];
-  }
-#pragma unroll
-  for (int q = 0; q < NQ; q++) F[Q0 + q] = tot[q] / wsum;
-}
-
-__global__ void __launch_bounds__(kLesLmThreads, 2)
-    k_les_lm(Grid g, LesLmIn in, CV3 csi, CV3 eta, CV3 zet, const double *__restrict__ aj,
-             const uint8_t *__restrict__ nv, double *LM, double *MM) {
-  extern __shared__ __align__(16) unsigned char les_raw[];
-  LesLmSmem &S = *reinterpret_cast<LesLmSmem *>(les_raw);
-  const int i0 = 1 + blockIdx.x * LTX, j0 = 1 + blockIdx.y * LTY, k0 = 1 + blockIdx.z * LTZ;
-  // stage the halo tile: own-point values of the 34 x 6 x 4 points around the tile
-  for (int t = threadIdx.x; t < LHN; t += blockDim.x) {
-    const int hi = t % LHX, hj = (t / LHX) % LHY, hk = t / (LHX * LHY);
-    const int i = i0 - 1 + hi, j = j0 - 1 + hj, k = k0 - 1 + hk;
-    if (i < g.mx && j < g.my && k < g.mz) {
-      const long long p = lidx(g, i, j, k);
-      S.v[0][t] = in.u.x[p]; S.v[1][t] = in.u.y[p]; S.v[2][t] = in.u.z[p];
-      S.v[3][t] = in.U[p]; S.v[4][t] = in.V[p]; S.v[5][t] = in.W[p];
-      S.v[6][t] = in.wgt[p];
-#pragma unroll
-      for (int q = 0; q < 6; q++) S.v[7 + q][t] = in.ss[q][p];
-    } else {
-#pragma unroll
-      for (int q = 0; q < kLesVals; q++) S.v[q][t] = 0.0;
-    }
-  }
-  __syncthreads();
-  const int ti = threadIdx.x % LTX, tj = (threadIdx.x / LTX) % LTY, tk = threadIdx.x / (LTX * LTY);
-  const int i = i0 + ti, j = j0 + tj, k = k0 + tk;
-  if (i > g.mx - 2 || j > g.my - 2 || k > g.mz - 2) return;
-  const long long p = lidx(g, i, j, k);
-  if (nv[p] > 1) { LM[p] = 0; MM[p] = 0; return; }
-  const int c0 = (tk + 1) * LHX * LHY + (tj + 1) * LHX + (ti + 1);  // tile index of the cell
-  auto nb = [&](int n) { return les_nb(c0, n); };
-
-  // weights stay in shared memory (S.v[6]); w1 + ... + w8 and sum_weight from there
-  double wsum = 0;
-#pragma unroll
-  for (int s = 0; s < 8; s++) {
-    double ws = S.v[6][nb(tf_base(s) + tf_off(0))];
-#pragma unroll
-    for (int m = 1; m < 8; m++) ws += S.v[6][nb(tf_base(s) + tf_off(m))];
-    wsum = (s == 0) ? ws : wsum + ws;
-  }
-  // sum_weight with the (1/2, 1, 1/2)^3 weights, loops p (i) outer, q (j), r (k) inner
-  // (les.c:433-452)
-  double sum_weight = 0;
-#pragma unroll
-  for (int pp = 0; pp < 3; pp++)
-#pragma unroll
-    for (int qq = 0; qq < 3; qq++)
-#pragma unroll
-      for (int rr = 0; rr < 3; rr++) {
-        const double cf = (rr == 1 ? 1.0 : 0.5) * (qq == 1 ? 1.0 : 0.5) * (pp == 1 ? 1.0 : 0.5);
-        sum_weight += S.v[6][nb(rr * 9 + qq * 3 + pp)] * cf;
-      }
-
-  // 15 test-filtered quantities, three passes of five to keep the accumulators in
-  // registers: U u, U v, U w, V u, ..., W w (Lij) and the six S_ab |S|
-  double F[15];
-  les_filter_pass<0, 5>(S, c0, wsum, F);
-  les_filter_pass<5, 5>(S, c0, wsum, F);
-  les_filter_pass<10, 5>(S, c0, wsum, F);
-
+// The contractions at one cell from its 15 test-filtered quantities F: U u, U v, ..., W w
+// (les.c:381-391), then the six S_ab |S| (les.c:428-430); wsum is the filter's weight sum.
+__device__ __forceinline__ void lm_cell(const Grid &g, const LesLmIn &in, CV3 csi, CV3 eta, CV3 zet,
+                                        const double *__restrict__ aj, const uint8_t *__restrict__ nv, long long p,
+                                        int i, int j, int k, const double *F, double wsum, double &lm, double &mm) {
   const double cc[3] = {csi.x[p], csi.y[p], csi.z[p]};
   const double ee[3] = {eta.x[p], eta.y[p], eta.z[p]};
   const double zz[3] = {zet.x[p], zet.y[p], zet.z[p]};
   const double ajc = aj[p];
-  const double filter = pow(1. / ajc, 1. / 3.);
-  const double test_filter = pow(sum_weight, 1. / 3.);
+  const double filter = cbrt(1. / ajc);
+  const double test_filter = cbrt(0.125 * wsum);  // the (1/2 1 1/2)^3 sum of the weights (les.c:433-452)
   // filtered velocity at the cell and its contravariant components (les.c:470-475)
   const double fu = in.uf.x[p], fv = in.uf.y[p], fw = in.uf.z[p];
   const double fU = fu * cc[0] + fv * cc[1] + fw * cc[2];
@@ -348,8 +284,8 @@ __global__ void __launch_bounds__(kLesLmThreads, 2)
   G[0][2] = G[2][0] = xzet * xcsi + yzet * ycsi + zzet * zcsi;
   G[1][2] = G[2][1] = xeta * xzet + yeta * yzet + zeta * zzet;
   // Mij (les.c:616-633)
-  const double tA = -pow(test_filter, 2.) * S_hat;
-  const double fB = pow(filter, 2.);
+  const double tA = -(test_filter * test_filter) * S_hat;
+  const double fB = filter * filter;
   double Mc[3][3], M[3][3];
 #pragma unroll
   for (int a = 0; a < 3; a++)
@@ -374,80 +310,109 @@ __global__ void __launch_bounds__(kLesLmThreads, 2)
     for (int n = 0; n < 3; n++)
 #pragma unroll
       for (int l = 0; l < 3; l++) denom += M[n][m] * M[n][l] * G[m][l];
-  LM[p] = num;
-  MM[p] = denom;
+  lm = num;
+  mm = denom;
 }
 
-// Test-filter weights of the Cs averaging and re-filtering loops (les.c:720-762,
-// les.c:1069-1110): 1/aj of the neighbour (0 where nvert > 1.1), zero at non-periodic
-// boundary neighbours, and the neighbour's value read at its periodic image.  In the j
-// direction the reference tests the cell's own j against my-1 (les.c:748, les.c:1097),
-// so only J == 0 is zeroed; that test is kept.
-__device__ __forceinline__ void wrap_weights(const Grid &g, const double *__restrict__ wgt, int i, int j, int k,
-                                             double w[27], long long src[27]) {
+
+__global__ void __launch_bounds__(kFilterThreads, 2)
+    k_les_lm(Grid g, int kz, LesLmIn in, CV3 csi, CV3 eta, CV3 zet, const double *__restrict__ aj,
+             const uint8_t *__restrict__ nv, double *LM, double *MM) {
+  box_filter<16>(
+      g, kz,
+      [&](int, int, int, long long p, double *v) {
+        const double w = in.wgt[p];
+        const double u = in.u.x[p] * w, vv = in.u.y[p] * w, ww = in.u.z[p] * w;
+        const double U = in.U[p], V = in.V[p], W = in.W[p];
+        v[0] = U * u; v[1] = U * vv; v[2] = U * ww;
+        v[3] = V * u; v[4] = V * vv; v[5] = V * ww;
+        v[6] = W * u; v[7] = W * vv; v[8] = W * ww;
 #pragma unroll
-  for (int n = 0; n < 27; n++) {
-    int K = k + n / 9 - 1, J = j + (n / 3) % 3 - 1, I = i + n % 3 - 1;
-    double wt = wgt[lidx(g, I, J, K)];  // 1/aj, 0 where nvert > 1.1
-    if (g.iper) { if (I == 0) I = g.mx - 2; else if (I == g.mx - 1) I = 1; }
-    else if (I == 0 || I == g.mx - 1) wt = 0;
-    if (g.jper) { if (J == 0) J = g.my - 2; else if (J == g.my - 1) J = 1; }
-    else if (J == 0 || j == g.my - 1) wt = 0;
-    if (g.kper) { if (K == 0) K = g.mz - 2; else if (K == g.mz - 1) K = 1; }
-    else if (K == 0 || K == g.mz - 1) wt = 0;
-    w[n] = wt;
-    src[n] = lidx(g, I, J, K);
+        for (int q = 0; q < 6; q++) v[9 + q] = in.ss[q][p] * w;
+        v[15] = w;
+      },
+      [&](int i, int j, int k, long long p, double *f) {
+        double lm = 0, mm = 0;
+        if (nv[p] <= 1) {
+          const double wsum = f[15];
+#pragma unroll
+          for (int q = 0; q < 15; q++) f[q] = f[q] / wsum;
+          lm_cell(g, in, csi, eta, zet, aj, nv, p, i, j, k, f, wsum, lm, mm);
+        }
+        LM[p] = lm;
+        MM[p] = mm;
+      });
+}
+
+// Test-filter weight of a point in the Cs averaging and re-filtering loops (les.c:720-762,
+// les.c:1069-1110): 1/aj (0 where nvert > 1.1), zero at non-periodic boundary points; the
+// value of a periodic ghost point is its image's, which the ghosts of the filtered fields
+// hold.  In the j direction the reference tests the cell's own j against my-1 (les.c:748,
+// les.c:1097), so only J == 0 is zeroed; that test is kept.
+__device__ __forceinline__ double wrap_weight(const Grid &g, const double *__restrict__ wgt, long long p, int i,
+                                              int j, int k) {
+  if (!g.iper && (i == 0 || i == g.mx - 1)) return 0.0;
+  if (!g.jper && j == 0) return 0.0;
+  if (!g.kper && (k == 0 || k == g.mz - 1)) return 0.0;
+  return wgt[p];
+}
+
+// Clipped Cs of the interior cells (les.c:708-788 with les = 2, then les.c:959-972).
+__global__ void __launch_bounds__(kFilterThreads, 3) k_les_cs(Grid g, int kz, const double *__restrict__ wgt,
+                                                              const uint8_t *__restrict__ nv,
+                                                              const double *__restrict__ LM,
+                                                              const double *__restrict__ MM, double max_cs, double *out) {
+  box_filter<3>(
+      g, kz,
+      [&](int i, int j, int k, long long p, double *v) {
+        const double w = wrap_weight(g, wgt, p, i, j, k);
+        v[0] = w; v[1] = LM[p] * w; v[2] = MM[p] * w;
+      },
+      [&](int, int, int, long long p, const double *f) {
+        double cs = 0;
+        if (nv[p] <= 1) {
+          const double LM_avg = f[1] / f[0], MM_avg = f[2] / f[0];
+          const double C = 0.5 * LM_avg / (MM_avg + kLesEps);
+          cs = (C < 0) ? 0 : C;                                // PetscMax(C, 0)
+          if (nv[p] == 1) cs = (kWallCs < cs) ? cs : kWallCs;  // PetscMax(wall_cs, Cs) at IB nodes
+          cs = (cs < 0) ? 0 : cs;
+          cs = (cs < max_cs) ? cs : max_cs;                    // PetscMin(PetscMax(Cs, 0), max_cs)
+        }
+        out[p] = cs;
+      });
+}
+
+// Second filtering of Cs over fluid cells (nvert < 0.1); every other interior cell keeps its
+// value (k_les_keep: the ghost points).
+__global__ void __launch_bounds__(kFilterThreads, 3) k_les_refilter(Grid g, int kz, const double *__restrict__ wgt,
+                                                                    const uint8_t *__restrict__ nv,
+                                                                    const double *__restrict__ cs_tmp, double *cs) {
+  box_filter<2>(
+      g, kz,
+      [&](int i, int j, int k, long long p, double *v) {
+        const double w = wrap_weight(g, wgt, p, i, j, k);
+        v[0] = w; v[1] = cs_tmp[p] * w;
+      },
+      [&](int, int, int, long long p, const double *f) { cs[p] = nv[p] != 0 ? cs_tmp[p] : f[1] / f[0]; });
+}
+__global__ void __launch_bounds__(256) k_les_keep(Grid g, const double *__restrict__ from, double *to) {
+  long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long ni = 2LL * g.my * g.mz, nj = 2LL * g.mx * g.mz, nk = 2LL * g.mx * g.my;
+  int i, j, k;
+  if (t < ni) {
+    const long long r = t >> 1;
+    i = (t & 1) ? g.mx - 1 : 0; j = (int)(r % g.my); k = (int)(r / g.my);
+  } else if ((t -= ni) < nj) {
+    const long long r = t >> 1;
+    j = (t & 1) ? g.my - 1 : 0; i = (int)(r % g.mx); k = (int)(r / g.mx);
+  } else if ((t -= nj) < nk) {
+    const long long r = t >> 1;
+    k = (t & 1) ? g.mz - 1 : 0; i = (int)(r % g.mx); j = (int)(r / g.mx);
+  } else {
+    return;
   }
-}
-
-// Clipped Cs of one interior cell (les.c:708-788 with les = 2, then les.c:959-972).
-__device__ __forceinline__ double cs_cell(const Grid &g, const double *__restrict__ wgt,
-                                          const uint8_t *__restrict__ nv, const double *__restrict__ LM,
-                                          const double *__restrict__ MM, int i, int j, int k, double max_cs) {
   const long long p = lidx(g, i, j, k);
-  if (nv[p] > 1) return 0.0;
-  double w[27], lm[27], mm[27];
-  long long src[27];
-  wrap_weights(g, wgt, i, j, k, w, src);
-#pragma unroll
-  for (int n = 0; n < 27; n++) { lm[n] = LM[src[n]]; mm[n] = MM[src[n]]; }
-  const double ws = tf_wsum(w);
-  const double LM_avg = tf_apply(lm, w, ws);
-  const double MM_avg = tf_apply(mm, w, ws);
-  const double C = 0.5 * LM_avg / (MM_avg + kLesEps);
-  double cs = (C < 0) ? 0 : C;                       // PetscMax(C, 0)
-  if (nv[p] == 1) cs = (kWallCs < cs) ? cs : kWallCs;  // PetscMax(wall_cs, Cs) at IB nodes
-  cs = (cs < 0) ? 0 : cs;
-  cs = (cs < max_cs) ? cs : max_cs;                 // PetscMin(PetscMax(Cs, 0), max_cs)
-  return cs;
-}
-
-// Every DA point: interior cells their clipped Cs, periodic ghosts the value of their image
-// (zero when the image is itself a boundary point), other ghosts zero.
-__global__ void k_les_cs(Grid g, const double *__restrict__ wgt, const uint8_t *__restrict__ nv,
-                         const double *__restrict__ LM, const double *__restrict__ MM, double max_cs, double *cs) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  int i, j, k;
-  dijk(g, p, i, j, k);
-  const int a = wrapi(g, i), b = wrapj(g, j), c = wrapk(g, k);
-  cs[p] = les_interior(g, a, b, c) ? cs_cell(g, wgt, nv, LM, MM, a, b, c, max_cs) : 0.0;
-}
-
-// Second filtering of Cs over fluid cells (nvert < 0.1); every other point keeps its value.
-__global__ void k_les_refilter(Grid g, const double *__restrict__ wgt, const uint8_t *__restrict__ nv,
-                               const double *__restrict__ cs_tmp, double *cs) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= g.N) return;
-  int i, j, k;
-  dijk(g, p, i, j, k);
-  if (!les_interior(g, i, j, k) || nv[p] != 0) { cs[p] = cs_tmp[p]; return; }
-  double w[27], v[27];
-  long long src[27];
-  wrap_weights(g, wgt, i, j, k, w, src);
-#pragma unroll
-  for (int n = 0; n < 27; n++) v[n] = cs_tmp[src[n]];
-  cs[p] = tf_apply(v, w, tf_wsum(w));
+  to[p] = from[p];
 }
 
 // nu_t of one interior cell (les.c:1177-1198).
@@ -463,8 +428,8 @@ __device__ __forceinline__ double nut_cell(const Grid &g, CV3 u, CV3 csi, CV3 et
   const double zz[3] = {zet.x[p], zet.y[p], zet.z[p]};
   du_dxyz(cc, ee, zz, aj[p], d, gr);
   const double sabs = strain(gr, s);
-  const double filter = pow(1. / aj[p], 1. / 3.);
-  return cs[p] * pow(filter, 2.0) * sabs;
+  const double filter = cbrt(1. / aj[p]);
+  return cs[p] * (filter * filter) * sabs;
 }
 
 // Interior cells and periodic ghosts (value of the image; the old value of the image when
@@ -517,27 +482,28 @@ int smagorinsky_constant(Ctx *c) {
   CV3 u = cv(field3(c, VFS_UCAT));
   c->launches++, k_les_prep<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, u, m.csi, m.eta, m.zet, m.aj, c->nv, o);
   if ((rc = check_launch(c, "k_les_prep"))) return rc;
-  c->launches++, k_les_image<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, u, m.csi, m.eta, m.zet, m.aj, c->nv, o);
+  // the shared-memory limit is an attribute of the kernel on a device
+  if (cudaFuncSetAttribute(k_les_lm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)filter_smem<16>()) != cudaSuccess)
+    return set_err(c, VFS_ERR_CUDA, "k_les_lm: shared-memory limit");
+  int kz;
+  const dim3 grid = filter_grid(g, kz);
+  c->launches++, k_les_image<<<grid, kFilterThreads, filter_smem<4>(), c->stream>>>(g, kz, u, m.csi, m.eta, m.zet, m.aj, c->nv, o);
   if ((rc = check_launch(c, "k_les_image"))) return rc;
-  cudaMemsetAsync(LM, 0, sizeof(double) * (size_t)g.N, c->stream);
-  cudaMemsetAsync(MM, 0, sizeof(double) * (size_t)g.N, c->stream);
-  static bool attr = false;
-  if (!attr) {
-    cudaFuncSetAttribute(k_les_lm, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(LesLmSmem));
-    attr = true;
-  }
+  if ((rc = les_ghosts(c, LesArrays{9, {o.ss[0], o.ss[1], o.ss[2], o.ss[3], o.ss[4], o.ss[5], o.uf[0], o.uf[1], o.uf[2]}}))) return rc;
   LesLmIn in;
   in.u = u;
   in.U = o.U; in.V = o.V; in.W = o.W; in.wgt = o.wgt;
   for (int q = 0; q < 6; q++) in.ss[q] = o.ss[q];
   in.uf = CV3{o.uf[0], o.uf[1], o.uf[2]};
-  dim3 grid((g.mx - 2 + LTX - 1) / LTX, (g.my - 2 + LTY - 1) / LTY, (g.mz - 2 + LTZ - 1) / LTZ);
-  c->launches++, k_les_lm<<<grid, kLesLmThreads, sizeof(LesLmSmem), c->stream>>>(g, in, m.csi, m.eta, m.zet, m.aj, c->nv, LM, MM);
+  c->launches++, k_les_lm<<<grid, kFilterThreads, filter_smem<16>(), c->stream>>>(g, kz, in, m.csi, m.eta, m.zet, m.aj, c->nv, LM, MM);
   if ((rc = check_launch(c, "k_les_lm"))) return rc;
-  if ((rc = periodic_copy3(c, V3{LM, MM, nullptr}))) return rc;
-  c->launches++, k_les_cs<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, o.wgt, c->nv, LM, MM, c->max_cs, cs_tmp);
+  if ((rc = les_ghosts(c, LesArrays{2, {LM, MM}}))) return rc;
+  c->launches++, k_les_cs<<<grid, kFilterThreads, filter_smem<3>(), c->stream>>>(g, kz, o.wgt, c->nv, LM, MM, c->max_cs, cs_tmp);
   if ((rc = check_launch(c, "k_les_cs"))) return rc;
-  c->launches++, k_les_refilter<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, o.wgt, c->nv, cs_tmp, cs);
+  if ((rc = les_ghosts(c, LesArrays{1, {cs_tmp}}))) return rc;
+  c->launches++, k_les_refilter<<<grid, kFilterThreads, filter_smem<2>(), c->stream>>>(g, kz, o.wgt, c->nv, cs_tmp, cs);
+  const long long ng = 2LL * g.my * g.mz + 2LL * g.mx * g.mz + 2LL * g.mx * g.my;
+  c->launches++, k_les_keep<<<nblocks(ng, 256), 256, 0, c->stream>>>(g, cs_tmp, cs);
   return check_launch(c, "k_les_refilter");
 }
 
