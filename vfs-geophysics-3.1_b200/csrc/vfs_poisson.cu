@@ -195,10 +195,47 @@ __global__ void k_poisson_coef(Grid g, Metrics m, const uint8_t *__restrict__ nv
   fluid[p] = 1;
 }
 
-// Neighbour index of slot s for an unknown (valid only where the coefficient is non-zero;
-// the index is always inside the array).
-__device__ __forceinline__ long long nb_index(const Grid &g, int i, int j, int k, int s) {
-  return lidx(g, wrapi(g, i + c_off[s][0]), wrapj(g, j + c_off[s][1]), wrapk(g, k + c_off[s][2]));
+// Offsets from an interior point to its neighbours along the lines, periodic images included.
+// (Forming every neighbour's index from its coordinates made the apply bound by its integer
+// instructions.)
+struct NbOff {
+  int e, w, n, s, t, b;
+};
+__device__ __forceinline__ NbOff nb_offsets(const Grid &g, int i, int j, int k) {
+  const int sy = g.mx, sz = g.mx * g.my;
+  NbOff o;
+  o.e = g.iper && i == g.mx - 2 ? 3 - g.mx : 1;
+  o.w = g.iper && i == 1 ? g.mx - 3 : -1;
+  o.n = g.jper && j == g.my - 2 ? (3 - g.my) * sy : sy;
+  o.s = g.jper && j == 1 ? (g.my - 3) * sy : -sy;
+  o.t = g.kper && k == g.mz - 2 ? (3 - g.mz) * sz : sz;
+  o.b = g.kper && k == 1 ? (g.mz - 3) * sz : -sz;
+  return o;
+}
+// Offset of slot t (valid only where the coefficient is non-zero; the index is always inside
+// the array).
+__device__ __forceinline__ int nb_off(const NbOff &o, int t) {
+  switch (t) {
+    case EP: return o.e;
+    case WP: return o.w;
+    case NP: return o.n;
+    case SP: return o.s;
+    case TP: return o.t;
+    case BP: return o.b;
+    case NE: return o.e + o.n;
+    case SE: return o.e + o.s;
+    case NW: return o.w + o.n;
+    case SW: return o.w + o.s;
+    case TN: return o.t + o.n;
+    case BN: return o.b + o.n;
+    case TS: return o.t + o.s;
+    case BS: return o.b + o.s;
+    case TE: return o.e + o.t;
+    case BE: return o.e + o.b;
+    case TW: return o.w + o.t;
+    case BW: return o.w + o.b;
+    default: return 0;
+  }
 }
 
 // (A x)[p] on the grid layout from the first NS stencil slots: NS = 7 when every cross
@@ -214,12 +251,14 @@ __device__ __forceinline__ double apply_row64(const Grid &g, const double *__res
   int i, j, k;
   dijk(g, p, i, j, k);
   if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return 0.0;
+  const NbOff o = nb_offsets(g, i, j, k);
+  const XT *__restrict__ xp = x + p;
   double cf[NS];
   XT xv[NS];
 #pragma unroll
   for (int t = 0; t < NS; t++) {
     cf[t] = __ldcs(coef + t * ld + p);
-    xv[t] = x[nb_index(g, i, j, k, t)];
+    xv[t] = xp[nb_off(o, t)];
   }
   double s = 0;
 #pragma unroll
@@ -252,10 +291,11 @@ __device__ __forceinline__ double apply_row64_t(const Grid &g, const double *__r
   int i, j, k;
   dijk(g, p, i, j, k);
   if (i < 1 || i > g.mx - 2 || j < 1 || j > g.my - 2 || k < 1 || k > g.mz - 2) return 0.0;
+  const NbOff o = nb_offsets(g, i, j, k);
   double s = 0;
 #pragma unroll
   for (int t = 0; t < NS; t++) {
-    const long long q = nb_index(g, i, j, k, t);
+    const long long q = p + nb_off(o, t);
     s += coef[opposite(t) * ld + q] * (double)x[q];
   }
   return s;
@@ -736,9 +776,11 @@ __device__ __forceinline__ void kry_givens(KryDev *kd, unsigned long long h_inne
 
 // w = A z_j.  The rows are FP64 sums of FP64 coefficients whatever the vectors' types (precision
 // 2: FP32 coefficients measured 20-40 % more iterations, since iterative refinement converges
-// at the rate of the inner operator's error), rounded to w's type.
+// at the rate of the inner operator's error), rounded to w's type.  Blocks of 64 threads without a
+// register cap: 19 slots at 192 x 128 x 192 215 us against 255 in blocks of 256.
+constexpr int kApplyThreads = 64;
 template <int NS, bool kT, typename B, typename ZT>
-__global__ void __launch_bounds__(256) k_apply_dyn(Grid g, long long ldv, const double *__restrict__ coef,
+__global__ void __launch_bounds__(kApplyThreads) k_apply_dyn(Grid g, long long ldv, const double *__restrict__ coef,
                                                    const ZT *__restrict__ Z, const KryDev *__restrict__ kd,
                                                    B *__restrict__ w) {
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1094,7 +1136,7 @@ static int kry_body_t(Ctx *c, const vfs_solve_opts &o, unsigned long long h_inne
   int rc;
   if ((rc = mg_precondition(c, DynPtrT<const B>{V, P.ldv, &kd->j, 0}, DynPtrT<ZT>{Z, P.ldv, &kd->j, 0}, o)))
     return rc;  // z_j = M^-1 v_j
-#define VFS_APPLY(NS, T) c->launches++, k_apply_dyn<NS, T><<<nblocks(N, 256), 256, 0, c->stream>>>(c->g, P.ldv, P.coef, Z, kd, w)
+#define VFS_APPLY(NS, T) c->launches++, k_apply_dyn<NS, T><<<nblocks(N, kApplyThreads), kApplyThreads, 0, c->stream>>>(c->g, P.ldv, P.coef, Z, kd, w)
   if (P.transpose) {
     if (P.nslot == 7) VFS_APPLY(7, true); else VFS_APPLY(NSLOT, true);
   } else {
