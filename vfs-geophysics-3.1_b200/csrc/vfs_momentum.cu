@@ -1064,12 +1064,14 @@ __device__ __forceinline__ void fp_point(const Grid &g, const FluxIn &f1, const 
   fpx[p] = fpv[0]; fpy[p] = fpv[1]; fpz[p] = fpv[2];
 }
 
-// Four resident blocks per SM (64 registers): 0.56 ms at 256 x 192 x 256 against 0.70 ms
-// uncapped (116 registers) and slower again at five or six (spills).
+// 64 registers: 0.58 ms at 256 x 192 x 256 in blocks of 256 threads against 0.70 ms uncapped
+// (116 registers) and slower again below (spills).  In blocks of 64 threads 0.51 ms: a block's
+// registers are free again as soon as its two warps end.
+constexpr int kFpThreads = 64;
 #ifndef VFS_FP_MINB
-#define VFS_FP_MINB 4
+#define VFS_FP_MINB 16
 #endif
-__global__ void __launch_bounds__(256, VFS_FP_MINB) k_fp(Grid g, FluxIn f1, FluxIn f2, FluxIn f3,
+__global__ void __launch_bounds__(kFpThreads, VFS_FP_MINB) k_fp(Grid g, FluxIn f1, FluxIn f2, FluxIn f3,
                                                          const uint8_t *__restrict__ nv, double *fpx, double *fpy,
                                                          double *fpz) {
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1514,7 +1516,7 @@ int formfunction2(Ctx *c, double scale, bool rk_stage, double rk_coeff) {
 // single-kernel launchers for the diagnostics entry point (vfs_run_kernel)
 void launch_face_flux(Ctx *c) { face_fluxes(c); }
 void launch_fp(Ctx *c) {
-  c->launches++, k_fp<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, flux_in(c, 0), flux_in(c, 1), flux_in(c, 2), c->nv,
+  c->launches++, k_fp<<<nblocks(c->g.N, kFpThreads), kFpThreads, 0, c->stream>>>(c->g, flux_in(c, 0), flux_in(c, 1), flux_in(c, 2), c->nv,
                                                    c->fp[0], c->fp[1], c->fp[2]);
 }
 void launch_rhs(Ctx *c) {
@@ -2492,7 +2494,7 @@ int ff2_stage_tangent(Ctx *c, const double *const uc[3], const double *const uk[
   FluxIn f[3];
   for (int d = 0; d < 3; d++)
     for (int q = 0; q < 3; q++) { f[d].div[q] = tf[d][q]; f[d].visc[q] = tf[d][3 + q]; }
-  c->launches++, k_fp<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, f[0], f[1], f[2], c->nv, c->fp[0], c->fp[1], c->fp[2]);
+  c->launches++, k_fp<<<nblocks(g.N, kFpThreads), kFpThreads, 0, c->stream>>>(g, f[0], f[1], f[2], c->nv, c->fp[0], c->fp[1], c->fp[2]);
   if ((rc = check_launch(c, "k_fp"))) return rc;
   c->launches++, k_rhs<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, m, c->nv, c->fp[0], c->fp[1], c->fp[2], 1.0, field3(c, VFS_RHS),
                                                  1, a, cv(ddp), cv(dpu), dU);
