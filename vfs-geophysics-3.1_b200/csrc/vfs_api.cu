@@ -331,6 +331,7 @@ int vfs_destroy(vfs_ctx *ctx) {
   if (c->ibn) cudaFree(c->ibn);
   if (c->ibbuf) cudaFree(c->ibbuf);
   step_graph_free(c);
+  solve_graphs_free(c->ps);
   if (c->ds) cudaFree(c->ds);
   if (c->ds_in) cudaFreeHost(c->ds_in);
   if (c->ds_out) cudaFreeHost(c->ds_out);

@@ -136,8 +136,26 @@ struct MGLevel {
   float *v32 = nullptr;
 };
 
+// A Poisson solve captured as a graph (a solve outside a captured step): what its kernels'
+// arguments depend on, and the graph from the second such solve on.
+struct SolveKey {
+  vfs_solve_opts o;
+  int warm, transpose, nslot, reserved;
+  long long alloc_epoch;
+  const void *x, *b, *red;
+};
+struct SolveGraph {
+  SolveKey key;
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  bool failed = false;           // it could not be captured: launch the kernels one by one
+  long long launches = 0, body_launches = 0, cycle_launches = 0;  // as in StepGraph
+};
+
 struct Poisson {
   bool built = false;
+  long long alloc_epoch = 0;        // bumped when a buffer of the solver moves
+  std::vector<SolveGraph> graphs;   // at most kSolveGraphs, the least recently used first
   double *coef = nullptr;   // NSLOT * vec_ld(N) doubles (SoA by slot)
   int nslot = NSLOT;        // 7 when every cross slot is zero (the apply reads slots 0..6)
   uint8_t *fluid = nullptr; // 1 if the cell is a Poisson unknown (gid >= 0)
@@ -194,6 +212,7 @@ enum DScal {
   DS_INLET_FLUX = 0, DS_INLET_AREA, DS_MEAN_K_AREA,
   DS_KFLUX_SUM, DS_MEAN_K_FLUX, DS_FLUX1, DS_FLUX_IN, DS_FLUX_OUT, DS_AREA_OUT,
   DS_BSUM, DS_PHISUM, DS_MAXDIV, DS_VF_FLUX, DS_VF_AREA,
+  DS_NFLUID,  // number of Poisson unknowns (poisson_lhs)
   DS_COUNT = 16
 };
 
@@ -296,6 +315,7 @@ int reduce_to(Ctx *c, const double *parts, int nparts, double *dst);
 int ds_fetch(Ctx *c);
 int ds_upload(Ctx *c);
 void step_graph_free(Ctx *c);
+void solve_graphs_free(Poisson &P);
 
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 

@@ -1076,6 +1076,7 @@ int mg_setup(Ctx *c) {
       old[l] = MGLevel();  // taken
     } else {
       if (l < old.size()) { level_free(old[l]); old[l] = MGLevel(); }
+      P.alloc_epoch++;
       bool ok = cudaMalloc(&L.op64, sizeof(double) * NOP * n) == cudaSuccess;
       ok &= cudaMalloc(&L.pk64, sizeof(double) * 8 * n) == cudaSuccess;
       ok &= cudaMalloc(&L.pk32, sizeof(float) * 8 * n) == cudaSuccess;

@@ -483,6 +483,8 @@ int poisson_lhs(Ctx *c) {
   if ((rc = reduce_sum(c, c->red + kRedBlocks, kRedBlocks, &saj))) return rc;
   P.nfluid = (long long)llround(cnt);
   P.sum_aj = saj;
+  c->ds_in[DS_NFLUID] = (double)P.nfluid;
+  cudaMemcpyAsync(c->ds + DS_NFLUID, c->ds_in + DS_NFLUID, sizeof(double), cudaMemcpyHostToDevice, c->stream);
   // the apply reads only slots CP..BP when no row has a cross-derivative entry
   c->launches++, k_count_cross<<<kRedBlocks, 256, 0, c->stream>>>(N, vec_ld(N), P.coef, c->red);
   if ((rc = check_launch(c, "k_count_cross"))) return rc;
@@ -1026,12 +1028,11 @@ __global__ void k_lincomb_add_dyn(long long n, long long ldv, const B *__restric
   for (int t = 0; t < m; t++) s += kd->y[t] * (double)Z[(long long)t * ldv + p];
   x[p] = s;
 }
-// x += -sum / nfluid on the fluid cells (sum = ds[DS_PHISUM]).
-__global__ void k_shift_mean(long long n, const uint8_t *fluid, const double *__restrict__ ds, double nfluid,
-                             double *x) {
+// x += -sum / nfluid on the fluid cells (sum = ds[DS_PHISUM], nfluid = ds[DS_NFLUID]).
+__global__ void k_shift_mean(long long n, const uint8_t *fluid, const double *__restrict__ ds, double *x) {
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= n || !fluid[p]) return;
-  const double val = -ds[DS_PHISUM] / nfluid;
+  const double val = -ds[DS_PHISUM] / ds[DS_NFLUID];
   x[p] += val;
 }
 
@@ -1308,7 +1309,8 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
       (z64 || P.restart_z32 >= m))
     return VFS_OK;
   if (c->capturing) return set_err(c, VFS_ERR_STATE, "poisson_solve: Krylov basis not allocated before capture");
-  c->setup_epoch++;  // a captured step graph holds the old buffers
+  c->setup_epoch++;  // captured graphs hold the old buffers
+  P.alloc_epoch++;
   if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "poisson_solve: failed");
   P.ldv = ldv;
   bool ok = true;
@@ -1333,18 +1335,14 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   return VFS_OK;
 }
 
-int poisson_solve(Ctx *c, const vfs_solve_opts *oin, vfs_solve_stats *st) {
-  const vfs_solve_opts o = solve_opts(c, oin);
+// The kernels of a solve: launched one by one, the host driving the two loops, or captured.
+static int solve_kernels(Ctx *c, const vfs_solve_opts &o, bool warm, long long *body_launches, long long *cycle_launches) {
   Poisson &P = c->ps;
   const long long N = c->g.N;
   int rc;
-  if ((rc = poisson_prepare(c, &o))) return rc;
-  if ((rc = ensure_red(c, 34 * std::max(kKryBlocks, kry_grid(c)) + (int)nblocks(N, 256) + 64))) return rc;
-  if (!c->capturing) cudaEventRecord(c->ev0, c->stream);
   KryDev *kd = c->kd;
   double *x = c->f[VFS_PHI][0];
   const double *b = c->f[VFS_B][0];
-  const bool warm = P.guess && !o.zero_guess && !P.transpose;
   if (warm) {
     const int nb = (int)nblocks(N, 256);
     c->launches++, k_guess<<<nb, 256, 0, c->stream>>>(N, P.fluid, b, x, c->red);
@@ -1371,10 +1369,10 @@ int poisson_solve(Ctx *c, const vfs_solve_opts *oin, vfs_solve_stats *st) {
     if ((rc = while_begin(c, 1, h_inner, w1))) return rc;
     const long long l1 = c->launches;
     if ((rc = kry_body(c, o, (unsigned long long)h_inner, 1))) return rc;
-    c->sg.body_launches = c->launches - l1;
+    *body_launches = c->launches - l1;
     if ((rc = while_end(c, w1))) return rc;
     if ((rc = kry_cycle_end(c, o, b, x, (unsigned long long)h_outer, 1))) return rc;
-    c->sg.cycle_launches = c->launches - l0 - c->sg.body_launches;
+    *cycle_launches = c->launches - l0 - *body_launches;
     if ((rc = while_end(c, w0))) return rc;
   } else {
     for (;;) {
@@ -1396,25 +1394,125 @@ int poisson_solve(Ctx *c, const vfs_solve_opts *oin, vfs_solve_stats *st) {
     c->launches++, k_sum_fluid<<<nb, 256, 0, c->stream>>>(N, P.fluid, x, c->red);
     if ((rc = check_launch(c, "k_sum_fluid"))) return rc;
     if ((rc = reduce_to(c, c->red, nb, c->ds + DS_PHISUM))) return rc;
-    c->launches++, k_shift_mean<<<nblocks(N, 256), 256, 0, c->stream>>>(N, P.fluid, c->ds, (double)P.nfluid, x);
+    c->launches++, k_shift_mean<<<nblocks(N, 256), 256, 0, c->stream>>>(N, P.fluid, c->ds, x);
     if ((rc = check_launch(c, "k_shift_mean"))) return rc;
   }
   // Convert_Phi2_Phi: periodic ghosts take their images (x is 0 elsewhere off-fluid)
-  if ((rc = periodic_copy1(c, x))) return rc;
+  return periodic_copy1(c, x);
+}
+
+static void solve_graph_destroy(SolveGraph &G) {
+  if (G.exec) cudaGraphExecDestroy(G.exec);
+  if (G.graph) cudaGraphDestroy(G.graph);
+  G.exec = nullptr;
+  G.graph = nullptr;
+}
+void solve_graphs_free(Poisson &P) {
+  for (SolveGraph &G : P.graphs) solve_graph_destroy(G);
+  P.graphs.clear();
+}
+
+// Solves kept as graphs: a step's, and the tangent and adjoint solves' of a window.  No graph
+// is in flight when one is dropped: every solve ends with a synchronisation.
+constexpr size_t kSolveGraphs = 4;
+
+// The graph of this solve, captured at its second occurrence (a first solve would not earn
+// the capture back); null: launch the kernels.
+static SolveGraph *solve_graph(Ctx *c, const vfs_solve_opts &o, bool warm) {
+  Poisson &P = c->ps;
+  SolveKey key;
+  memset(&key, 0, sizeof(key));
+  key.o = o;
+  key.warm = warm;
+  key.transpose = P.transpose;
+  key.nslot = P.nslot;
+  key.alloc_epoch = P.alloc_epoch;
+  key.x = c->f[VFS_PHI][0];
+  key.b = c->f[VFS_B][0];
+  key.red = c->red;
+  size_t at = 0;
+  while (at < P.graphs.size() && memcmp(&P.graphs[at].key, &key, sizeof(key))) at++;
+  if (at == P.graphs.size()) {
+    if (P.graphs.size() == kSolveGraphs) {
+      solve_graph_destroy(P.graphs.front());
+      P.graphs.erase(P.graphs.begin());
+    }
+    SolveGraph G;
+    G.key = key;
+    P.graphs.push_back(G);
+    return nullptr;
+  }
+  std::rotate(P.graphs.begin() + at, P.graphs.begin() + at + 1, P.graphs.end());
+  SolveGraph &G = P.graphs.back();
+  if (G.exec) return &G;
+  if (G.failed) return nullptr;
+  const long long l0 = c->launches;
+  if (cudaStreamBeginCapture(c->stream, cudaStreamCaptureModeRelaxed) != cudaSuccess) {
+    cudaGetLastError();
+    G.failed = true;
+    return nullptr;
+  }
+  c->capturing = true;
+  const cudaStream_t own = c->stream;
+  const int rc = solve_kernels(c, o, warm, &G.body_launches, &G.cycle_launches);
+  c->capturing = false;
+  c->stream = own;
+  for (cudaStream_t q : c->cap_streams) {  // a loop body left open by an error
+    cudaStreamCaptureStatus cs;
+    cudaGraph_t open = nullptr;
+    if (q && cudaStreamIsCapturing(q, &cs) == cudaSuccess && cs != cudaStreamCaptureStatusNone) cudaStreamEndCapture(q, &open);
+  }
+  const cudaError_t e = cudaStreamEndCapture(c->stream, &G.graph);
+  if (rc || e != cudaSuccess || cudaGraphInstantiate(&G.exec, G.graph, 0) != cudaSuccess) {
+    cudaGetLastError();
+    if (G.graph) cudaGraphDestroy(G.graph);
+    G.graph = nullptr;
+    G.exec = nullptr;
+    G.failed = true;
+  }
+  G.launches = c->launches - l0;  // with one Krylov cycle and iteration
+  c->launches = l0;
+  return G.exec ? &G : nullptr;
+}
+
+int poisson_solve(Ctx *c, const vfs_solve_opts *oin, vfs_solve_stats *st) {
+  const vfs_solve_opts o = solve_opts(c, oin);
+  Poisson &P = c->ps;
+  KryDev *kd = c->kd;
+  int rc;
+  if ((rc = poisson_prepare(c, &o))) return rc;
+  if ((rc = ensure_red(c, 34 * kKryBlocks + (int)nblocks(c->g.N, 256) + 64))) return rc;
+  const bool warm = P.guess && !o.zero_guess && !P.transpose;
+  if (c->capturing) {  // inside a captured step: statistics after the replay
+    rc = solve_kernels(c, o, warm, &c->sg.body_launches, &c->sg.cycle_launches);
+    if (!rc && !P.transpose) P.guess = true;
+    return rc;
+  }
+  SolveGraph *G = solve_graph(c, o, warm);
+  cudaEventRecord(c->ev0, c->stream);
+  if (G) {
+    if (cudaGraphLaunch(G->exec, c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "poisson_solve: graph launch failed");
+  } else {
+    long long bl, cl;
+    if ((rc = solve_kernels(c, o, warm, &bl, &cl))) return rc;
+  }
   if (!P.transpose) P.guess = true;
-  if (c->capturing) return VFS_OK;  // statistics after the replay
   cudaEventRecord(c->ev1, c->stream);
   cudaMemcpyAsync(c->kd_host, kd, sizeof(KryDev), cudaMemcpyDeviceToHost, c->stream);
   if (cudaEventSynchronize(c->ev1) != cudaSuccess || cudaStreamSynchronize(c->stream) != cudaSuccess)
     return set_err(c, VFS_ERR_CUDA, "poisson_solve: failed");
+  const KryDev &k = *c->kd_host;
+  if (G)
+    c->launches += G->launches + (long long)(k.it > 0 ? k.it - 1 : 0) * G->body_launches +
+                   (long long)(k.cycles > 0 ? k.cycles - 1 : 0) * G->cycle_launches;
   float ms = 0;
   cudaEventElapsedTime(&ms, c->ev0, c->ev1);
   vfs_solve_stats s;
   memset(&s, 0, sizeof(s));
-  s.iterations = c->kd_host->it;
-  s.converged = c->kd_host->conv ? 1 : 0;
-  s.rfinal = c->kd_host->rnorm;
-  s.r0 = c->kd_host->r0;
+  s.iterations = k.it;
+  s.converged = k.conv ? 1 : 0;
+  s.rfinal = k.rnorm;
+  s.r0 = k.r0;
   s.ms = ms;
   if (st) *st = s;
   return s.converged ? VFS_OK : set_err(c, VFS_ERR_NOT_CONVERGED, "poisson_solve: iteration cap reached");
