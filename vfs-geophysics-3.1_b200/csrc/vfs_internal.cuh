@@ -317,6 +317,43 @@ int ds_upload(Ctx *c);
 void step_graph_free(Ctx *c);
 void solve_graphs_free(Poisson &P);
 
+// Programmatic dependent launch along the solver's chain of short kernels: a kernel may
+// start while its predecessor drains, reads what no kernel of a solve writes (the packed
+// operator), then waits for the predecessor grid to complete (and its writes to be visible)
+// before touching any vector; only then does it let its own successor start, so at most
+// two kernels of the chain are in flight and the results are those of plain stream order.
+// Outside such a launch both are no-ops.
+__device__ __forceinline__ void pdl_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+#ifndef VFS_PDL_CAPTURE
+#define VFS_PDL_CAPTURE 1
+#endif
+// Every launch is counted in the context's launch counter and its status is checked: the
+// return value of cudaLaunchKernelEx, then the sticky launch error.
+template <typename... KArgs, typename... Args>
+int launch_chain(Ctx *c, const char *what, void (*kernel)(KArgs...), unsigned grid, unsigned block,
+                        size_t smem, Args... args) {
+  c->launches++;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = c->stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = !c->capturing || VFS_PDL_CAPTURE ? 1 : 0;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    return set_err(c, VFS_ERR_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+  }
+  return check_launch(c, what);
+}
+
 inline unsigned nblocks(long long n, int bs) { return (unsigned)((n + bs - 1) / bs); }
 
 // momentum path

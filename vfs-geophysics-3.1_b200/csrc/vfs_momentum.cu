@@ -25,6 +25,7 @@ __device__ __forceinline__ double dot3(double ax, double ay, double az, double b
 // image, whose indices are all interior or non-periodic ghosts, so no thread reads a
 // point another one writes.
 __global__ void k_periodic_copy(Grid g, double *a, double *b, double *c) {
+  pdl_wait();
   long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   const long long ni = g.iper ? 2LL * g.my * g.mz : 0, nj = g.jper ? 2LL * g.mx * g.mz : 0;
   const long long nk = g.kper ? 2LL * g.mx * g.my : 0;
@@ -54,13 +55,12 @@ static long long ghost_points(const Grid &g) {
 
 int periodic_copy3(Ctx *c, V3 v) {
   if (!(c->g.iper || c->g.jper || c->g.kper)) return VFS_OK;
-  c->launches++, k_periodic_copy<<<nblocks(ghost_points(c->g), 256), 256, 0, c->stream>>>(c->g, v.x, v.y, v.z);
-  return check_launch(c, "k_periodic_copy");
+  return launch_chain(c, "k_periodic_copy", k_periodic_copy, nblocks(ghost_points(c->g), 256), 256, 0, c->g, v.x, v.y, v.z);
 }
 int periodic_copy1(Ctx *c, double *s) {
   if (!(c->g.iper || c->g.jper || c->g.kper)) return VFS_OK;
-  c->launches++, k_periodic_copy<<<nblocks(ghost_points(c->g), 256), 256, 0, c->stream>>>(c->g, s, nullptr, nullptr);
-  return check_launch(c, "k_periodic_copy");
+  return launch_chain(c, "k_periodic_copy", k_periodic_copy, nblocks(ghost_points(c->g), 256), 256, 0, c->g, s,
+                      (double *)nullptr, (double *)nullptr);
 }
 
 // ------------------------------------------------------------------ Contra2Cart
@@ -68,6 +68,7 @@ int periodic_copy1(Ctx *c, double *s) {
 // metrics (rhs.c:186-233).  Cells with nvert >= 0.1 keep their value.
 __global__ void k_contra2cart_interior(Grid g, CV3 uc, CV3 csi, CV3 eta, CV3 zet,
                                        const uint8_t *__restrict__ nv, V3 ucat) {
+  pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
   int i, j, k;
@@ -320,48 +321,41 @@ __device__ __forceinline__ long long edge_point(const Grid &g, long long t, int 
   return lidx(g, i, j, k);
 }
 
-__global__ void k_contra2cart_bc_edges(Grid g, Metrics m, const uint8_t *__restrict__ nv, CV3 lu, CV3 uo, V3 out,
-                                       uint8_t *flag) {
+// The boundary phase over its points: thread t < ne the edge points, then the ns listed solid
+// cells (nvert 3), which get zero (rhs.c:296-299).
+__global__ void k_contra2cart_bc_points(Grid g, Metrics m, const uint8_t *__restrict__ nv, CV3 lu, CV3 uo, V3 out,
+                                        uint8_t *flag, long long ne, long long ns, const long long *__restrict__ solid) {
+  pdl_wait();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= edge_points(g)) return;
-  int i, j, k;
-  const long long p = edge_point(g, t, i, j, k);
-  contra2cart_bc_point(g, m, nv, lu, uo, out, flag, p, i, j, k);
+  if (t < ne) {
+    int i, j, k;
+    const long long p = edge_point(g, t, i, j, k);
+    contra2cart_bc_point(g, m, nv, lu, uo, out, flag, p, i, j, k);
+  } else if (t < ne + ns) {
+    const long long p = solid[t - ne];
+    out.x[p] = 0; out.y[p] = 0; out.z[p] = 0;
+    flag[p] = 1;
+  }
 }
 
-// Solid cells (nvert 3) get zero (rhs.c:296-299), through the same two-phase buffer.
-__global__ void k_solid_zero(long long n, const long long *__restrict__ idx, V3 out, uint8_t *flag) {
+// Copies the marked values and clears the marks for the next call.  Of the two threads of a point
+// on two planes the second may find its mark cleared: the first has copied it.
+__global__ void k_bc_commit_points(Grid g, CV3 in, uint8_t *flag, V3 dst, long long ne, long long ns,
+                                   const long long *__restrict__ solid) {
+  pdl_wait();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const long long p = idx[t];
-  out.x[p] = 0; out.y[p] = 0; out.z[p] = 0;
-  flag[p] = 1;
-}
-
-__global__ void k_bc_commit_edges(Grid g, CV3 in, uint8_t *flag, V3 dst) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= edge_points(g)) return;
-  int i, j, k;
-  const long long p = edge_point(g, t, i, j, k);
-  if (!flag[p]) return;
+  long long p;
+  if (t < ne) {
+    int i, j, k;
+    p = edge_point(g, t, i, j, k);
+    if (!flag[p]) return;
+  } else if (t < ne + ns) {
+    p = solid[t - ne];
+  } else {
+    return;
+  }
   dst.x[p] = in.x[p]; dst.y[p] = in.y[p]; dst.z[p] = in.z[p];
-}
-__global__ void k_bc_commit_list(long long n, const long long *__restrict__ idx, CV3 in, V3 dst) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= n) return;
-  const long long p = idx[t];
-  dst.x[p] = in.x[p]; dst.y[p] = in.y[p]; dst.z[p] = in.z[p];
-}
-// Flags are cleared after every commit so the next call starts from zero.
-__global__ void k_bc_clear_edges(Grid g, uint8_t *flag) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= edge_points(g)) return;
-  int i, j, k;
-  flag[edge_point(g, t, i, j, k)] = 0;
-}
-__global__ void k_bc_clear_list(long long n, const long long *__restrict__ idx, uint8_t *flag) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t < n) flag[idx[t]] = 0;
+  flag[p] = 0;
 }
 
 // Indices of the solid (nvert 3) points, in any order.
@@ -430,9 +424,9 @@ int contra2cart_div(Ctx *c, bool with_divergence) {
   if (with_divergence)
     c->launches++, k_contra2cart_div<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, cv(uc), m.csi, m.eta, m.zet, m.aj,
                                                                                c->nv, ucat, c->red + 64);
-  else
-    c->launches++, k_contra2cart_interior<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, cv(uc), m.csi, m.eta, m.zet, c->nv,
-                                                                                    ucat);
+  else if ((rc = launch_chain(c, "k_contra2cart_interior", k_contra2cart_interior, nblocks(g.N, 256), 256, 0, g, cv(uc), m.csi,
+                              m.eta, m.zet, c->nv, ucat)))
+    return rc;
   if ((rc = check_launch(c, "k_contra2cart_interior"))) return rc;
   if ((rc = periodic_copy3(c, ucat))) return rc;
   V3 out{c->bcbuf[0], c->bcbuf[1], c->bcbuf[2]};
@@ -440,15 +434,11 @@ int contra2cart_div(Ctx *c, bool with_divergence) {
   if ((rc = solid_list(c))) return rc;
   // solid points get Ucat = 0, except with moving bodies (rhs.c:298)
   const long long ne = edge_points(g), ns = g.moving ? 0 : c->nsolid;
-  c->launches++, k_contra2cart_bc_edges<<<nblocks(ne, 256), 256, 0, c->stream>>>(g, m, c->nv, cv(ucat), cv(field3(c, VFS_UCAT_O)),
-                                                                  out, fl);
-  if (ns > 0) c->launches++, k_solid_zero<<<nblocks(ns, 256), 256, 0, c->stream>>>(ns, c->solid, out, fl);
-  if ((rc = check_launch(c, "k_contra2cart_bc"))) return rc;
-  c->launches++, k_bc_commit_edges<<<nblocks(ne, 256), 256, 0, c->stream>>>(g, cv(out), fl, ucat);
-  if (ns > 0) c->launches++, k_bc_commit_list<<<nblocks(ns, 256), 256, 0, c->stream>>>(ns, c->solid, cv(out), ucat);
-  c->launches++, k_bc_clear_edges<<<nblocks(ne, 256), 256, 0, c->stream>>>(g, fl);
-  if (ns > 0) c->launches++, k_bc_clear_list<<<nblocks(ns, 256), 256, 0, c->stream>>>(ns, c->solid, fl);
-  if ((rc = check_launch(c, "k_bc_commit"))) return rc;
+  if ((rc = launch_chain(c, "k_contra2cart_bc_points", k_contra2cart_bc_points, nblocks(ne + ns, 256), 256, 0, g, m, c->nv, cv(ucat),
+                         cv(field3(c, VFS_UCAT_O)), out, fl, ne, ns, c->solid)))
+    return rc;
+  if ((rc = launch_chain(c, "k_bc_commit_points", k_bc_commit_points, nblocks(ne + ns, 256), 256, 0, g, cv(out), fl, ucat, ne, ns, c->solid)))
+    return rc;
   return periodic_copy3(c, ucat);
 }
 
@@ -490,7 +480,7 @@ __global__ void k_c2c_bc_adjoint(Grid g, Metrics m, const uint8_t *__restrict__ 
   if (q >= g.N) return;
   int i, j, k;
   dijk(g, q, i, j, k);
-  const bool solid = nv[q] == 3 && !g.moving;  // k_solid_zero
+  const bool solid = nv[q] == 3 && !g.moving;  // the listed solid cells
   if (!c2c_near(g, i, j, k) && !solid) return;
   bool assigned = solid;
   double a[3] = {0.0, 0.0, 0.0}, o[3] = {0.0, 0.0, 0.0};
@@ -938,6 +928,7 @@ __global__ void __launch_bounds__(VFS_FF_THREADS, VFS_FF_MINB) k_face_flux(Grid 
                                                                            const uint8_t *__restrict__ nv,
                                                                            const double *__restrict__ nut, FluxOut f1,
                                                                            FluxOut f2, FluxOut f3) {
+  pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
   face_flux_point(g, m, uc, u, nv, nut, p, f1, f2, f3);
@@ -1074,6 +1065,7 @@ constexpr int kFpThreads = 64;
 __global__ void __launch_bounds__(kFpThreads, VFS_FP_MINB) k_fp(Grid g, FluxIn f1, FluxIn f2, FluxIn f3,
                                                          const uint8_t *__restrict__ nv, double *fpx, double *fpy,
                                                          double *fpz) {
+  pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
   fp_point(g, f1, f2, f3, nv, p, fpx, fpy, fpz);
@@ -1148,6 +1140,7 @@ struct GlobalFp {
 __global__ void k_rhs(Grid g, Metrics m, const uint8_t *__restrict__ nv, const double *__restrict__ fpx,
                       const double *__restrict__ fpy, const double *__restrict__ fpz, double scale,
                       V3 rhs, int rk, double a, CV3 dP, CV3 pu, V3 ucont) {
+  pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
   const int mx = g.mx, my = g.my, mz = g.mz;
@@ -1198,9 +1191,8 @@ static int face_fluxes(Ctx *c) {
   Metrics m = metrics(c);
   CV3 uc = cv(field3(c, VFS_UCONT)), u = cv(field3(c, VFS_UCAT));
   const unsigned nb = nblocks(g.N, VFS_FF_THREADS);
-  c->launches++, k_face_flux<<<nb, VFS_FF_THREADS, 0, c->stream>>>(g, m, uc, u, c->nv, c->f[VFS_NU_T][0], flux_out(c, 0),
-                                                    flux_out(c, 1), flux_out(c, 2));
-  return check_launch(c, "k_face_flux");
+  return launch_chain(c, "k_face_flux", k_face_flux, nb, VFS_FF_THREADS, 0, g, m, uc, u, c->nv, c->f[VFS_NU_T][0],
+                      flux_out(c, 0), flux_out(c, 1), flux_out(c, 2));
 }
 
 // Formfunction_2 as three kernels: face fluxes (written to 18 arrays), Fp, right-hand
@@ -1210,16 +1202,15 @@ int formfunction2_split(Ctx *c, double scale, bool rk_stage, double rk_coeff) {
   const Grid &g = c->g;
   int rc;
   V3 uc = field3(c, VFS_UCONT);
-  if ((rc = periodic_copy3(c, uc))) return rc;
+  // a Runge-Kutta stage follows the Contra2Cart of the same Ucont, which has made this copy
+  if (!rk_stage && (rc = periodic_copy3(c, uc))) return rc;
   Metrics m = metrics(c);
   if ((rc = face_fluxes(c))) return rc;
   launch_fp(c);
   if ((rc = check_launch(c, "k_fp"))) return rc;
   V3 pu{c->pucont[0], c->pucont[1], c->pucont[2]};
-  c->launches++, k_rhs<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, m, c->nv, c->fp[0], c->fp[1], c->fp[2], scale,
-                                                 field3(c, VFS_RHS), rk_stage ? 1 : 0, rk_coeff,
-                                                 cv(field3(c, VFS_DP)), cv(pu), uc);
-  return check_launch(c, "k_rhs");
+  return launch_chain(c, "k_rhs", k_rhs, nblocks(g.N, 256), 256, 0, g, m, c->nv, c->fp[0], c->fp[1], c->fp[2], scale,
+                      field3(c, VFS_RHS), rk_stage ? 1 : 0, rk_coeff, cv(field3(c, VFS_DP)), cv(pu), uc);
 }
 
 // One-pass Formfunction_2: face fluxes, Fp and the right-hand side (with the RK stage
@@ -1516,8 +1507,8 @@ int formfunction2(Ctx *c, double scale, bool rk_stage, double rk_coeff) {
 // single-kernel launchers for the diagnostics entry point (vfs_run_kernel)
 void launch_face_flux(Ctx *c) { face_fluxes(c); }
 void launch_fp(Ctx *c) {
-  c->launches++, k_fp<<<nblocks(c->g.N, kFpThreads), kFpThreads, 0, c->stream>>>(c->g, flux_in(c, 0), flux_in(c, 1), flux_in(c, 2), c->nv,
-                                                   c->fp[0], c->fp[1], c->fp[2]);
+  launch_chain(c, "k_fp", k_fp, nblocks(c->g.N, kFpThreads), kFpThreads, 0, c->g, flux_in(c, 0), flux_in(c, 1), flux_in(c, 2),
+               c->nv, c->fp[0], c->fp[1], c->fp[2]);
 }
 void launch_rhs(Ctx *c) {
   V3 pu{c->pucont[0], c->pucont[1], c->pucont[2]};

@@ -785,6 +785,7 @@ template <int NS, bool kT, typename B, typename ZT>
 __global__ void __launch_bounds__(kApplyThreads) k_apply_dyn(Grid g, long long ldv, const double *__restrict__ coef,
                                                    const ZT *__restrict__ Z, const KryDev *__restrict__ kd,
                                                    B *__restrict__ w) {
+  pdl_wait();
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
   w[p] = (B)op_row<NS, kT>(g, coef, Z + (long long)kd->j * ldv, p);
@@ -824,6 +825,7 @@ template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_multidot(long long N, long long ldv,
                                                                          const B *__restrict__ V, KryDev *kd,
                                                                          const B *__restrict__ w, double *parts) {
+  pdl_wait();
   const int nv = kd->j + 1;
   if (nv <= 4) multidot_body<4>(N, ldv, V, nv, w, parts);
   else if (nv <= 8) multidot_body<8>(N, ldv, V, nv, w, parts);
@@ -887,6 +889,7 @@ template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_reorth(long long n, long long ldv,
                                                                        const B *__restrict__ V, KryDev *kd,
                                                                        B *__restrict__ w, double *parts) {
+  pdl_wait();
   if (!kd->reorth) return;
   const int nv = kd->j + 1;
   update_dots<B>(n, ldv, V, nv, kd->h, w, parts);
@@ -900,6 +903,7 @@ __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_hessenberg(long l
                                                                            const B *__restrict__ V, KryDev *kd,
                                                                            B *__restrict__ w, double *parts,
                                                                            unsigned long long h_inner, int use_graph) {
+  pdl_wait();
   if (kd->reorth && kd->degen) {
     const int nv = kd->j + 1;
     update_dots<B>(n, ldv, V, nv, kd->h2, w, parts);
@@ -949,6 +953,7 @@ template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_next_vector(long long N, long long ldv, B *V,
                                                                             const KryDev *__restrict__ kd,
                                                                             const B *__restrict__ w) {
+  pdl_wait();
   if (!kd->inner_go) return;
   const int jd = kd->jdone;
   B *o = V + (long long)jd * ldv;
@@ -1137,19 +1142,20 @@ static int kry_body_t(Ctx *c, const vfs_solve_opts &o, unsigned long long h_inne
   int rc;
   if ((rc = mg_precondition(c, DynPtrT<const B>{V, P.ldv, &kd->j, 0}, DynPtrT<ZT>{Z, P.ldv, &kd->j, 0}, o)))
     return rc;  // z_j = M^-1 v_j
-#define VFS_APPLY(NS, T) c->launches++, k_apply_dyn<NS, T><<<nblocks(N, kApplyThreads), kApplyThreads, 0, c->stream>>>(c->g, P.ldv, P.coef, Z, kd, w)
+#define VFS_APPLY(NS, T) \
+  rc = launch_chain(c, "k_apply_dyn", k_apply_dyn<NS, T, B, ZT>, nblocks(N, kApplyThreads), kApplyThreads, 0, c->g, P.ldv, P.coef, Z, kd, w)
   if (P.transpose) {
     if (P.nslot == 7) VFS_APPLY(7, true); else VFS_APPLY(NSLOT, true);
   } else {
     if (P.nslot == 7) VFS_APPLY(7, false); else VFS_APPLY(NSLOT, false);
   }
 #undef VFS_APPLY
-  if ((rc = check_launch(c, "k_apply_dyn"))) return rc;
-  c->launches++, k_multidot<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red);
-  c->launches++, k_reorth<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red);
-  c->launches++, k_hessenberg<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w, c->red, h_inner, use_graph);
-  c->launches++, k_next_vector<B><<<kg, kKryThreads, 0, c->stream>>>(N, P.ldv, V, kd, w);
-  return check_launch(c, "FGMRES Arnoldi step");
+  if (rc) return rc;
+  if ((rc = launch_chain(c, "k_multidot", k_multidot<B>, kg, kKryThreads, 0, N, P.ldv, V, kd, w, c->red))) return rc;
+  if ((rc = launch_chain(c, "k_reorth", k_reorth<B>, kg, kKryThreads, 0, N, P.ldv, V, kd, w, c->red))) return rc;
+  if ((rc = launch_chain(c, "k_hessenberg", k_hessenberg<B>, kg, kKryThreads, 0, N, P.ldv, V, kd, w, c->red, h_inner, use_graph)))
+    return rc;
+  return launch_chain(c, "k_next_vector", k_next_vector<B>, kg, kKryThreads, 0, N, P.ldv, V, kd, w);
 }
 
 static bool fp32_inner(const vfs_solve_opts &o) { return o.precision == 2; }
