@@ -320,11 +320,10 @@ __device__ __forceinline__ void zload(const ZL &L, const Q4<T> *__restrict__ cpl
 // d_j = r_j / pivot - (cs_j / pivot) d_{j-1} and the back substitution
 // x_j = d_j - cpr_j x_{j+1} as first-order linear recurrences: each lane composes its rows,
 // a shuffle scan combines the lanes, each lane then replays its rows.  Every lane of the
-// warp takes part; `omega` is used by line Jacobi only (kJac: xr is the previous iterate);
-// kFull: all 32 lanes hold rows (ls = 32).
-template <typename T, int SEG, bool kJac, bool kFull>
+// warp takes part.  kFull: all 32 lanes hold rows (ls = 32).
+template <typename T, int SEG, bool kFull>
 __device__ __forceinline__ void zsolve(const ZL &L, const ZCol &z, int l, const ZRows<T, SEG> &R, const T *b,
-                                       const T *xr, T *xw, int flags, T omega) {
+                                       const T *xr, T *xw, int flags) {
   const unsigned q0 = z.p0 + (unsigned)l;
   const int ls = kFull ? 32 : L.ls, lw = kFull ? 32 : L.lw;
   const bool own = kFull || l < ls;
@@ -384,19 +383,12 @@ __device__ __forceinline__ void zsolve(const ZL &L, const ZCol &z, int l, const 
   for (int s = SEG - 1; s >= 0; s--) { x = -R.cx[s] * x + r[s]; r[s] = x; }
   if (!z.valid || !own) return;
 #pragma unroll
-  for (int s = 0; s < SEG; s++) {
-    const unsigned q = q0 + (unsigned)(s * ls);
-    if (kJac) {
-      const T xo = (flags & Z_OWN_ZERO) ? T(0) : xr[q];
-      xw[q] = xo + omega * (r[s] - xo);
-    } else {
-      xw[q] = r[s];
-    }
-  }
+  for (int s = 0; s < SEG; s++) xw[q0 + (unsigned)(s * ls)] = r[s];
 }
 
 // The same for columns of more rows per lane than the register forms take: the rows are
 // replayed through the column's own slots of xw, which no other column of the pass reads.
+// kJac: damped by omega against the previous iterate xr.
 template <typename T, bool kJac>
 __device__ void zsolve_long(const ZL &L, const ZCol &z, int l, const Q4<T> *__restrict__ cpl,
                             const Q2<T> *__restrict__ tri, const T *__restrict__ cpr, const T *b, const T *xr, T *xw,
@@ -508,14 +500,8 @@ __device__ __forceinline__ void thomas_rows(T *r, const T *lo, const T *id, cons
 // operator 28, b 4, the other colour's x 4, x 4); registers set the occupancy.  SEG = 0: columns
 // of more than eight rows a lane.
 template <typename T> struct ZBounds;
-#ifndef VFS_ZCOL_MINB32
-#define VFS_ZCOL_MINB32 5
-#endif
-#ifndef VFS_ZCOL_MINB64
-#define VFS_ZCOL_MINB64 3
-#endif
-template <> struct ZBounds<float> { static constexpr int v = VFS_ZCOL_MINB32; };
-template <> struct ZBounds<double> { static constexpr int v = VFS_ZCOL_MINB64; };
+template <> struct ZBounds<float> { static constexpr int v = 5; };
+template <> struct ZBounds<double> { static constexpr int v = 3; };
 constexpr int kColThreads = 128;
 template <typename T>
 struct ZOp {
@@ -533,14 +519,15 @@ __global__ void __launch_bounds__(kColThreads, ZBounds<T>::v) k_zcol(ZL L, ZOp<T
     ZRows<T, SEG> R;
     zload<T, SEG, kFull>(L, op.cpl, op.tri, op.cpr, z.p0, l, flags, R);
     pdl_wait();
-    zsolve<T, SEG, false, kFull>(L, z, l, R, b, x, x, flags, T(1));
+    zsolve<T, SEG, kFull>(L, z, l, R, b, x, x, flags);
   } else {
     pdl_wait();
     zsolve_long<T, false>(L, z, l, op.cpl, op.tri, op.cpr, b, x, x, flags, T(1));
   }
 }
 
-// A pass over columns too long for the kernel below, by lane groups.
+// A line Jacobi sweep or a small level's pass over columns too long for the kernel below, by lane
+// groups.
 template <typename T, bool kJac>
 __global__ void __launch_bounds__(kColThreads) k_zlong(ZL L, ZOp<T> op, const T *b, const T *xr, T *xw, int colour,
                                                        int flags, T omega) {
@@ -744,6 +731,50 @@ __global__ void __launch_bounds__(128) k_zprolong(ZL F, ZL C, const unsigned lon
   zprolong_cell<T, kColour1>(F, C, mask, x, xc, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
+// The same prolongation, one colour-1 fine cell per thread: eight coarse values in flight instead
+// of 27 and four times the threads.  The coarse-centric form loads less, this one waits less:
+// it serves the levels too small to fill the GPU (kFineProlong: up to 64^3 cells; a whole step of
+// 12 x 10 x 14 cells 668 -> 606 us, of 64^3 1572 -> 1528, while at 256 x 192 x 256 it costs a
+// V-cycle 35 us).
+template <typename T>
+__global__ void __launch_bounds__(128) k_zprolong_fine(ZL F, ZL C, const unsigned long long *__restrict__ mask, T *x,
+                                                       const T *__restrict__ xc) {
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned col = t / (unsigned)F.S, pos = t - col * (unsigned)F.S;
+  const unsigned k = col / (unsigned)F.hx, h = col - k * (unsigned)F.hx;
+  const int j = zrow_of(F, pos), i = (int)(2 * h + (1 ^ (k & 1)));
+  const bool cell = k < (unsigned)F.nz && j < F.ny && i < F.nx;
+  if (!cell) { pdl_wait(); return; }
+  const int I = i >> 1, J = j >> 1, K = (int)k >> 1, ai = i & 1, aj = j & 1, ak = (int)k & 1;
+  // the other nearest coarse cell along each direction (the cell itself where there is none: masked out)
+  auto other = [](int v, int up, int n, int per) {
+    const int w = up ? v + 1 : v - 1;
+    return w < 0 ? (per ? n - 1 : v) : (w >= n ? (per ? 0 : v) : w);
+  };
+  const int In = other(I, ai, C.nx, C.ip), Jn = other(J, aj, C.ny, C.jp), Kn = other(K, ak, C.nz, C.kp);
+  const unsigned c00 = zcol(C, I, K), c10 = zcol(C, In, K), c01 = zcol(C, I, Kn), c11 = zcol(C, In, Kn);
+  const unsigned r0 = zrow(C, J), r1 = zrow(C, Jn);
+  const unsigned q = ((k * 2 + 1) * (unsigned)F.hx + h) * (unsigned)F.S + pos;
+  const unsigned long long ok = mask[c00 + r0];
+  pdl_wait();
+  const T xo = xc[c00 + r0];
+  const T v[8] = {xo, xc[c10 + r0], xc[c00 + r1], xc[c10 + r1], xc[c01 + r0], xc[c11 + r0], xc[c01 + r1], xc[c11 + r1]};
+  const T xq = x[q];
+  const int di = ai ? 2 : 0, dj = aj ? 2 : 0, dk = ak ? 2 : 0;
+  T wown = T(27) / T(64);
+  T s = 0;
+#pragma unroll
+  for (int n = 1; n < 8; n++) {
+    const int a = n & 1, bb = (n >> 1) & 1, c = n >> 2;
+    const T w = (a ? T(1) : T(3)) * (bb ? T(1) : T(3)) * (c ? T(1) : T(3)) / T(64);
+    const int e = (a ? di : 1) + 3 * (bb ? dj : 1) + 9 * (c ? dk : 1);
+    if (!((ok >> e) & 1ull)) { wown += w; continue; }
+    s += w * v[n];
+  }
+  if ((ok >> (27 + ai + 2 * aj + 4 * ak)) & 1ull) x[q] = xq + (s + wown * xo);
+}
+constexpr long long kFineProlong = 64 * 64 * 64;  // cells of the fine level
+
 // ------------------------------------------------------------------ bottom of the V-cycle
 // The coarse levels are too small to fill the GPU, and a launch per colour pass costs more
 // than the work.  From the first level of at most kSerialCells cells down, one thread block
@@ -753,10 +784,7 @@ __global__ void __launch_bounds__(128) k_zprolong(ZL F, ZL C, const unsigned lon
 // to L2.  Starting at 4096 cells (lane groups in the same block) took 156 us a V-cycle of
 // 64^3 cells against 133 (FP32); a cluster of eight blocks exchanging through L2 186.
 constexpr int kBottomMaxLevels = 12;
-#ifndef VFS_BOTTOM_THREADS
-#define VFS_BOTTOM_THREADS 512
-#endif
-constexpr int kBottomThreads = VFS_BOTTOM_THREADS;
+constexpr int kBottomThreads = 512;
 constexpr size_t kBottomSmem = 200 * 1024;
 
 template <typename T>
@@ -1237,9 +1265,13 @@ static int mg_vcycle(const VCycle<T> &V, int l) {
             : launch_chain(c, "k_zrestrict", k_zrestrict<T, false>, nb, 128, 0, F.z, C.z, f.cpl, f.tri, f.dg, f.x, f.b, cc.b);
   if (rc) return rc;
   if ((rc = mg_vcycle<T>(V, l + 1))) return rc;
-  rc = half && V.o.post_smooth > 0
-           ? launch_chain(c, "k_zprolong", k_zprolong<T, true>, nb, 128, 0, F.z, C.z, C.pmask, f.x, cc.x)
-           : launch_chain(c, "k_zprolong", k_zprolong<T, false>, nb, 128, 0, F.z, C.z, C.pmask, f.x, cc.x);
+  if (half && V.o.post_smooth > 0 && (long long)F.z.nx * F.z.ny * F.z.nz <= kFineProlong)
+    rc = launch_chain(c, "k_zprolong", k_zprolong_fine<T>, nblocks((long long)F.z.nz * F.z.hx * F.z.S, 128), 128, 0, F.z, C.z,
+                      C.pmask, f.x, cc.x);
+  else
+    rc = half && V.o.post_smooth > 0
+             ? launch_chain(c, "k_zprolong", k_zprolong<T, true>, nb, 128, 0, F.z, C.z, C.pmask, f.x, cc.x)
+             : launch_chain(c, "k_zprolong", k_zprolong<T, false>, nb, 128, 0, F.z, C.z, C.pmask, f.x, cc.x);
   if (rc) return rc;
   return mg_smooth<T>(V, l, V.o.post_smooth, false);
 }

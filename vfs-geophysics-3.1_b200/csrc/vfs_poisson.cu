@@ -320,7 +320,8 @@ int poisson_apply_dev(Ctx *c, const double *x, double *y) {
 // ------------------------------------------------------------------ Krylov kernels
 // The FGMRES vectors are exactly zero off the unknowns, so every dot product runs over
 // the whole grid layout.  Reductions are deterministic: per-thread sums in a fixed order,
-// warp shuffles, a fixed-order sum over warps, then k_sum_rows over the block partials.
+// warp shuffles, a fixed-order sum over warps, then the last block's sum_rows over the block
+// partials.
 #ifndef VFS_KRY_BLOCKS_PER_SM
 #define VFS_KRY_BLOCKS_PER_SM 4
 #endif
