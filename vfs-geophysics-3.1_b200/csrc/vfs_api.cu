@@ -320,6 +320,7 @@ int vfs_destroy(vfs_ctx *ctx) {
   if (c->ibv) cudaFree(c->ibv);
   if (c->bcflag) cudaFree(c->bcflag);
   if (c->solid) cudaFree(c->solid);
+  if (c->irr) cudaFree(c->irr);
   for (int d = 0; d < 3; d++)
     for (int q = 0; q < 3; q++) { cudaFree(c->div[d][q]); cudaFree(c->visc[d][q]); }
   for (int q = 0; q < 3; q++) { cudaFree(c->fp[q]); cudaFree(c->pucont[q]); cudaFree(c->bcbuf[q]); }

@@ -266,6 +266,9 @@ struct Ctx {
   uint8_t *bcflag = nullptr;    // points written by the boundary phase
   long long *solid = nullptr;   // indices of the solid (nvert 3) points
   long long nsolid = -1;        // their number; -1 until built for the current nvert
+  long long *irr = nullptr;     // points with faces outside the interior form of Formfunction_2
+  long long nirr = 0;           // their number (valid with nsolid)
+  long long solid_cap = 0, irr_cap = 0;
   // reductions
   double *red = nullptr;        // partial sums (device)
   double *red_host = nullptr;   // pinned host mirror

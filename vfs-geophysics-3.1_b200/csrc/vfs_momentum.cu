@@ -358,13 +358,31 @@ __global__ void k_bc_commit_points(Grid g, CV3 in, uint8_t *flag, V3 dst, long l
   flag[p] = 0;
 }
 
-// Indices of the solid (nvert 3) points, in any order.
-__global__ void k_collect_solid(long long n, const uint8_t *__restrict__ nv, long long *idx,
-                                unsigned long long *count) {
+__device__ __forceinline__ bool regular_faces(const uint8_t *__restrict__ nv, long long p, long long sy, long long sz);
+
+// Interior form of the three faces of point (i, j, k): none of them next to a boundary or a periodic
+// image (only a face's own direction matters), no solid or IB node in their stencils.
+__device__ __forceinline__ bool regular_flux_point(const Grid &g, const uint8_t *__restrict__ nv, long long p, int i,
+                                                   int j, int k) {
+  return i >= 1 && i <= g.mx - 3 && j >= 1 && j <= g.my - 3 && k >= 1 && k <= g.mz - 3 &&
+         regular_faces(nv, p, g.mx, (long long)g.mx * g.my);
+}
+
+// Indices, in any order, of the solid (nvert 3) points and of the points with faces that do not
+// take the interior form of Formfunction_2; n[0] and n[1] count them.
+__global__ void k_collect_points(Grid g, const uint8_t *__restrict__ nv, long long *solid, long long *irr,
+                                 unsigned long long *n) {
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= n || nv[p] != 3) return;
-  const unsigned long long s = atomicAdd(count, 1ull);
-  if (idx) idx[s] = p;
+  if (p >= g.N) return;
+  if (nv[p] == 3) {
+    const unsigned long long s = atomicAdd(n, 1ull);
+    if (solid) solid[s] = p;
+  }
+  int i, j, k;
+  dijk(g, p, i, j, k);
+  if (i == g.mx - 1 || j == g.my - 1 || k == g.mz - 1 || regular_flux_point(g, nv, p, i, j, k)) return;
+  const unsigned long long s = atomicAdd(n + 1, 1ull);
+  if (irr) irr[s] = p;
 }
 
 __global__ void k_bc_commit(long long n, CV3 in, uint8_t *flag, V3 dst) {
@@ -375,27 +393,35 @@ __global__ void k_bc_commit(long long n, CV3 in, uint8_t *flag, V3 dst) {
   flag[p] = 0;
 }
 
-// The solid-point list is built once per nvert field (the count, then the indices).
+// The point lists are built once per nvert field (the counts, then the indices) in arrays that
+// only grow: a moving body has a new nvert field every step.
+static int grow_list(Ctx *c, long long *&list, long long &cap, long long n) {
+  if (n <= cap) return VFS_OK;
+  cudaFree(list);
+  list = nullptr;
+  cap = 0;
+  if (cudaMalloc(&list, sizeof(long long) * (size_t)(n + n / 8)) != cudaSuccess)
+    return set_err(c, VFS_ERR_CUDA, "point lists: allocation failed");
+  cap = n + n / 8;
+  return VFS_OK;
+}
 int solid_list(Ctx *c) {
   if (c->nsolid >= 0) return VFS_OK;
   int rc;
   if ((rc = ensure_red(c, 64))) return rc;
   unsigned long long *cnt = (unsigned long long *)(c->red + 62);
-  cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), c->stream);
-  c->launches++, k_collect_solid<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g.N, c->nv, nullptr, cnt);
-  unsigned long long n = 0;
-  cudaMemcpyAsync(&n, cnt, sizeof(n), cudaMemcpyDeviceToHost, c->stream);
-  if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "solid_list: count failed");
-  cudaFree(c->solid);
-  c->solid = nullptr;
-  if (n > 0) {
-    if (cudaMalloc(&c->solid, sizeof(long long) * n) != cudaSuccess)
-      return set_err(c, VFS_ERR_CUDA, "solid_list: allocation failed");
-    cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), c->stream);
-    c->launches++, k_collect_solid<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g.N, c->nv, c->solid, cnt);
-    if ((rc = check_launch(c, "k_collect_solid"))) return rc;
-  }
-  c->nsolid = (long long)n;
+  cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), c->stream);
+  c->launches++, k_collect_points<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, c->nv, nullptr, nullptr, cnt);
+  unsigned long long n[2] = {0, 0};
+  cudaMemcpyAsync(n, cnt, sizeof(n), cudaMemcpyDeviceToHost, c->stream);
+  if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "point lists: count failed");
+  if ((rc = grow_list(c, c->solid, c->solid_cap, (long long)n[0])) || (rc = grow_list(c, c->irr, c->irr_cap, (long long)n[1])))
+    return rc;
+  cudaMemsetAsync(cnt, 0, 2 * sizeof(unsigned long long), c->stream);
+  c->launches++, k_collect_points<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, c->nv, c->solid, c->irr, cnt);
+  if ((rc = check_launch(c, "k_collect_points"))) return rc;
+  c->nsolid = (long long)n[0];
+  c->nirr = (long long)n[1];
   c->setup_epoch++;
   return VFS_OK;
 }
@@ -868,70 +894,66 @@ __device__ __forceinline__ bool regular_faces(const uint8_t *__restrict__ nv, lo
   return s == 0;
 }
 
-// One thread per DA point (i,j,k) with i<mx-1, j<my-1, k<mz-1: computes the fluxes of
-// its i-face (if j,k >= 1), j-face (if i,k >= 1) and k-face (if i,j >= 1), following
-// the three face loops of Formfunction_2 (momentum.c:671-1415).
-// Points whose whole stencil is regular fluid interior take a branch-free path with
-// constant offsets (regular_faces); the rest run the general form.
-// Launch shape: VFS_FF_THREADS threads per block, at least VFS_FF_MINB blocks per SM (the
-// register cap that follows from it sets the occupancy of this latency-bound kernel:
-// 5 blocks cap it at 96 registers, which at 256 x 192 x 256 runs Formfunction_2 in
-// 2.20 ms against 2.50 ms uncapped at 154 registers and 2.45 ms at 64).
-#ifndef VFS_FF_THREADS
-#define VFS_FF_THREADS 128
-#endif
-#ifndef VFS_FF_MINB
-#define VFS_FF_MINB 5
-#endif
-__device__ __forceinline__ void face_flux_point(const Grid &g, const Metrics &m, CV3 uc, CV3 u,
-                                                const uint8_t *__restrict__ nv, const double *__restrict__ nut,
-                                                long long p, const FluxOut &f1, const FluxOut &f2, const FluxOut &f3) {
-  const int mx = g.mx, my = g.my, mz = g.mz;
+// The fluxes of the i-face (if j, k >= 1), j-face (if i, k >= 1) and k-face (if i, j >= 1) of
+// every DA point with i < mx-1, j < my-1, k < mz-1, following the three face loops of
+// Formfunction_2 (momentum.c:671-1415).  Points whose whole stencil is regular fluid interior
+// take a branch-free path with constant offsets, one thread per point; the others are listed
+// (solid_list) and take the general form in a launch of their own, one thread per listed face.
+// Both forms in one thread cost 1360 us at 256 x 192 x 256: a warp with one boundary or body point
+// ran both, a fifth of all warps, and the general form's registers spilled.  Apart, the
+// interior form is 1010 us (bound by the latency of its velocity loads at 24 warps per SM; 80
+// registers, 5 blocks per SM at 96: 1020, 8 at 64: 1060), the listed faces 180; in the first blocks
+// of the same launch, 1215 together (their registers spill at 80).
+constexpr int kFluxThreads = 128;
+__device__ __forceinline__ void put_flux(const FluxOut &f, long long p, const double d[3], const double v[3]) {
+  f.div[0][p] = d[0]; f.div[1][p] = d[1]; f.div[2][p] = d[2];
+  f.visc[0][p] = v[0]; f.visc[1][p] = v[1]; f.visc[2][p] = v[2];
+}
+// 128 registers (6 blocks per SM at 80: 196 us at 128 x 96 x 128 for both launches against 182).
+__global__ void __launch_bounds__(kFluxThreads, 4)
+    k_face_flux_listed(Grid g, Metrics m, CV3 uc, CV3 u, const uint8_t *__restrict__ nv,
+                       const double *__restrict__ nut, FluxOut f1, FluxOut f2, FluxOut f3, unsigned n,
+                       const long long *__restrict__ list) {
+  pdl_wait();
+  const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
+  const unsigned dir = t / n;
+  if (dir > 2) return;
+  const long long p = list[t - dir * n];
   int i, j, k;
   dijk(g, p, i, j, k);
-  if (i == mx - 1 || j == my - 1 || k == mz - 1) return;
   double d[3], v[3];
-  const long long sy = mx, sz = (long long)mx * my;
-  if (i >= 2 && i <= mx - 3 && j >= 2 && j <= my - 3 && k >= 2 && k <= mz - 3 &&
-      regular_faces(nv, p, sy, sz)) {
-    // Away from walls, periodic images, the outlet plane and solid cells every branch of
-    // the three face fluxes takes its interior form: the same arithmetic with constant offsets.
-    flux_i<true>(g, m, uc, u, nv, nut, p, i, j, k, d, v);
-    f1.div[0][p] = d[0]; f1.div[1][p] = d[1]; f1.div[2][p] = d[2];
-    f1.visc[0][p] = v[0]; f1.visc[1][p] = v[1]; f1.visc[2][p] = v[2];
-    flux_j<true>(g, m, uc, u, nv, nut, p, i, j, k, d, v);
-    f2.div[0][p] = d[0]; f2.div[1][p] = d[1]; f2.div[2][p] = d[2];
-    f2.visc[0][p] = v[0]; f2.visc[1][p] = v[1]; f2.visc[2][p] = v[2];
-    flux_k<true>(g, m, uc, u, nv, nut, p, i, j, k, d, v);
-    f3.div[0][p] = d[0]; f3.div[1][p] = d[1]; f3.div[2][p] = d[2];
-    f3.visc[0][p] = v[0]; f3.visc[1][p] = v[1]; f3.visc[2][p] = v[2];
-    return;
-  }
-  if (j != 0 && k != 0) {
+  if (dir == 0) {
+    if (j == 0 || k == 0) return;
     flux_i(g, m, uc, u, nv, nut, p, i, j, k, d, v);
-    f1.div[0][p] = d[0]; f1.div[1][p] = d[1]; f1.div[2][p] = d[2];
-    f1.visc[0][p] = v[0]; f1.visc[1][p] = v[1]; f1.visc[2][p] = v[2];
-  }
-  if (i != 0 && k != 0) {
+    put_flux(f1, p, d, v);
+  } else if (dir == 1) {
+    if (i == 0 || k == 0) return;
     flux_j(g, m, uc, u, nv, nut, p, i, j, k, d, v);
-    f2.div[0][p] = d[0]; f2.div[1][p] = d[1]; f2.div[2][p] = d[2];
-    f2.visc[0][p] = v[0]; f2.visc[1][p] = v[1]; f2.visc[2][p] = v[2];
-  }
-  if (i != 0 && j != 0) {
+    put_flux(f2, p, d, v);
+  } else {
+    if (i == 0 || j == 0) return;
     flux_k(g, m, uc, u, nv, nut, p, i, j, k, d, v);
-    f3.div[0][p] = d[0]; f3.div[1][p] = d[1]; f3.div[2][p] = d[2];
-    f3.visc[0][p] = v[0]; f3.visc[1][p] = v[1]; f3.visc[2][p] = v[2];
+    put_flux(f3, p, d, v);
   }
 }
 
-__global__ void __launch_bounds__(VFS_FF_THREADS, VFS_FF_MINB) k_face_flux(Grid g, Metrics m, CV3 uc, CV3 u,
-                                                                           const uint8_t *__restrict__ nv,
-                                                                           const double *__restrict__ nut, FluxOut f1,
-                                                                           FluxOut f2, FluxOut f3) {
+__global__ void __launch_bounds__(kFluxThreads, 6) k_face_flux(Grid g, Metrics m, CV3 uc, CV3 u,
+                                                               const uint8_t *__restrict__ nv,
+                                                               const double *__restrict__ nut, FluxOut f1,
+                                                               FluxOut f2, FluxOut f3) {
   pdl_wait();
-  long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
-  face_flux_point(g, m, uc, u, nv, nut, p, f1, f2, f3);
+  int i, j, k;
+  dijk(g, p, i, j, k);
+  if (!regular_flux_point(g, nv, p, i, j, k)) return;
+  double d[3], v[3];
+  flux_i<true>(g, m, uc, u, nv, nut, p, i, j, k, d, v);
+  put_flux(f1, p, d, v);
+  flux_j<true>(g, m, uc, u, nv, nut, p, i, j, k, d, v);
+  put_flux(f2, p, d, v);
+  flux_k<true>(g, m, uc, u, nv, nut, p, i, j, k, d, v);
+  put_flux(f3, p, d, v);
 }
 
 // Fp at interior cells: 4th-order divergence correction 9/8*div - 1/8*wide/denom plus the
@@ -1184,15 +1206,22 @@ static FluxIn flux_in(Ctx *c, int d) {
 
 void launch_fp(Ctx *c);
 
-// The 18 face-flux arrays of Formfunction_2 (one launch for the three face directions;
-// one launch per direction measured 30 % slower on the B200).
+// The 18 face-flux arrays of Formfunction_2 (one launch for the three directions of the interior
+// form; one launch per direction measured 30 % slower, a warp per direction 40 %).
 static int face_fluxes(Ctx *c) {
   const Grid &g = c->g;
   Metrics m = metrics(c);
   CV3 uc = cv(field3(c, VFS_UCONT)), u = cv(field3(c, VFS_UCAT));
-  const unsigned nb = nblocks(g.N, VFS_FF_THREADS);
-  return launch_chain(c, "k_face_flux", k_face_flux, nb, VFS_FF_THREADS, 0, g, m, uc, u, c->nv, c->f[VFS_NU_T][0],
-                      flux_out(c, 0), flux_out(c, 1), flux_out(c, 2));
+  int rc;
+  if ((rc = solid_list(c))) return rc;
+  const unsigned n = (unsigned)c->nirr;
+  const double *nut = c->f[VFS_NU_T][0];
+  const FluxOut f1 = flux_out(c, 0), f2 = flux_out(c, 1), f3 = flux_out(c, 2);
+  if (n > 0 && (rc = launch_chain(c, "k_face_flux_listed", k_face_flux_listed, nblocks(3LL * n, kFluxThreads), kFluxThreads,
+                                  0, g, m, uc, u, c->nv, nut, f1, f2, f3, n, c->irr)))
+    return rc;
+  return launch_chain(c, "k_face_flux", k_face_flux, nblocks(g.N, kFluxThreads), kFluxThreads, 0, g, m, uc, u, c->nv, nut,
+                      f1, f2, f3);
 }
 
 // Formfunction_2 as three kernels: face fluxes (written to 18 arrays), Fp, right-hand
@@ -1256,8 +1285,8 @@ struct MarchSmem {
 
 // Fluxes of one face; zero where the face does not exist.  reg: the point's whole flux
 // stencil is regular fluid interior (regular_faces), so the branch-free form applies.
-// True when the three faces of point (i, j, k) take the interior form (face_flux_point's
-// test); false for a point that does not exist.
+// True when the three faces of point (i, j, k) take the interior form (the split form's test,
+// with a wider margin); false for a point that does not exist.
 __device__ __forceinline__ bool point_regular(const Grid &g, const uint8_t *__restrict__ nv, int i, int j, int k) {
   if (i < 2 || i > g.mx - 3 || j < 2 || j > g.my - 3 || k < 2 || k > g.mz - 3) return false;
   return regular_faces(nv, lidx(g, i, j, k), g.mx, (long long)g.mx * g.my);
