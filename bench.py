@@ -577,7 +577,7 @@ STEP_BYTES = {
     "divergence": 8.0,                    # aj, in Projection's Contra2Cart
     "end_of_step_copies": 96.0,           # Ucont -> Ucont_o, Ucat -> Ucat_o
     # per FGMRES iteration: the FP64 apply 73, one FP32 V-cycle (3+3 zebra sweeps at 32 B,
-    # restriction and prolongation about 40, the zebra layout conversions 24, coarser
+    # restriction and prolongation about 40, the column layout conversions 24, coarser
     # levels x 8/7: about 293), the basis passes (three over j+1 vectors, 8 B each, about
     # 24 (j+1)) and the Z and V writes 16
     "per_iteration_fixed": 73.0 + 293.0 + 16.0,
