@@ -334,10 +334,11 @@ __device__ __forceinline__ void pdl_wait() {
 #define VFS_PDL_CAPTURE 1
 #endif
 // Every launch is counted in the context's launch counter and its status is checked: the
-// return value of cudaLaunchKernelEx, then the sticky launch error.
+// return value of cudaLaunchKernelEx, then the sticky launch error.  A failed launch's error is
+// cleared here, so no later check_launch sees it: the result must be passed on.
 template <typename... KArgs, typename... Args>
-int launch_chain(Ctx *c, const char *what, void (*kernel)(KArgs...), unsigned grid, unsigned block,
-                        size_t smem, Args... args) {
+[[nodiscard]] int launch_chain(Ctx *c, const char *what, void (*kernel)(KArgs...), unsigned grid, unsigned block,
+                               size_t smem, Args... args) {
   c->launches++;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);

@@ -1204,7 +1204,7 @@ static FluxIn flux_in(Ctx *c, int d) {
   return f;
 }
 
-void launch_fp(Ctx *c);
+int launch_fp(Ctx *c);
 
 // The 18 face-flux arrays of Formfunction_2 (one launch for the three directions of the interior
 // form; one launch per direction measured 30 % slower, a warp per direction 40 %).
@@ -1235,8 +1235,7 @@ int formfunction2_split(Ctx *c, double scale, bool rk_stage, double rk_coeff) {
   if (!rk_stage && (rc = periodic_copy3(c, uc))) return rc;
   Metrics m = metrics(c);
   if ((rc = face_fluxes(c))) return rc;
-  launch_fp(c);
-  if ((rc = check_launch(c, "k_fp"))) return rc;
+  if ((rc = launch_fp(c))) return rc;
   V3 pu{c->pucont[0], c->pucont[1], c->pucont[2]};
   return launch_chain(c, "k_rhs", k_rhs, nblocks(g.N, 256), 256, 0, g, m, c->nv, c->fp[0], c->fp[1], c->fp[2], scale,
                       field3(c, VFS_RHS), rk_stage ? 1 : 0, rk_coeff, cv(field3(c, VFS_DP)), cv(pu), uc);
@@ -1534,16 +1533,17 @@ int formfunction2(Ctx *c, double scale, bool rk_stage, double rk_coeff) {
 }
 
 // single-kernel launchers for the diagnostics entry point (vfs_run_kernel)
-void launch_face_flux(Ctx *c) { face_fluxes(c); }
-void launch_fp(Ctx *c) {
-  launch_chain(c, "k_fp", k_fp, nblocks(c->g.N, kFpThreads), kFpThreads, 0, c->g, flux_in(c, 0), flux_in(c, 1), flux_in(c, 2),
-               c->nv, c->fp[0], c->fp[1], c->fp[2]);
+int launch_face_flux(Ctx *c) { return face_fluxes(c); }
+int launch_fp(Ctx *c) {
+  return launch_chain(c, "k_fp", k_fp, nblocks(c->g.N, kFpThreads), kFpThreads, 0, c->g, flux_in(c, 0), flux_in(c, 1),
+                      flux_in(c, 2), c->nv, c->fp[0], c->fp[1], c->fp[2]);
 }
-void launch_rhs(Ctx *c) {
+int launch_rhs(Ctx *c) {
   V3 pu{c->pucont[0], c->pucont[1], c->pucont[2]};
   c->launches++, k_rhs<<<nblocks(c->g.N, 256), 256, 0, c->stream>>>(c->g, metrics(c), c->nv, c->fp[0], c->fp[1], c->fp[2], 1.0,
                                                     field3(c, VFS_RHS), 0, 0.0, cv(field3(c, VFS_DP)), cv(pu),
                                                     field3(c, VFS_UCONT));
+  return check_launch(c, "k_rhs");
 }
 
 // ------------------------------------------------------------------ face-metric products

@@ -1772,9 +1772,21 @@ int run_kernel(Ctx *c, int which, int reps) {
   Metrics m = metrics(c);
   for (int r = 0; r < reps; r++) {
     switch (which) {
-      case 0: extern void launch_face_flux(Ctx *); launch_face_flux(c); break;
-      case 1: extern void launch_fp(Ctx *); launch_fp(c); break;
-      case 2: extern void launch_rhs(Ctx *); launch_rhs(c); break;
+      case 0: {
+        extern int launch_face_flux(Ctx *);
+        if ((rc = launch_face_flux(c))) return rc;
+        break;
+      }
+      case 1: {
+        extern int launch_fp(Ctx *);
+        if ((rc = launch_fp(c))) return rc;
+        break;
+      }
+      case 2: {
+        extern int launch_rhs(Ctx *);
+        if ((rc = launch_rhs(c))) return rc;
+        break;
+      }
       case 3:
         rc = poisson_apply_dev(c, c->f[VFS_PHI][0], P.t);
         if (rc) return rc;
