@@ -325,7 +325,9 @@ void solve_graphs_free(Poisson &P);
 // operator), then waits for the predecessor grid to complete (and its writes to be visible)
 // before touching any vector; only then does it let its own successor start, so at most
 // two kernels of the chain are in flight and the results are those of plain stream order.
-// Outside such a launch both are no-ops.
+// Outside such a launch both are no-ops.  A kernel of the chain has no __restrict__ parameters
+// apart from what it may read before the wait: the qualifier says that nothing else writes the
+// memory while the kernel runs, so the compiler could move a load of it above the wait.
 __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

@@ -738,7 +738,7 @@ __global__ void __launch_bounds__(128) k_zprolong(ZL F, ZL C, const unsigned lon
 // V-cycle 35 us).
 template <typename T>
 __global__ void __launch_bounds__(128) k_zprolong_fine(ZL F, ZL C, const unsigned long long *__restrict__ mask, T *x,
-                                                       const T *__restrict__ xc) {
+                                                       const T *xc) {
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned col = t / (unsigned)F.S, pos = t - col * (unsigned)F.S;
   const unsigned k = col / (unsigned)F.hx, h = col - k * (unsigned)F.hx;
@@ -952,11 +952,11 @@ __host__ __device__ inline size_t tile_bytes(const ZL &L) { return sizeof(T) * k
 __host__ __device__ inline unsigned tiles_i(const ZL &L) { return (unsigned)(L.nx + kTileI - 1) / kTileI; }
 
 template <typename T, typename VT>
-__global__ void __launch_bounds__(256) k_to_columns(Grid g, ZL L, DynPtrT<const VT> vv, T *__restrict__ b) {
+__global__ void __launch_bounds__(256) k_to_columns(Grid g, ZL L, DynPtrT<const VT> vv, T *b) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
   T *sm = reinterpret_cast<T *>(tile_raw);
   pdl_wait();
-  const VT *__restrict__ v = vv.get();
+  const VT *v = vv.get();
   const unsigned ib = tiles_i(L);
   const int k = (int)(blockIdx.x / ib), i0 = (int)(blockIdx.x % ib) * kTileI, ld = L.S | 1;
   const int a = threadIdx.x % kTileI;
@@ -972,7 +972,7 @@ __global__ void __launch_bounds__(256) k_to_columns(Grid g, ZL L, DynPtrT<const 
   }
 }
 template <typename T, typename VT>
-__global__ void __launch_bounds__(256) k_to_columns_direct(Grid g, ZL L, DynPtrT<const VT> vv, T *__restrict__ b) {
+__global__ void __launch_bounds__(256) k_to_columns_direct(Grid g, ZL L, DynPtrT<const VT> vv, T *b) {
   pdl_wait();
   const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
   int i, j, k;
@@ -981,11 +981,11 @@ __global__ void __launch_bounds__(256) k_to_columns_direct(Grid g, ZL L, DynPtrT
 }
 // The interior points of the grid vector (the V-cycle's solution is zero off the unknowns).
 template <typename T>
-__global__ void __launch_bounds__(256) k_from_columns(Grid g, ZL L, const T *__restrict__ x, DynPtrT<T> zv) {
+__global__ void __launch_bounds__(256) k_from_columns(Grid g, ZL L, const T *x, DynPtrT<T> zv) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
   T *sm = reinterpret_cast<T *>(tile_raw);
   pdl_wait();
-  T *__restrict__ z = zv.get();
+  T *z = zv.get();
   const unsigned ib = tiles_i(L);
   const int k = (int)(blockIdx.x / ib), i0 = (int)(blockIdx.x % ib) * kTileI, ld = L.S | 1;
   for (int c = threadIdx.x >> 5; c < kTileI && i0 + c < L.nx; c += 8) {  // a warp a column
@@ -1000,7 +1000,7 @@ __global__ void __launch_bounds__(256) k_from_columns(Grid g, ZL L, const T *__r
     z[lidx(g, i0 + a + 1, j + 1, k + 1)] = sm[a * ld + (int)zrow(L, j)];
 }
 template <typename T>
-__global__ void __launch_bounds__(256) k_from_columns_direct(Grid g, ZL L, const T *__restrict__ x, DynPtrT<T> zv) {
+__global__ void __launch_bounds__(256) k_from_columns_direct(Grid g, ZL L, const T *x, DynPtrT<T> zv) {
   pdl_wait();
   const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
   int i, j, k;

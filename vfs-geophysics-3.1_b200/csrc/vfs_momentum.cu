@@ -67,7 +67,7 @@ int periodic_copy1(Ctx *c, double *s) {
 // Interior Cartesian velocity from averaged face fluxes by Cramer's rule on the centre
 // metrics (rhs.c:186-233).  Cells with nvert >= 0.1 keep their value.
 __global__ void k_contra2cart_interior(Grid g, CV3 uc, CV3 csi, CV3 eta, CV3 zet,
-                                       const uint8_t *__restrict__ nv, V3 ucat) {
+                                       const uint8_t *nv, V3 ucat) {
   pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
@@ -323,8 +323,8 @@ __device__ __forceinline__ long long edge_point(const Grid &g, long long t, int 
 
 // The boundary phase over its points: thread t < ne the edge points, then the ns listed solid
 // cells (nvert 3), which get zero (rhs.c:296-299).
-__global__ void k_contra2cart_bc_points(Grid g, Metrics m, const uint8_t *__restrict__ nv, CV3 lu, CV3 uo, V3 out,
-                                        uint8_t *flag, long long ne, long long ns, const long long *__restrict__ solid) {
+__global__ void k_contra2cart_bc_points(Grid g, Metrics m, const uint8_t *nv, CV3 lu, CV3 uo, V3 out,
+                                        uint8_t *flag, long long ne, long long ns, const long long *solid) {
   pdl_wait();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t < ne) {
@@ -341,7 +341,7 @@ __global__ void k_contra2cart_bc_points(Grid g, Metrics m, const uint8_t *__rest
 // Copies the marked values and clears the marks for the next call.  Of the two threads of a point
 // on two planes the second may find its mark cleared: the first has copied it.
 __global__ void k_bc_commit_points(Grid g, CV3 in, uint8_t *flag, V3 dst, long long ne, long long ns,
-                                   const long long *__restrict__ solid) {
+                                   const long long *solid) {
   pdl_wait();
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   long long p;
@@ -911,9 +911,8 @@ __device__ __forceinline__ void put_flux(const FluxOut &f, long long p, const do
 }
 // 128 registers (6 blocks per SM at 80: 196 us at 128 x 96 x 128 for both launches against 182).
 __global__ void __launch_bounds__(kFluxThreads, 4)
-    k_face_flux_listed(Grid g, Metrics m, CV3 uc, CV3 u, const uint8_t *__restrict__ nv,
-                       const double *__restrict__ nut, FluxOut f1, FluxOut f2, FluxOut f3, unsigned n,
-                       const long long *__restrict__ list) {
+    k_face_flux_listed(Grid g, Metrics m, CV3 uc, CV3 u, const uint8_t *nv, const double *nut, FluxOut f1, FluxOut f2,
+                       FluxOut f3, unsigned n, const long long *list) {
   pdl_wait();
   const unsigned t = blockIdx.x * blockDim.x + threadIdx.x;
   const unsigned dir = t / n;
@@ -937,10 +936,8 @@ __global__ void __launch_bounds__(kFluxThreads, 4)
   }
 }
 
-__global__ void __launch_bounds__(kFluxThreads, 6) k_face_flux(Grid g, Metrics m, CV3 uc, CV3 u,
-                                                               const uint8_t *__restrict__ nv,
-                                                               const double *__restrict__ nut, FluxOut f1,
-                                                               FluxOut f2, FluxOut f3) {
+__global__ void __launch_bounds__(kFluxThreads, 6) k_face_flux(Grid g, Metrics m, CV3 uc, CV3 u, const uint8_t *nv,
+                                                               const double *nut, FluxOut f1, FluxOut f2, FluxOut f3) {
   pdl_wait();
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
@@ -1085,7 +1082,7 @@ constexpr int kFpThreads = 64;
 #define VFS_FP_MINB 16
 #endif
 __global__ void __launch_bounds__(kFpThreads, VFS_FP_MINB) k_fp(Grid g, FluxIn f1, FluxIn f2, FluxIn f3,
-                                                         const uint8_t *__restrict__ nv, double *fpx, double *fpy,
+                                                         const uint8_t *nv, double *fpx, double *fpy,
                                                          double *fpz) {
   pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -1159,9 +1156,8 @@ struct GlobalFp {
 // of the right-hand side (momentum.c:1686-1900).  In RK mode the stage update
 // Ucont = pUcont + a*(RHS - dP) (rhs.c:1644-1650) is fused into the epilogue and the
 // accumulation starts from a zeroed RHS (VecSet(Rhs,0) at rhs.c:1643).
-__global__ void k_rhs(Grid g, Metrics m, const uint8_t *__restrict__ nv, const double *__restrict__ fpx,
-                      const double *__restrict__ fpy, const double *__restrict__ fpz, double scale,
-                      V3 rhs, int rk, double a, CV3 dP, CV3 pu, V3 ucont) {
+__global__ void k_rhs(Grid g, Metrics m, const uint8_t *nv, const double *fpx, const double *fpy, const double *fpz,
+                      double scale, V3 rhs, int rk, double a, CV3 dP, CV3 pu, V3 ucont) {
   pdl_wait();
   long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;

@@ -784,8 +784,7 @@ __device__ __forceinline__ void kry_givens(KryDev *kd, unsigned long long h_inne
 constexpr int kApplyThreads = 64;
 template <int NS, bool kT, typename B, typename ZT>
 __global__ void __launch_bounds__(kApplyThreads) k_apply_dyn(Grid g, long long ldv, const double *__restrict__ coef,
-                                                   const ZT *__restrict__ Z, const KryDev *__restrict__ kd,
-                                                   B *__restrict__ w) {
+                                                   const ZT *Z, const KryDev *kd, B *w) {
   pdl_wait();
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (p >= g.N) return;
@@ -824,8 +823,7 @@ __device__ __forceinline__ void multidot_body(long long N, long long ldv, const 
 }
 template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_multidot(long long N, long long ldv,
-                                                                         const B *__restrict__ V, KryDev *kd,
-                                                                         const B *__restrict__ w, double *parts) {
+                                                                         const B *V, KryDev *kd, const B *w, double *parts) {
   pdl_wait();
   const int nv = kd->j + 1;
   if (nv <= 4) multidot_body<4>(N, ldv, V, nv, w, parts);
@@ -888,8 +886,7 @@ __device__ __forceinline__ void update_dots(long long n, long long ldv, const B 
 // The second Gram-Schmidt pass where the first asked for it.
 template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_reorth(long long n, long long ldv,
-                                                                       const B *__restrict__ V, KryDev *kd,
-                                                                       B *__restrict__ w, double *parts) {
+                                                                       const B *V, KryDev *kd, B *w, double *parts) {
   pdl_wait();
   if (!kd->reorth) return;
   const int nv = kd->j + 1;
@@ -901,8 +898,7 @@ __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_reorth(long long 
 // The explicit w - V h2 of the degenerate case, and the Hessenberg column.
 template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_hessenberg(long long n, long long ldv,
-                                                                           const B *__restrict__ V, KryDev *kd,
-                                                                           B *__restrict__ w, double *parts,
+                                                                           const B *V, KryDev *kd, B *w, double *parts,
                                                                            unsigned long long h_inner, int use_graph) {
   pdl_wait();
   if (kd->reorth && kd->degen) {
@@ -952,8 +948,7 @@ __device__ __forceinline__ void update_scale_body(long long N, long long ldv, co
 }
 template <typename B>
 __global__ void __launch_bounds__(kKryThreads, VFS_KRY_MINB) k_next_vector(long long N, long long ldv, B *V,
-                                                                            const KryDev *__restrict__ kd,
-                                                                            const B *__restrict__ w) {
+                                                                            const KryDev *kd, const B *w) {
   pdl_wait();
   if (!kd->inner_go) return;
   const int jd = kd->jdone;
