@@ -1,0 +1,60 @@
+"""What the host code does when a CUDA call fails, on a CUDA runtime in host memory whose calls fail
+on request: the failure is reported, and a call after it neither uses what was not allocated nor
+forgets to allocate it."""
+import pytest
+
+import vfs_b200 as vfs
+from fake_cuda import context, fake, fake_library  # noqa: F401
+
+ERR_CUDA = 2
+
+
+@pytest.mark.parametrize("kernel", ["k_face_flux", "k_fp", "k_rhs", "k_periodic_copy"])
+def test_a_failed_launch_of_formfunction2_is_reported(fake, kernel):
+    ctx = context()
+    ctx.formfunction2(1.0)
+    fake.fake_fail_kernel(kernel.encode())
+    with pytest.raises(vfs.VfsError) as e:
+        ctx.formfunction2(1.0)
+    assert kernel in str(e.value)
+    fake.fake_fail_kernel(b"")
+    ctx.formfunction2(1.0)
+    ctx.close()
+
+
+@pytest.mark.parametrize("kernel,which", [("k_face_flux", 0), ("k_fp", 1), ("k_rhs", 2), ("k_zcol", 4)])
+def test_a_failed_launch_of_a_single_kernel_is_reported(fake, kernel, which):
+    ctx = context()
+    ctx.poisson_lhs()
+    ctx.run_kernel(which)
+    fake.fake_fail_kernel(kernel.encode())
+    with pytest.raises(vfs.VfsError):
+        ctx.run_kernel(which)
+    ctx.close()
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_a_solve_after_a_failed_allocation_allocates_what_is_missing(fake, precision):
+    """Each allocation of the first solve fails in turn; the same solve again allocates the rest."""
+    ctx = context()
+    ctx.poisson_rhs()
+    n0 = fake.fake_mallocs()
+    ctx.poisson_solve(precision=precision, allow_unconverged=True)
+    need = fake.fake_mallocs() - n0
+    assert need >= 2
+    ctx.close()
+    for nth in range(1, need + 1):
+        ctx = context()
+        ctx.poisson_rhs()
+        fake.fake_fail_malloc(nth)
+        with pytest.raises(vfs.VfsError) as e:
+            ctx.poisson_solve(precision=precision, allow_unconverged=True)
+        assert "allocation" in str(e.value)
+        with pytest.raises(vfs.VfsError) as e:  # still no memory: nothing may be launched without its buffers
+            ctx.poisson_solve(precision=precision, allow_unconverged=True)
+        assert "allocation" in str(e.value)
+        fake.fake_fail_malloc(0)
+        n0 = fake.fake_mallocs()
+        ctx.poisson_solve(precision=precision, allow_unconverged=True)
+        assert fake.fake_mallocs() - n0 == need - nth + 1
+        ctx.close()

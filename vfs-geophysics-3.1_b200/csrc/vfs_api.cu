@@ -13,7 +13,10 @@ static std::string g_last_err;
 
 namespace vfs {
 
+// A CUDA error that is reported here is not found again by the next launch's check (a failed
+// allocation leaves one behind).
 int set_err(Ctx *c, int code, const std::string &msg) {
+  if (code == VFS_ERR_CUDA) cudaGetLastError();
   if (c) c->err = msg;
   g_last_err = msg;
   return code;
