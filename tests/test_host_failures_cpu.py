@@ -33,7 +33,7 @@ def test_a_failed_launch_of_a_single_kernel_is_reported(fake, kernel, which):
     ctx.close()
 
 
-@pytest.mark.parametrize("precision", [0, 1])
+@pytest.mark.parametrize("precision", [0, 1, 2])
 def test_a_solve_after_a_failed_allocation_allocates_what_is_missing(fake, precision):
     """Each allocation of the first solve fails in turn; the same solve again allocates the rest."""
     ctx = context()

@@ -1307,7 +1307,7 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   const long long ldv = vec_ld(c->g.N);
   const int m = o.restart;
   const bool f64 = o.precision != 2, z64 = o.precision == 1;
-  if ((!f64 || P.restart >= m) && (f64 || P.restart32 >= m) && (!z64 || P.restart_z64 >= m) &&
+  if ((!f64 || P.restart >= m) && (f64 || (P.restart32 >= m && P.w32)) && (!z64 || P.restart_z64 >= m) &&
       (z64 || P.restart_z32 >= m))
     return VFS_OK;
   if (c->capturing) return set_err(c, VFS_ERR_STATE, "poisson_solve: Krylov basis not allocated before capture");
