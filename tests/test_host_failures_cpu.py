@@ -58,3 +58,55 @@ def test_a_solve_after_a_failed_allocation_allocates_what_is_missing(fake, preci
         ctx.poisson_solve(precision=precision, allow_unconverged=True)
         assert fake.fake_mallocs() - n0 == need - nth + 1
         ctx.close()
+
+
+def test_an_operator_after_a_failed_allocation_allocates_what_is_missing(fake):
+    """Each allocation of the operator and its multigrid levels fails in turn."""
+    ctx = context()
+    ctx.form_bcs()  # what is allocated on the way (reduction buffer, point lists) is there
+    ctx.poisson_lhs()
+    ctx.close()
+    ctx = context()
+    ctx.form_bcs()
+    n0 = fake.fake_mallocs()
+    ctx.poisson_lhs()
+    need = fake.fake_mallocs() - n0
+    assert need > 15  # the operator's five, six or seven a level
+    ctx.close()
+    for nth in range(1, need + 1):
+        ctx = context()
+        ctx.form_bcs()
+        fake.fake_fail_malloc(nth)
+        for _ in range(2):
+            with pytest.raises(vfs.VfsError) as e:
+                ctx.poisson_lhs()
+            assert "allocation" in str(e.value)
+        fake.fake_fail_malloc(0)
+        ctx.poisson_lhs()
+        ctx.poisson_rhs()
+        ctx.poisson_solve(allow_unconverged=True)
+        n0 = fake.fake_mallocs()
+        ctx.poisson_lhs()
+        assert fake.fake_mallocs() == n0
+        ctx.close()
+
+
+def test_no_reduction_without_its_buffer(fake):
+    """The solve asks for a larger reduction buffer; when that fails the old one is gone."""
+    ctx = context()
+    ctx.poisson_rhs()
+    ctx.poisson_solve(allow_unconverged=True, precision=0)
+    ctx.close()
+    ctx = context()
+    ctx.poisson_rhs()
+    fake.fake_fail_malloc(3)  # after the basis and the preconditioned vectors
+    with pytest.raises(vfs.VfsError) as e:
+        ctx.poisson_solve(allow_unconverged=True, precision=0)
+    assert "reduction buffer" in str(e.value)
+    with pytest.raises(vfs.VfsError) as e:
+        ctx.divergence()
+    assert "reduction buffer" in str(e.value)
+    assert fake.fake_launches(b"k_divergence") == 0
+    fake.fake_fail_malloc(0)
+    ctx.divergence()
+    ctx.close()

@@ -50,6 +50,7 @@ int ensure_red(Ctx *c, int n) {
   if (c->red) cudaFree(c->red);
   if (c->red_host) cudaFreeHost(c->red_host);
   c->red = nullptr; c->red_host = nullptr;
+  c->red_cap = 0;
   if (cudaMalloc(&c->red, sizeof(double) * n) != cudaSuccess ||
       cudaMallocHost(&c->red_host, sizeof(double) * n) != cudaSuccess)
     return set_err(c, VFS_ERR_CUDA, "reduction buffer allocation failed");

@@ -1032,7 +1032,7 @@ static ZL make_zl(int nx, int ny, int nz, const Grid &g, bool finest) {
 static void level_free(MGLevel &L) {
   cudaFree(L.op64); cudaFree(L.pk64); cudaFree(L.pk32); cudaFree(L.v64); cudaFree(L.v32); cudaFree(L.act);
   cudaFree(L.pmask);
-  L.op64 = nullptr;
+  L = MGLevel();
 }
 void mg_free(Poisson &P) {
   for (MGLevel &L : P.lv) level_free(L);
@@ -1066,7 +1066,7 @@ int mg_setup(Ctx *c) {
       L.v64 = old[l].v64; L.v32 = old[l].v32; L.act = old[l].act; L.pmask = old[l].pmask;
       old[l] = MGLevel();  // taken
     } else {
-      if (l < old.size()) { level_free(old[l]); old[l] = MGLevel(); }
+      if (l < old.size()) level_free(old[l]);
       P.alloc_epoch++;
       bool ok = cudaMalloc(&L.op64, sizeof(double) * NOP * n) == cudaSuccess;
       ok &= cudaMalloc(&L.pk64, sizeof(double) * 8 * n) == cudaSuccess;
@@ -1076,7 +1076,7 @@ int mg_setup(Ctx *c) {
       ok &= cudaMalloc(&L.act, n) == cudaSuccess;
       if (l > 0) ok &= cudaMalloc(&L.pmask, sizeof(unsigned long long) * n) == cudaSuccess;
       if (!ok) {
-        P.lv.push_back(L);
+        level_free(L);
         return fail(VFS_ERR_CUDA, "poisson_lhs: multigrid allocation failed");
       }
     }

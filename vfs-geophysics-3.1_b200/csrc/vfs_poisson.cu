@@ -462,13 +462,19 @@ int poisson_lhs(Ctx *c) {
   const Grid &g = c->g;
   const long long N = g.N;
   int rc;
+  P.built = false;
   if (!P.coef) {
     bool ok = cudaMalloc(&P.coef, sizeof(double) * NSLOT * vec_ld(N)) == cudaSuccess;
     ok &= cudaMalloc(&P.fluid, N) == cudaSuccess;
     ok &= cudaMalloc(&P.w, sizeof(double) * N) == cudaSuccess;
     ok &= cudaMalloc(&P.r, sizeof(double) * N) == cudaSuccess;
     ok &= cudaMalloc(&P.t, sizeof(double) * N) == cudaSuccess;
-    if (!ok) return set_err(c, VFS_ERR_CUDA, "poisson_lhs: allocation failed");
+    if (!ok) {
+      cudaFree(P.coef); cudaFree(P.fluid); cudaFree(P.w); cudaFree(P.r); cudaFree(P.t);
+      P.coef = P.w = P.r = P.t = nullptr;
+      P.fluid = nullptr;
+      return set_err(c, VFS_ERR_CUDA, "poisson_lhs: allocation failed");
+    }
     cudaMemsetAsync(P.w, 0, sizeof(double) * N, c->stream);
     cudaMemsetAsync(P.r, 0, sizeof(double) * N, c->stream);
     cudaMemsetAsync(P.t, 0, sizeof(double) * N, c->stream);
