@@ -332,9 +332,6 @@ __device__ __forceinline__ void pdl_wait() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
-#ifndef VFS_PDL_CAPTURE
-#define VFS_PDL_CAPTURE 1
-#endif
 // Every launch is counted in the context's launch counter and its status is checked: the
 // return value of cudaLaunchKernelEx, then the sticky launch error.  A failed launch's error is
 // cleared here, so no later check_launch sees it: the result must be passed on.
@@ -351,7 +348,7 @@ template <typename... KArgs, typename... Args>
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = !c->capturing || VFS_PDL_CAPTURE ? 1 : 0;
+  cfg.numAttrs = 1;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
   if (e != cudaSuccess) {
     cudaGetLastError();

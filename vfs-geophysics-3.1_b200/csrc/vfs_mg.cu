@@ -526,14 +526,15 @@ __global__ void __launch_bounds__(kColThreads, ZBounds<T>::v) k_zcol(ZL L, ZOp<T
   }
 }
 
-// A line Jacobi sweep or a small level's pass over columns too long for the kernel below, by lane
+// A line Jacobi sweep over columns too long for the kernel below (the finest level only), by lane
 // groups.
-template <typename T, bool kJac>
-__global__ void __launch_bounds__(kColThreads) k_zlong(ZL L, ZOp<T> op, const T *b, const T *xr, T *xw, int colour,
-                                                       int flags, T omega) {
+template <typename T>
+__global__ void __launch_bounds__(kColThreads) k_zlong(ZL L, ZOp<T> op, const T *b, const T *xr, T *xw, int flags,
+                                                       T omega) {
   const unsigned tid = blockIdx.x * blockDim.x + threadIdx.x;
   pdl_wait();
-  zsolve_long<T, kJac>(L, zcolumn(L, colour, tid >> L.lwl), (int)(tid & (unsigned)(L.lw - 1)), op.cpl, op.tri, op.cpr, b, xr, xw, flags, omega);
+  zsolve_long<T, true>(L, zcolumn(L, -1, tid >> L.lwl), (int)(tid & (unsigned)(L.lw - 1)), op.cpl, op.tri, op.cpr, b, xr,
+                       xw, flags, omega);
 }
 
 // One pass by Thomas' recurrence row by row (small levels, and every line Jacobi sweep: kJac,
@@ -542,7 +543,7 @@ __global__ void __launch_bounds__(kColThreads) k_zlong(ZL L, ZOp<T> op, const T 
 // (One thread a column straight from global memory took 22 us a pass on 45 x 37 x 53 cells.)
 constexpr int kSerialCols = 16, kSerialThreads = 32 * kSerialCols;
 template <typename T>
-static size_t serial_smem(const ZL &L) { return sizeof(T) * 4 * kSerialCols * ((size_t)L.ny | 1); }
+static size_t serial_smem(int ny) { return sizeof(T) * 4 * kSerialCols * ((size_t)ny | 1); }
 constexpr size_t kSerialSmem = 200 * 1024;
 template <typename T, bool kJac>
 __global__ void __launch_bounds__(kSerialThreads) k_zserial(ZL L, ZOp<T> op, const T *b, const T *xr, T *xw, int colour,
@@ -1018,7 +1019,8 @@ static ZL make_zl(int nx, int ny, int nz, const Grid &g, bool finest) {
   L.nx = nx; L.ny = ny; L.nz = nz;
   L.hx = (nx + 1) / 2;
   L.ip = g.iper; L.jp = g.jper; L.kp = g.kper;
-  L.serial = (long long)nx * ny * nz <= kSerialCells || (!finest && !two_colours(L) && ny <= 256);
+  L.serial = ((long long)nx * ny * nz <= kSerialCells || (!finest && !two_colours(L) && ny <= 256)) &&
+             serial_smem<double>(ny) <= kSerialSmem;  // k_zserial is the only kernel for its layout
   L.seg = L.serial ? 1 : (ny + 31) / 32;
   L.ls = L.serial ? ny | 1 : (ny + L.seg - 1) / L.seg;
   L.S = L.seg * L.ls;
@@ -1145,7 +1147,7 @@ static const double kJacobiOmega = 0.8;
 template <typename T>
 static int launch_serial(Ctx *c, const MGLevel &L, const LvT<T> &v, const T *xr, T *xw, int colour, int flags) {
   const unsigned ncol = (unsigned)L.z.nz * L.z.hx * (colour >= 0 ? 1 : 2), nb = nblocks(ncol, kSerialCols);
-  const size_t smem = serial_smem<T>(L.z);
+  const size_t smem = serial_smem<T>(L.z.ny);
   const T om = T(kJacobiOmega);
   const ZOp<T> op{v.cpl, v.tri, v.cpr};
   // the shared-memory limit is an attribute of the kernel on a device
@@ -1161,11 +1163,11 @@ template <typename T>
 static int launch_pass(Ctx *c, const MGLevel &L, const LvT<T> &v, const T *xr, T *xw, int colour, int flags) {
   const unsigned ncol = (unsigned)L.z.nz * L.z.hx * (colour >= 0 ? 1 : 2);
   const ZOp<T> op{v.cpl, v.tri, v.cpr};
-  if ((L.z.serial || colour < 0) && serial_smem<T>(L.z) <= kSerialSmem) return launch_serial<T>(c, L, v, xr, xw, colour, flags);
+  if (L.z.serial || (colour < 0 && serial_smem<T>(L.z.ny) <= kSerialSmem))
+    return launch_serial<T>(c, L, v, xr, xw, colour, flags);
   const unsigned nb = nblocks((long long)ncol << L.z.lwl, kColThreads);
-  if (colour < 0 || L.z.serial)  // columns too long for shared memory
-    return launch_chain(c, "k_zlong", colour < 0 ? k_zlong<T, true> : k_zlong<T, false>, nb, kColThreads, 0, L.z, op, v.b,
-                        xr, xw, colour, flags, T(kJacobiOmega));
+  if (colour < 0)  // columns too long for shared memory
+    return launch_chain(c, "k_zlong", k_zlong<T>, nb, kColThreads, 0, L.z, op, v.b, xr, xw, flags, T(kJacobiOmega));
 #define VFS_PASS(S)                                                                                                \
   case S:                                                                                                          \
     return L.z.ls == 32 ? launch_chain(c, "k_zcol", k_zcol<T, S, true>, nb, kColThreads, 0, L.z, op, v.b, xw, colour, flags) \

@@ -1137,15 +1137,6 @@ __device__ __forceinline__ void rhs_point(const Grid &g, const Metrics &m, const
   }
 }
 
-// The stage update Ucont = pUcont + a * RHS (RHS already holding -dP) over every point.
-__global__ void k_rk_update(long long n, double a, CV3 rhs, CV3 pu, V3 ucont) {
-  const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= n) return;
-  ucont.x[p] = a * rhs.x[p] + pu.x[p];
-  ucont.y[p] = a * rhs.y[p] + pu.y[p];
-  ucont.z[p] = a * rhs.z[p] + pu.z[p];
-}
-
 struct GlobalFp {
   const double *f[3];
   long long q[4];

@@ -20,8 +20,7 @@
 // Kernels of the Contra2Cart path, defined in vfs_momentum.cu / vfs_api.cu.
 namespace vfs {
 __global__ void k_periodic_copy(Grid g, double *a, double *b, double *c);
-__global__ void k_contra2cart_interior(Grid g, CV3 uc, CV3 csi, CV3 eta, CV3 zet, const uint8_t *__restrict__ nv,
-                                       V3 ucat);
+__global__ void k_contra2cart_interior(Grid g, CV3 uc, CV3 csi, CV3 eta, CV3 zet, const uint8_t *nv, V3 ucat);
 __global__ void k_contra2cart_bc(Grid g, Metrics m, const uint8_t *__restrict__ nv, CV3 lu, CV3 uo, V3 out,
                                  uint8_t *flag);
 __global__ void k_bc_commit(long long n, CV3 in, uint8_t *flag, V3 dst);

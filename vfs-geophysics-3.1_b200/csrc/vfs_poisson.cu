@@ -542,13 +542,6 @@ __global__ void k_shift_scaled(long long n, const uint8_t *fluid, const double *
   double val = -sum * aj[p] / sum_aj;
   b[p] += val;
 }
-// x += val on fluid cells (Remove_Nullspace, poisson_hypre.c:194).
-__global__ void k_shift(long long n, const uint8_t *fluid, double val, double *x) {
-  long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (p >= n || !fluid[p]) return;
-  x[p] += val;
-}
-
 __global__ void k_sum_fluid(long long n, const uint8_t *fluid, const double *a, double *parts) {
   __shared__ double sh[8];
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
