@@ -110,3 +110,16 @@ def test_no_reduction_without_its_buffer(fake):
     fake.fake_fail_malloc(0)
     ctx.divergence()
     ctx.close()
+
+
+@pytest.mark.parametrize("precision,size", [(0, 4), (1, 8), (2, 4)])
+def test_the_first_solve_clears_no_more_than_the_preconditioned_vectors(fake, precision, size):
+    """Their ghost points are never written; the basis is written whole before it is read."""
+    ctx = context()
+    ctx.poisson_rhs()
+    n0 = fake.fake_cleared_bytes()
+    ctx.poisson_solve(precision=precision, restart=20, allow_unconverged=True)
+    n = ctx.shape[0] * ctx.shape[1] * ctx.shape[2]
+    ld = (n + 31) // 32 * 32
+    assert fake.fake_cleared_bytes() - n0 == 20 * ld * size + 8 * n  # and Phi, the zero guess
+    ctx.close()

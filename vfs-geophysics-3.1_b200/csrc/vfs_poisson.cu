@@ -1312,25 +1312,25 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   if (c->capturing) return set_err(c, VFS_ERR_STATE, "poisson_solve: Krylov basis not allocated before capture");
   c->setup_epoch++;  // captured graphs hold the old buffers
   P.alloc_epoch++;
-  if (cudaStreamSynchronize(c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "poisson_solve: failed");
   P.ldv = ldv;
   bool ok = true;
-  // the ghost points of the preconditioned vectors are never written: zero from the start
-  auto grow = [&](auto **v, int &have, int extra) {
+  // the ghost points of the preconditioned vectors are never written: zero from the start (the
+  // basis vectors are written whole before they are read)
+  auto grow = [&](auto **v, int &have, bool basis) {
     if (!ok || have >= m) return;
-    const size_t bytes = sizeof(**v) * (size_t)ldv * (m + extra);
+    const size_t bytes = sizeof(**v) * (size_t)ldv * (basis ? m + 1 : m);
     cudaFree(*v);
     *v = nullptr;
     have = 0;
     ok = cudaMalloc(v, bytes) == cudaSuccess;
     if (!ok) return;
-    cudaMemsetAsync(*v, 0, bytes, c->stream);
+    if (!basis) cudaMemsetAsync(*v, 0, bytes, c->stream);
     have = m;
   };
-  if (f64) grow(&P.V, P.restart, 1);
-  else grow(&P.V32, P.restart32, 1);
-  if (z64) grow(&P.Z64, P.restart_z64, 0);
-  else grow(&P.Z32, P.restart_z32, 0);
+  if (f64) grow(&P.V, P.restart, true);
+  else grow(&P.V32, P.restart32, true);
+  if (z64) grow(&P.Z64, P.restart_z64, false);
+  else grow(&P.Z32, P.restart_z32, false);
   if (!f64 && ok && !P.w32) ok = cudaMalloc(&P.w32, sizeof(float) * (size_t)ldv) == cudaSuccess;
   if (!ok) return set_err(c, VFS_ERR_CUDA, "poisson_solve: Krylov basis allocation failed");
   return VFS_OK;
