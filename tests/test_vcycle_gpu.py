@@ -73,6 +73,11 @@ def test_vcycle(dims, precision):
 
 
 @pytest.mark.gpu
+def test_vcycle_of_columns_too_long_for_the_set_up_in_shared_memory():
+    _check(_case((4, 12900, 4)), 1)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("precision", [0, 1])
 @pytest.mark.parametrize("dims,periodic", [((16, 24, 20), (1, 1, 1)), ((32, 264, 32), (1, 1, 1)), ((6, 300, 8), (0, 1, 0)),
                                            ((9, 13, 11), (0, 0, 0)), ((24, 40, 33), (1, 0, 0))])

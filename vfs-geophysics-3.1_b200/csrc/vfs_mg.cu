@@ -63,33 +63,58 @@ __device__ __forceinline__ bool zcell(const ZL &L, unsigned q, int &i, int &j, i
 }
 
 // ------------------------------------------------------------------ set-up (FP64)
-// Fine-level couplings from the reference operator (19 slots on the DA layout).
-__global__ void k_mg_fine_couplings(Grid g, ZL L, const double *__restrict__ coef, const uint8_t *__restrict__ fluid,
-                                    double *__restrict__ op) {
+// Fine-level couplings from the reference operator (19 slots on the DA layout): the coupling of
+// cell (i, j, k) to its +i (q = 0), +j (1) or +k (2) neighbour.
+__device__ __forceinline__ double fine_coupling(const Grid &g, const ZL &L, const double *__restrict__ coef,
+                                                const uint8_t *__restrict__ fluid, int q, int i, int j, int k) {
+  const long long N = vec_ld(g.N), p = lidx(g, i + 1, j + 1, k + 1);
+  // every load is issued before the first is tested
+  const long long e = q == 0 ? lidx(g, wrapi(g, i + 2), j + 1, k + 1)
+                             : (q == 1 ? lidx(g, i + 1, wrapj(g, j + 2), k + 1) : lidx(g, i + 1, j + 1, wrapk(g, k + 2)));
+  const double c = coef[(q == 0 ? EP : (q == 1 ? NP : TP)) * N + p], d = coef[(q == 0 ? WP : (q == 1 ? SP : BP)) * N + e];
+  const bool f = fluid[p] && fluid[e];
+  const bool has = q == 0 ? i + 1 < L.nx || L.ip : (q == 1 ? j + 1 < L.ny || L.jp : k + 1 < L.nz || L.kp);
+  return f && has ? fmax(0.0, 0.5 * (c + d)) : 0.0;
+}
+
+// A block moves kTileI consecutive i of one k plane and all rows through shared memory, so that
+// both the grid arrays and the columns are accessed in runs.  Columns too long for that go directly.
+constexpr int kTileI = 16;
+constexpr size_t kTileSmem = 200 * 1024;
+template <typename T>
+__host__ __device__ inline size_t tile_bytes(const ZL &L) { return sizeof(T) * kTileI * ((size_t)L.S | 1); }
+__host__ __device__ inline unsigned tiles_i(const ZL &L) { return (unsigned)(L.nx + kTileI - 1) / kTileI; }
+
+// One direction after the other through the same tile.  Bound by the latency of the loads between the
+// barriers.  (A thread per slot, in column order, read the coefficients a grid row apart: 444 us at
+// 256 x 192 x 256 cells against 286, 55 at 128 x 96 x 128 against 34; tiles of 32 i 361 and 50.)
+__global__ void __launch_bounds__(256) k_mg_fine_couplings(Grid g, ZL L, const double *__restrict__ coef,
+                                                           const uint8_t *__restrict__ fluid, double *__restrict__ op) {
+  extern __shared__ __align__(16) unsigned char fine_raw[];
+  double *sm = reinterpret_cast<double *>(fine_raw);
+  const unsigned ib = tiles_i(L);
+  const int k = (int)(blockIdx.x / ib), i0 = (int)(blockIdx.x % ib) * kTileI, ld = L.S | 1;
+  const int a = threadIdx.x % kTileI;
+#pragma unroll
+  for (int q = 0; q < 3; q++) {
+#pragma unroll 2
+    for (int j = threadIdx.x / kTileI; j < L.S; j += 256 / kTileI)  // rows past ny: the empty slots
+      sm[a * ld + (int)zrow(L, j)] =
+          j < L.ny && i0 + a < L.nx ? fine_coupling(g, L, coef, fluid, q, i0 + a, j, k) : 0.0;
+    __syncthreads();
+    for (int c = threadIdx.x >> 5; c < kTileI && i0 + c < L.nx; c += 8) {  // a warp a column
+      const unsigned p0 = zcol(L, i0 + c, k);
+      for (int s = threadIdx.x & 31; s < L.S; s += 32) op[(OP_CE + q) * L.n + p0 + s] = sm[c * ld + s];
+    }
+    __syncthreads();
+  }
+}
+__global__ void k_mg_fine_couplings_direct(Grid g, ZL L, const double *__restrict__ coef,
+                                           const uint8_t *__restrict__ fluid, double *__restrict__ op) {
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int i, j, k;
   if (t >= L.n || !zcell(L, (unsigned)t, i, j, k)) return;
-  const long long N = vec_ld(g.N);
-  const long long p = lidx(g, i + 1, j + 1, k + 1);
-  const long long q = t;
-  double ce = 0, cn = 0, ct = 0;
-  if (fluid[p]) {
-    if (i + 1 < L.nx || L.ip) {
-      const long long e = lidx(g, wrapi(g, i + 2), j + 1, k + 1);
-      if (fluid[e]) ce = fmax(0.0, 0.5 * (coef[EP * N + p] + coef[WP * N + e]));
-    }
-    if (j + 1 < L.ny || L.jp) {
-      const long long e = lidx(g, i + 1, wrapj(g, j + 2), k + 1);
-      if (fluid[e]) cn = fmax(0.0, 0.5 * (coef[NP * N + p] + coef[SP * N + e]));
-    }
-    if (k + 1 < L.nz || L.kp) {
-      const long long e = lidx(g, i + 1, j + 1, wrapk(g, k + 2));
-      if (fluid[e]) ct = fmax(0.0, 0.5 * (coef[TP * N + p] + coef[BP * N + e]));
-    }
-  }
-  op[OP_CE * L.n + q] = ce;
-  op[OP_CN * L.n + q] = cn;
-  op[OP_CT * L.n + q] = ct;
+  for (int q = 0; q < 3; q++) op[(OP_CE + q) * L.n + t] = fine_coupling(g, L, coef, fluid, q, i, j, k);
 }
 
 // Coarse couplings: 0.5 x the sum of the four fine couplings across each coarse face.
@@ -124,44 +149,98 @@ __device__ __forceinline__ ZNb znb(const ZL &L, int i, int j, int k) {
   return r;
 }
 
-__global__ void k_mg_diag(ZL L, double *__restrict__ op) {
+// The diagonal, and act[q] = 1 where it is non-zero (an active unknown).
+__global__ void k_mg_diag(ZL L, double *__restrict__ op, uint8_t *__restrict__ act) {
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x, n = L.n;
   int i, j, k;
-  if (q >= n || !zcell(L, (unsigned)q, i, j, k)) return;
+  if (q >= n) return;
+  if (!zcell(L, (unsigned)q, i, j, k)) { act[q] = 0; return; }
   const ZNb b = znb(L, i, j, k);
+  const unsigned p0 = zcol(L, i, k), pos = (unsigned)q - p0;  // a column neighbour's cell has the same slot
   double s = op[OP_CE * n + q] + op[OP_CN * n + q] + op[OP_CT * n + q];
-  if (b.iw >= 0) s += op[OP_CE * n + zidx(L, b.iw, j, k)];
-  if (b.js >= 0) s += op[OP_CN * n + zidx(L, i, b.js, k)];
-  if (b.kb >= 0) s += op[OP_CT * n + zidx(L, i, j, b.kb)];
+  if (b.iw >= 0) s += op[OP_CE * n + zcol(L, b.iw, k) + pos];
+  if (b.js >= 0) s += op[OP_CN * n + p0 + zrow(L, b.js)];
+  if (b.kb >= 0) s += op[OP_CT * n + zcol(L, i, b.kb) + pos];
   op[OP_DG * n + q] = -s;
+  act[q] = s != 0.0 ? 1 : 0;
 }
 
 // Thomas factors of every j-line (the in-line couplings only; a periodic j wrap is left
 // to the right-hand side): cpr_j = upper_j / den_j, iden_j = 1 / den_j,
 // den_j = dg_j - lower_j * cpr_{j-1}.  Inactive or degenerate rows get zero factors, so
 // the smoother leaves their unknown at zero.
-__global__ void k_mg_thomas(ZL L, double *__restrict__ op) {
-  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (t >= (long long)L.nx * L.nz) return;
-  const int i = (int)(t % L.nx), k = (int)(t / L.nx);
-  const long long n = L.n;
+struct Thomas {
   double cprev = 0, lower = 0;
-  for (int j = 0; j < L.ny; j++) {
-    const long long q = zidx(L, i, j, k);
-    const double dg = op[OP_DG * n + q];
-    const double upper = j + 1 < L.ny ? op[OP_CN * n + q] : 0.0;
+  // dg and upper of the row in, iden and cpr out
+  __device__ __forceinline__ void row(double &dg, double &upper) {
+    const double up = upper;
     double cpr = 0, iden = 0;
     if (dg != 0) {
       const double den = dg - lower * cprev;
       if (fabs(den) > 1e-12 * fabs(dg)) {
         iden = 1.0 / den;
-        cpr = upper * iden;
+        cpr = up * iden;
       }
     }
-    op[OP_CPR * n + q] = cpr;
-    op[OP_IDEN * n + q] = iden;
+    dg = iden;
+    upper = cpr;
     cprev = cpr;
-    lower = upper;
+    lower = up;
+  }
+};
+// A block stages `cols` columns in shared memory (dg and upper, replaced by iden and cpr), one
+// thread a column runs the recurrence there: its rows are not neighbours in the column's slots, and
+// straight from global memory every load was a sector of its own.  Bound by the chain of divisions of a
+// row.  All levels of 256 x 192 x 256 cells 1410 -> 271 us (32 columns a block 329), 64 x 48 x 64 37 -> 22.
+constexpr int kThomasThreads = 256;
+constexpr size_t kThomasSmem = 200 * 1024;
+static size_t thomas_smem(const ZL &L, int cols) { return sizeof(double) * 2 * cols * ((size_t)L.ny | 1); }
+// Columns a block: 16, fewer where they are long (0: one does not fit).
+static int thomas_cols(const ZL &L) {
+  int cols = 16;
+  while (cols > 0 && thomas_smem(L, cols) > kThomasSmem) cols /= 2;
+  return cols;
+}
+__global__ void __launch_bounds__(kThomasThreads) k_mg_thomas(ZL L, int cols, double *__restrict__ op) {
+  extern __shared__ __align__(16) unsigned char tho_raw[];
+  const int ld = L.ny | 1, ny = L.ny;
+  double *sd = reinterpret_cast<double *>(tho_raw), *su = sd + cols * ld;
+  const unsigned c0 = blockIdx.x * (unsigned)cols, ncol = (unsigned)L.nz * 2u * (unsigned)L.hx, S = (unsigned)L.S;
+  const int nc = (int)min((unsigned)cols, ncol - c0);
+  const long long n = L.n;
+  const unsigned p0 = c0 * S;
+  for (unsigned t = threadIdx.x; t < (unsigned)nc * S; t += kThomasThreads) {
+    const unsigned c = t / S;
+    const int j = zrow_of(L, t - c * S);
+    if (j >= ny) continue;
+    sd[c * ld + j] = op[OP_DG * n + p0 + t];
+    su[c * ld + j] = j + 1 < ny ? op[OP_CN * n + p0 + t] : 0.0;
+  }
+  __syncthreads();
+  if ((int)threadIdx.x < nc) {
+    Thomas T;
+    for (int j = 0; j < ny; j++) T.row(sd[threadIdx.x * ld + j], su[threadIdx.x * ld + j]);
+  }
+  __syncthreads();
+  for (unsigned t = threadIdx.x; t < (unsigned)nc * S; t += kThomasThreads) {
+    const unsigned c = t / S;
+    const int j = zrow_of(L, t - c * S);
+    if (j >= ny) continue;
+    op[OP_IDEN * n + p0 + t] = sd[c * ld + j];
+    op[OP_CPR * n + p0 + t] = su[c * ld + j];
+  }
+}
+__global__ void k_mg_thomas_direct(ZL L, double *__restrict__ op) {
+  const unsigned col = blockIdx.x * blockDim.x + threadIdx.x;
+  if (col >= (unsigned)L.nz * 2u * (unsigned)L.hx) return;
+  const long long n = L.n;
+  Thomas T;
+  for (int j = 0; j < L.ny; j++) {
+    const long long q = (long long)col * L.S + zrow(L, j);
+    double a = op[OP_DG * n + q], b = j + 1 < L.ny ? op[OP_CN * n + q] : 0.0;
+    T.row(a, b);
+    op[OP_IDEN * n + q] = a;
+    op[OP_CPR * n + q] = b;
   }
 }
 
@@ -190,21 +269,16 @@ __global__ void k_mg_pack(ZL L, const double *__restrict__ op, Q4<T> *__restrict
   Q4<T> a;
   Q2<T> b;
   a.a = (T)op[OP_CE * n + q];
-  a.b = nb.iw >= 0 ? (T)op[OP_CE * n + zidx(L, nb.iw, j, k)] : T(0);
+  const unsigned p0 = zcol(L, i, k), pos = (unsigned)q - p0;
+  a.b = nb.iw >= 0 ? (T)op[OP_CE * n + zcol(L, nb.iw, k) + pos] : T(0);
   a.c = (T)op[OP_CT * n + q];
-  a.d = nb.kb >= 0 ? (T)op[OP_CT * n + zidx(L, i, j, nb.kb)] : T(0);
-  b.a = nb.js >= 0 ? (T)op[OP_CN * n + zidx(L, i, nb.js, k)] : T(0);
+  a.d = nb.kb >= 0 ? (T)op[OP_CT * n + zcol(L, i, nb.kb) + pos] : T(0);
+  b.a = nb.js >= 0 ? (T)op[OP_CN * n + p0 + zrow(L, nb.js)] : T(0);
   b.b = (T)op[OP_IDEN * n + q];
   cpl[q] = a;
   tri[q] = b;
   cpr[q] = (T)op[OP_CPR * n + q];
   dg[q] = (T)op[OP_DG * n + q];
-}
-
-// act[q] = 1 where the level's diagonal is non-zero (an active unknown).
-__global__ void k_mg_active(long long n, const double *__restrict__ op, uint8_t *__restrict__ act) {
-  const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-  if (q < n) act[q] = op[OP_DG * n + q] != 0.0 ? 1 : 0;
 }
 
 // Coarse cell q: bit e (0..26) set where the cell of its 3 x 3 x 3 neighbourhood at
@@ -215,14 +289,29 @@ __global__ void k_mg_pmask(ZL F, ZL C, const uint8_t *__restrict__ actF, const u
   const long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   int I, J, K;
   if (q >= C.n || !zcell(C, (unsigned)q, I, J, K)) return;
-  unsigned long long m = 0;
-  for (int e = 0; e < 27; e++) {
-    const int i = wrap_or_none(I + e % 3 - 1, C.nx, C.ip), j = wrap_or_none(J + e / 3 % 3 - 1, C.ny, C.jp);
-    const int k = wrap_or_none(K + e / 9 - 1, C.nz, C.kp);
-    if (i >= 0 && j >= 0 && k >= 0 && actC[zidx(C, i, j, k)]) m |= 1ull << e;
+  // every byte is loaded (the cell's own where there is no neighbour) before the first is used
+  int Iv[3], Jv[3], Kv[3];
+  bool Io[3], Jo[3], Ko[3];
+#pragma unroll
+  for (int d = 0; d < 3; d++) {
+    const int i = wrap_or_none(I + d - 1, C.nx, C.ip), j = wrap_or_none(J + d - 1, C.ny, C.jp);
+    const int k = wrap_or_none(K + d - 1, C.nz, C.kp);
+    Io[d] = i >= 0; Jo[d] = j >= 0; Ko[d] = k >= 0;
+    Iv[d] = Io[d] ? i : I; Jv[d] = (int)zrow(C, Jo[d] ? j : J); Kv[d] = Ko[d] ? k : K;
   }
+  uint8_t a[27], b[8];
+#pragma unroll
+  for (int e = 0; e < 27; e++) a[e] = actC[zcol(C, Iv[e % 3], Kv[e / 9]) + (unsigned)Jv[e / 3 % 3]];
+  const unsigned r[2] = {zrow(F, 2 * J), zrow(F, 2 * J + 1)};
+#pragma unroll
+  for (int ch = 0; ch < 8; ch++) b[ch] = actF[zcol(F, 2 * I + (ch & 1), 2 * K + (ch >> 2)) + r[(ch >> 1) & 1]];
+  unsigned long long m = 0;
+#pragma unroll
+  for (int e = 0; e < 27; e++)
+    if (Io[e % 3] && Jo[e / 3 % 3] && Ko[e / 9] && a[e]) m |= 1ull << e;
+#pragma unroll
   for (int ch = 0; ch < 8; ch++)
-    if (actF[zidx(F, 2 * I + (ch & 1), 2 * J + ((ch >> 1) & 1), 2 * K + (ch >> 2))]) m |= 1ull << (27 + ch);
+    if (b[ch]) m |= 1ull << (27 + ch);
   mask[q] = m;
 }
 
@@ -944,14 +1033,6 @@ __global__ void __launch_bounds__(kBottomThreads) k_mg_bottom(const __grid_const
 }
 
 // ------------------------------------------------------------------ grid layout <-> columns
-// A block moves kTileI consecutive i of one k plane and all rows through shared memory, so that
-// both sides are accessed in runs.  Columns too long for that go directly.
-constexpr int kTileI = 16;
-constexpr size_t kTileSmem = 200 * 1024;
-template <typename T>
-__host__ __device__ inline size_t tile_bytes(const ZL &L) { return sizeof(T) * kTileI * ((size_t)L.S | 1); }
-__host__ __device__ inline unsigned tiles_i(const ZL &L) { return (unsigned)(L.nx + kTileI - 1) / kTileI; }
-
 template <typename T, typename VT>
 __global__ void __launch_bounds__(256) k_to_columns(Grid g, ZL L, DynPtrT<const VT> vv, T *b) {
   extern __shared__ __align__(16) unsigned char tile_raw[];
@@ -1089,15 +1170,29 @@ int mg_setup(Ctx *c) {
     cudaMemsetAsync(L.v32, 0, sizeof(float) * 3 * n, c->stream);
     const unsigned nb = nblocks(n, 128);
     if (P.lv.empty()) {
-      c->launches++, k_mg_fine_couplings<<<nb, 128, 0, c->stream>>>(g, L.z, P.coef, P.fluid, L.op64);
+      const size_t smem = tile_bytes<double>(L.z);
+      // the shared-memory limits are attributes of the kernels on a device
+      if (cudaFuncSetAttribute(k_mg_fine_couplings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem) != cudaSuccess ||
+          cudaFuncSetAttribute(k_mg_thomas, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kThomasSmem) != cudaSuccess) {
+        P.lv.push_back(L);
+        return fail(VFS_ERR_CUDA, "poisson_lhs: shared-memory limit");
+      }
+      if (smem <= kTileSmem)
+        c->launches++, k_mg_fine_couplings<<<tiles_i(L.z) * (unsigned)nz, 256, smem, c->stream>>>(g, L.z, P.coef, P.fluid, L.op64);
+      else
+        c->launches++, k_mg_fine_couplings_direct<<<nb, 128, 0, c->stream>>>(g, L.z, P.coef, P.fluid, L.op64);
     } else {
       const MGLevel &F = P.lv.back();
       c->launches++, k_mg_coarse_couplings<<<nb, 128, 0, c->stream>>>(F.z, L.z, F.op64, L.op64);
     }
     if ((rc = check_launch(c, "k_mg_couplings"))) { P.lv.push_back(L); return fail(rc, "poisson_lhs: multigrid set-up failed"); }
-    c->launches++, k_mg_diag<<<nb, 128, 0, c->stream>>>(L.z, L.op64);
-    c->launches++, k_mg_thomas<<<nblocks((long long)nx * nz, 64), 64, 0, c->stream>>>(L.z, L.op64);
-    c->launches++, k_mg_active<<<nblocks(n, 256), 256, 0, c->stream>>>(n, L.op64, L.act);
+    c->launches++, k_mg_diag<<<nb, 128, 0, c->stream>>>(L.z, L.op64, L.act);
+    const unsigned ncol = (unsigned)nz * 2u * (unsigned)L.z.hx;
+    const int cols = thomas_cols(L.z);
+    if (cols > 0)
+      c->launches++, k_mg_thomas<<<nblocks(ncol, cols), kThomasThreads, thomas_smem(L.z, cols), c->stream>>>(L.z, cols, L.op64);
+    else
+      c->launches++, k_mg_thomas_direct<<<nblocks(ncol, 64), 64, 0, c->stream>>>(L.z, L.op64);
     c->launches++, k_mg_pack<double><<<nb, 128, 0, c->stream>>>(L.z, L.op64, (Q4<double> *)L.pk64, (Q2<double> *)(L.pk64 + 4 * n), L.pk64 + 6 * n,
                                                                 L.pk64 + 7 * n);
     c->launches++, k_mg_pack<float><<<nb, 128, 0, c->stream>>>(L.z, L.op64, (Q4<float> *)L.pk32, (Q2<float> *)(L.pk32 + 4 * n), L.pk32 + 6 * n,
