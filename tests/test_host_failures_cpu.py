@@ -123,3 +123,19 @@ def test_the_first_solve_clears_no_more_than_the_preconditioned_vectors(fake, pr
     ld = (n + 31) // 32 * 32
     assert fake.fake_cleared_bytes() - n0 == 20 * ld * size + 8 * n  # and Phi, the zero guess
     ctx.close()
+
+
+def test_solves_that_differ_in_their_targets_share_a_graph(fake):
+    """A caller who changes the tolerance every two solves does not pay a capture for each replay."""
+    ctx = context()
+    ctx.poisson_rhs()
+    kw = dict(zero_guess=1, allow_unconverged=True)
+    for rtol in (1e-4, 1e-6, 1e-8):
+        for max_iter in (50, 100):
+            for _ in range(2):
+                ctx.poisson_solve(rtol=rtol, max_iter=max_iter, **kw)
+    assert (fake.fake_captures(), fake.fake_graph_launches()) == (1, 11)
+    ctx.poisson_solve(rtol=1e-8, max_iter=100, pre_smooth=2, **kw)
+    ctx.poisson_solve(rtol=1e-8, max_iter=100, pre_smooth=2, **kw)
+    assert (fake.fake_captures(), fake.fake_graph_launches()) == (2, 12)
+    ctx.close()

@@ -65,3 +65,22 @@ def test_more_kinds_of_solves_than_graphs():
             for _ in range(2):
                 np.testing.assert_array_equal(_solve(ctx, **k)[0], w)
     ctx.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("precision", [0, 2])
+def test_replays_with_other_targets(precision):
+    """The targets are not part of a graph: each solve stops where a fresh context's does."""
+    case = cases.channel(20, 18, 24, wavy=0.1)
+    ctx = _context(case, 4)
+    targets = [(1e-9, 500), (1e-9, 500), (1e-4, 500), (1e-9, 3), (1e-11, 500), (1e-4, 500), (1e-9, 500)]
+    for rtol, max_iter in targets:
+        kw = dict(precision=precision, rtol=rtol, max_iter=max_iter, zero_guess=1, allow_unconverged=True)
+        st = ctx.poisson_solve(**kw)
+        fresh = _context(case, 4)
+        want = fresh.poisson_solve(**kw)
+        assert (st.iterations, st.converged) == (want.iterations, want.converged)
+        assert st.converged == (max_iter > 3)
+        np.testing.assert_array_equal(ctx.get_field(vfs.PHI), fresh.get_field(vfs.PHI))
+        fresh.close()
+    ctx.close()

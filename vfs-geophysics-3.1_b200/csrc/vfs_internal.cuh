@@ -137,9 +137,10 @@ struct MGLevel {
 };
 
 // A Poisson solve captured as a graph (a solve outside a captured step): what its kernels'
-// arguments depend on, and the graph from the second such solve on.
+// arguments depend on, and the graph from the second such solve on.  The targets (tolerances and
+// iteration cap) are not part of it: a replay reads them from KryDev::want.
 struct SolveKey {
-  vfs_solve_opts o;
+  vfs_solve_opts o;  // targets and zero_guess zero (warm says how the solve starts)
   int warm, transpose, nslot, reserved;
   long long alloc_epoch;
   const void *x, *b, *red;
@@ -174,6 +175,7 @@ struct Poisson {
   float *w32 = nullptr;     // w of precision 2
   bool transpose = false;   // apply A^T (the adjoint solve)
   bool guess = false;       // VFS_PHI holds the last solution for the current unknowns
+  double want[3] = {-1, -1, -1};  // the targets last put into KryDev::want
 };
 // Distance between the vectors of a set (16-byte pair loads need it even).
 __host__ __device__ inline long long vec_ld(long long n) { return (n + 31) / 32 * 32; }
@@ -220,6 +222,10 @@ enum DScal {
 // matrix, the Givens rotations and the loop control, so that the solve's kernels decide
 // on the device (and a captured graph can loop on conditional nodes).
 constexpr int kKryMax = 31;
+struct SolveTargets {
+  double rtol, atol;
+  int maxit;
+};
 struct KryDev {
   int j, it, jdone, reorth, degen, inner_go, outer_go, conv, fresh, check, maxit, m, cycles;
   unsigned ticket;  // blocks of the running reduction that have stored their partial sums
@@ -227,6 +233,7 @@ struct KryDev {
   double inner_rtol, beta;  // precision 2: a cycle ends once its estimate is below inner_rtol * beta
   double h[kKryMax + 3], h2[kKryMax + 3], h3[kKryMax + 3];
   double H[(kKryMax + 1) * kKryMax], cs[kKryMax], sn[kKryMax], gv[kKryMax + 1], y[kKryMax];
+  SolveTargets want;  // of the next replayed solve graph
 };
 
 // A step captured as one CUDA graph (vfs_solve_opts.graph), with the options it was

@@ -1037,9 +1037,14 @@ __global__ void k_shift_mean(long long n, const uint8_t *fluid, const double *__
 }
 
 // ---- control kernels (one thread)
-// After the initial residual (kd->rr) and, with a starting guess, <b, b> (kd->bb).
-__global__ void k_kry_init(KryDev *kd, double rtol, double atol, int warm, int maxit, int m, unsigned long long h_outer,
+__global__ void k_kry_targets(KryDev *kd, SolveTargets t) { kd->want = t; }
+// After the initial residual (kd->rr) and, with a starting guess, <b, b> (kd->bb).  use_want: the
+// targets are kd->want instead of t.
+__global__ void k_kry_init(KryDev *kd, SolveTargets t, int use_want, int warm, int m, unsigned long long h_outer,
                            int use_graph, double inner_rtol) {
+  if (use_want) t = kd->want;
+  const double rtol = t.rtol, atol = t.atol;
+  const int maxit = t.maxit;
   kd->inner_rtol = inner_rtol;
   kd->rnorm = sqrt(kd->rr);
   kd->bnorm = warm ? sqrt(kd->bb) : kd->rnorm;
@@ -1336,8 +1341,10 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   return VFS_OK;
 }
 
-// The kernels of a solve: launched one by one, the host driving the two loops, or captured.
-static int solve_kernels(Ctx *c, const vfs_solve_opts &o, bool warm, long long *body_launches, long long *cycle_launches) {
+// The kernels of a solve: launched one by one, the host driving the two loops, or captured
+// (use_want: with the targets of each replay in kd->want).
+static int solve_kernels(Ctx *c, const vfs_solve_opts &o, bool warm, bool use_want, long long *body_launches,
+                         long long *cycle_launches) {
   Poisson &P = c->ps;
   const long long N = c->g.N;
   int rc;
@@ -1357,8 +1364,8 @@ static int solve_kernels(Ctx *c, const vfs_solve_opts &o, bool warm, long long *
   const int use_graph = c->capturing ? 1 : 0;
   cudaGraphConditionalHandle h_outer = 0, h_inner = 0;
   if (use_graph && (rc = cond_handle(c, &h_outer))) return rc;
-  c->launches++, k_kry_init<<<1, 1, 0, c->stream>>>(kd, o.rtol, o.atol, warm ? 1 : 0, o.max_iter, m,
-                                                     (unsigned long long)h_outer, use_graph,
+  c->launches++, k_kry_init<<<1, 1, 0, c->stream>>>(kd, SolveTargets{o.rtol, o.atol, o.max_iter}, use_want ? 1 : 0,
+                                                     warm ? 1 : 0, m, (unsigned long long)h_outer, use_graph,
                                                      o.precision == 2 ? kInnerRtol : 0.0);
   if ((rc = check_launch(c, "k_kry_init"))) return rc;
   if (use_graph) {
@@ -1424,6 +1431,8 @@ static SolveGraph *solve_graph(Ctx *c, const vfs_solve_opts &o, bool warm) {
   SolveKey key;
   memset(&key, 0, sizeof(key));
   key.o = o;
+  key.o.rtol = key.o.atol = 0;
+  key.o.max_iter = key.o.zero_guess = 0;
   key.warm = warm;
   key.transpose = P.transpose;
   key.nslot = P.nslot;
@@ -1455,7 +1464,7 @@ static SolveGraph *solve_graph(Ctx *c, const vfs_solve_opts &o, bool warm) {
   }
   c->capturing = true;
   const cudaStream_t own = c->stream;
-  const int rc = solve_kernels(c, o, warm, &G.body_launches, &G.cycle_launches);
+  const int rc = solve_kernels(c, o, warm, true, &G.body_launches, &G.cycle_launches);
   c->capturing = false;
   c->stream = own;
   for (cudaStream_t q : c->cap_streams) {  // a loop body left open by an error
@@ -1485,17 +1494,23 @@ int poisson_solve(Ctx *c, const vfs_solve_opts *oin, vfs_solve_stats *st) {
   if ((rc = ensure_red(c, 34 * kKryBlocks + (int)nblocks(c->g.N, 256) + 64))) return rc;
   const bool warm = P.guess && !o.zero_guess && !P.transpose;
   if (c->capturing) {  // inside a captured step: statistics after the replay
-    rc = solve_kernels(c, o, warm, &c->sg.body_launches, &c->sg.cycle_launches);
+    rc = solve_kernels(c, o, warm, false, &c->sg.body_launches, &c->sg.cycle_launches);
     if (!rc && !P.transpose) P.guess = true;
     return rc;
   }
+  cudaEventRecord(c->ev0, c->stream);  // st->ms has the time of a capture in it
   SolveGraph *G = solve_graph(c, o, warm);
-  cudaEventRecord(c->ev0, c->stream);
   if (G) {
+    const double want[3] = {o.rtol, o.atol, (double)o.max_iter};
+    if (memcmp(P.want, want, sizeof(want))) {
+      c->launches++, k_kry_targets<<<1, 1, 0, c->stream>>>(kd, SolveTargets{o.rtol, o.atol, o.max_iter});
+      if ((rc = check_launch(c, "k_kry_targets"))) return rc;
+      memcpy(P.want, want, sizeof(want));
+    }
     if (cudaGraphLaunch(G->exec, c->stream) != cudaSuccess) return set_err(c, VFS_ERR_CUDA, "poisson_solve: graph launch failed");
   } else {
     long long bl, cl;
-    if ((rc = solve_kernels(c, o, warm, &bl, &cl))) return rc;
+    if ((rc = solve_kernels(c, o, warm, false, &bl, &cl))) return rc;
   }
   if (!P.transpose) P.guess = true;
   cudaEventRecord(c->ev1, c->stream);
