@@ -32,7 +32,8 @@ def fake(fake_library):
     lib = vfs.load_library(fake_library)
     lib.fake_fail_kernel.argtypes = [ctypes.c_char_p]
     lib.fake_launches.argtypes = [ctypes.c_char_p]
-    for f in ("launches", "mallocs", "cleared_bytes", "captures", "graph_launches"):
+    lib.fake_limit.argtypes = [ctypes.c_long]
+    for f in ("launches", "mallocs", "allocated", "cleared_bytes", "captures", "graph_launches"):
         getattr(lib, "fake_" + f).restype = ctypes.c_long
     lib.fake_reset()
     yield lib

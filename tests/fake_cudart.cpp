@@ -13,7 +13,8 @@ static std::map<const void *, std::string> &names() {
   return n;
 }
 static cudaError_t last_error = cudaSuccess;
-static long fail_malloc = 0, fail_sync = 0, n_malloc = 0, n_clear_bytes = 0;
+static long fail_malloc = 0, n_malloc = 0, n_clear_bytes = 0, n_bytes = 0, max_bytes = 0;
+static std::map<void *, size_t> sizes;
 static std::string fail_kernel;
 static std::map<std::string, long> launched;
 static long n_captures = 0, n_graph_launches = 0;
@@ -27,12 +28,14 @@ static cudaError_t done(cudaError_t e) {
 extern "C" {
 // ---- control of the tests
 void fake_reset() {
-  fail_malloc = fail_sync = n_malloc = n_clear_bytes = n_captures = n_graph_launches = 0;
+  fail_malloc = max_bytes = n_malloc = n_clear_bytes = n_captures = n_graph_launches = 0;
   fail_kernel.clear();
   launched.clear();
   last_error = cudaSuccess;
 }
 void fake_fail_malloc(long nth) { fail_malloc = nth; }  // the nth allocation from now on and all after it (0: none)
+void fake_limit(long bytes) { max_bytes = bytes; }  // allocations past this total fail (0: none)
+long fake_allocated() { return n_bytes; }
 void fake_fail_kernel(const char *name) { fail_kernel = name; }
 long fake_launches(const char *name) {
   long n = 0;
@@ -49,12 +52,20 @@ cudaError_t cudaMalloc(void **p, size_t n) {
   n_malloc++;
   *p = nullptr;
   if (fail_malloc && --fail_malloc <= 0) { fail_malloc = 1; return done(cudaErrorMemoryAllocation); }
+  if (max_bytes && n_bytes + (long)n > max_bytes) return done(cudaErrorMemoryAllocation);
   *p = calloc(n ? n : 1, 1);
+  sizes[*p] = n;
+  n_bytes += (long)n;
   return cudaSuccess;
 }
 cudaError_t cudaMallocAsync(void **p, size_t n, cudaStream_t) { return cudaMalloc(p, n); }
-cudaError_t cudaFree(void *p) { free(p); return cudaSuccess; }
-cudaError_t cudaFreeAsync(void *p, cudaStream_t) { free(p); return cudaSuccess; }
+cudaError_t cudaFree(void *p) {
+  auto it = sizes.find(p);
+  if (it != sizes.end()) { n_bytes -= (long)it->second; sizes.erase(it); }
+  free(p);
+  return cudaSuccess;
+}
+cudaError_t cudaFreeAsync(void *p, cudaStream_t) { return cudaFree(p); }
 cudaError_t cudaHostAlloc(void **p, size_t n, unsigned) { *p = calloc(n, 1); return cudaSuccess; }
 cudaError_t cudaMallocHost(void **p, size_t n) { *p = calloc(n, 1); return cudaSuccess; }
 cudaError_t cudaFreeHost(void *p) { free(p); return cudaSuccess; }

@@ -139,3 +139,25 @@ def test_solves_that_differ_in_their_targets_share_a_graph(fake):
     ctx.poisson_solve(rtol=1e-8, max_iter=100, pre_smooth=2, **kw)
     assert (fake.fake_captures(), fake.fake_graph_launches()) == (2, 12)
     ctx.close()
+
+
+def test_precisions_in_turn_where_memory_holds_one(fake):
+    """The vectors of another precision are given back when a solve's own do not fit: a context that
+    alternates between the precisions needs no more memory than its largest."""
+    need = {}
+    for precision in (0, 1, 2):
+        ctx = context()
+        ctx.poisson_rhs()
+        ctx.poisson_solve(precision=precision, allow_unconverged=True)
+        need[precision] = fake.fake_allocated()
+        ctx.close()
+    ctx = context()
+    ctx.poisson_rhs()
+    fake.fake_limit(need[1])
+    for precision in (0, 1, 2, 1, 0, 2, 0):
+        ctx.poisson_solve(precision=precision, allow_unconverged=True)
+        assert fake.fake_allocated() <= need[1]
+    n0 = fake.fake_mallocs()
+    ctx.poisson_solve(precision=0, allow_unconverged=True)  # nothing is given back while it fits
+    assert fake.fake_mallocs() == n0
+    ctx.close()

@@ -1319,6 +1319,26 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   P.alloc_epoch++;
   P.ldv = ldv;
   bool ok = true;
+  // memory, from the vectors that only other precisions use if there is none left
+  auto alloc = [&](void **v, size_t bytes) {
+    if (cudaMalloc(v, bytes) == cudaSuccess) return true;
+    auto drop = [](auto *&u, int &have) {
+      cudaFree(u);
+      u = nullptr;
+      have = 0;
+    };
+    if (f64) {
+      drop(P.V32, P.restart32);
+      cudaFree(P.w32);
+      P.w32 = nullptr;
+    } else {
+      drop(P.V, P.restart);
+    }
+    if (z64) drop(P.Z32, P.restart_z32);
+    else drop(P.Z64, P.restart_z64);
+    cudaGetLastError();
+    return cudaMalloc(v, bytes) == cudaSuccess;
+  };
   // the ghost points of the preconditioned vectors are never written: zero from the start (the
   // basis vectors are written whole before they are read)
   auto grow = [&](auto **v, int &have, bool basis) {
@@ -1327,7 +1347,7 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
     cudaFree(*v);
     *v = nullptr;
     have = 0;
-    ok = cudaMalloc(v, bytes) == cudaSuccess;
+    ok = alloc((void **)v, bytes);
     if (!ok) return;
     if (!basis) cudaMemsetAsync(*v, 0, bytes, c->stream);
     have = m;
@@ -1336,7 +1356,7 @@ int poisson_prepare(Ctx *c, const vfs_solve_opts *oin) {
   else grow(&P.V32, P.restart32, true);
   if (z64) grow(&P.Z64, P.restart_z64, false);
   else grow(&P.Z32, P.restart_z32, false);
-  if (!f64 && ok && !P.w32) ok = cudaMalloc(&P.w32, sizeof(float) * (size_t)ldv) == cudaSuccess;
+  if (!f64 && ok && !P.w32) ok = alloc((void **)&P.w32, sizeof(float) * (size_t)ldv);
   if (!ok) return set_err(c, VFS_ERR_CUDA, "poisson_solve: Krylov basis allocation failed");
   return VFS_OK;
 }
