@@ -46,7 +46,7 @@ METRIC = "ms/step @256x192x256: mixed vs FP64 GPU at max|div u|<=1e-8; adjoint/f
 # The mixed form of the metric: precision 0 (the V-cycle in FP32 inside FP64 FGMRES).  The
 # other mixed form, precision 2 (the FGMRES basis, preconditioned vectors and V-cycle in
 # FP32, every restart cycle an FP64 iterative-refinement sweep), is timed beside it; on this
-# workload it takes about one FGMRES iteration more per step and is slower.
+# workload it takes up to one FGMRES iteration more per step.
 MIXED = 0
 ALT = 2
 NX, NY, NZ = 256, 192, 256
@@ -216,9 +216,9 @@ def timed(ctx, fn, reps, torch):
 # input read once, each output written once, at the stored precision, nvert as 1 byte).
 # DRAM bytes (read + write) per launch of the profiled kernels from one ncu capture at
 # 128x96x128 cells, scaled by the cell ratio (x8) to 256x192x256 (profiles/
-# formfunction2_128x96x128.md): Formfunction_2 as the step runs it (k_face_flux, k_fp,
-# k_rhs) moved 1285.6 MB per launch there.
-KERNEL_TRAFFIC = {"formfunction2": 1285.6e6 * 8}
+# formfunction2_128x96x128.md): Formfunction_2 as the step runs it (k_face_flux_listed,
+# k_face_flux, k_fp, k_rhs) moved 1366.0 MB per launch there.
+KERNEL_TRAFFIC = {"formfunction2": 1366.0e6 * 8}
 
 KERNEL_BYTES = {
     # Formfunction_2 accumulating into Rhs (Formfunction_2(user, Rhs, scale) adds), les = 0
@@ -501,9 +501,9 @@ def adjoint_window(nx, ny, nz, steps, every, torch):
     for _ in range(2):  # warm-up: tapes, checkpoints, Krylov space, clocks
         ctx.adjoint_gradient(steps, checkpoint_every=every, **kw)
     torch.cuda.synchronize()
-    # the launched steps of both sweeps read the solver's loop flags and the adjoint's global
-    # sums back on the host, so a busy host stretches their event times: five windows, the
-    # median ratio, the smallest beside it
+    # the launched steps of both sweeps and the adjoint's global sums, which are read back on the
+    # host, let a busy host stretch their event times: five windows, the median ratio, the
+    # smallest beside it
     sampler = ClockSampler(torch.cuda.current_device())
     with sampler:
         runs = [ctx.adjoint_gradient(steps, checkpoint_every=every, **kw) for _ in range(5)]
@@ -652,7 +652,7 @@ def large_window(torch, nx=384, ny=256, nz=384, steps=50, every=7):
 # ncu (2 x DFMA + DMUL + DADD, executed thread instructions, every kernel of the call; the
 # division and square-root sequences count by their instructions):
 # profiles/les_dynamic_smagorinsky_128x96x128.md.
-LES_FLOPS_PER_CELL = 5373
+LES_FLOPS_PER_CELL = 1548
 FP64_PEAK_TFLOPS = 37.0   # nominal B200 FP64 (vector), no measured figure in MEASURED_PEAKS.json
 
 
@@ -824,7 +824,9 @@ def main():
         ctx.step(precision=MIXED, rtol=1e-10)   # the mixed form's workspace
         torch.cuda.synchronize()
         torch.cuda.profiler.start()
-        ctx.step(precision=MIXED, rtol=1e-10)
+        # a solve whose form differs from those before it is launched kernel by kernel, not replayed as
+        # a graph, so that every kernel is listed (a shorter basis changes nothing in these solves)
+        ctx.step(precision=MIXED, rtol=1e-10, restart=29)
         ctx.synchronize()
         torch.cuda.profiler.stop()
         ctx.close()
@@ -1017,7 +1019,8 @@ def main():
             "fp64_ms_per_step": round(ms_fp64, 3),
             "launched_ms_per_step": round(ms_launched, 3),
             "step_form": "one CUDA graph per step (captured once, replayed; the Poisson solve's loops as "
-                         "conditional nodes); launched_ms_per_step: the same kernels launched one by one",
+                         "conditional nodes); launched_ms_per_step: the same kernels launched one by one, the "
+                         "Poisson solve as a graph of its own",
             "mixed_speedup_vs_fp64": round(ms_fp64 / ms_mixed, 3),
             "fp32_krylov_form": {"ms_per_step": round(ms_alt, 3), "speedup_vs_fp64": round(ms_fp64 / ms_alt, 3),
                                  "poisson_iterations": its_alt, "max_div": maxdiv_alt,

@@ -134,7 +134,8 @@ typedef struct {
   int graph;         /* vfs_step only: 1 runs the step as one CUDA graph, captured on the
                         first such step (and again after a set-up change) and replayed: the
                         Poisson solve's loops are conditional nodes and no kernel waits for
-                        the host.  Same kernels, same results as 0 (launched one by one).
+                        the host.  Same kernels, same results as 0 (launched one by one, the
+                        Poisson solve as a graph of its own from its second occurrence).
                         Steps with set-up work (the first step, a new operator, moving
                         bodies, the first two LES steps of a fresh run, a recorded tape)
                         and implicit momentum steps run launched one by one. */
@@ -148,7 +149,8 @@ typedef struct {
   int iterations;       /* outer FGMRES iterations taken */
   int converged;        /* 1 if rtol/atol met */
   double r0, rfinal;    /* initial / final residual 2-norms */
-  double ms;            /* device time of the solve */
+  double ms;            /* device time of the solve (with the recording of its graph, where
+                           the call made one) */
   double reserved[4];
 } vfs_solve_stats;
 

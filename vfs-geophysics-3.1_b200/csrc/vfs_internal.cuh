@@ -128,7 +128,7 @@ struct MGLevel {
   ZL z;
   bool zebra = true;        // two-colour line Gauss-Seidel is race-free on this level
   double *op64 = nullptr;   // 6n: couplings +i, +j, +k, diagonal, Thomas factors cpr, 1/pivot
-  double *pk64 = nullptr;   // 6n: packed operator (a 4-vector and a 2-vector per cell), FP64
+  double *pk64 = nullptr;   // 8n: packed operator (a 4-vector, a 2-vector, cpr and the diagonal per cell), FP64
   float *pk32 = nullptr;    // the same in FP32
   uint8_t *act = nullptr;   // n: 1 for an active unknown (non-zero diagonal)
   unsigned long long *pmask = nullptr;  // n: per cell of a coarse level, active neighbours and children

@@ -179,8 +179,8 @@ static int les_ghosts(Ctx *c, const LesArrays &o) {
 struct LesPrep {
   double *U, *V, *W;   // contravariant centre velocity (own point)
   double *wgt;         // 0 where nvert > 1.1, else 1/aj (own point)
-  double *ss[6];       // S_ab*|S| at the periodic image, zero at solid/boundary images
-  double *uf[3];       // test-filtered velocity at the periodic image
+  double *ss[6];       // S_ab*|S| of the interior cells (zero at solid ones); ghosts by k_les_ghosts
+  double *uf[3];       // test-filtered velocity, the same way
 };
 
 // ------------------------------------------------------------------ k_les_prep

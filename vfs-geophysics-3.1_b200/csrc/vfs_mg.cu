@@ -824,8 +824,7 @@ __global__ void __launch_bounds__(128) k_zprolong(ZL F, ZL C, const unsigned lon
 // The same prolongation, one colour-1 fine cell per thread: eight coarse values in flight instead
 // of 27 and four times the threads.  The coarse-centric form loads less, this one waits less:
 // it serves the levels too small to fill the GPU (kFineProlong: up to 64^3 cells; a whole step of
-// 12 x 10 x 14 cells 668 -> 606 us, of 64^3 1572 -> 1528, while at 256 x 192 x 256 it costs a
-// V-cycle 35 us).
+// 64^3 cells 1572 -> 1528 us, while on every level of 256 x 192 x 256 it costs a V-cycle 35 us).
 template <typename T>
 __global__ void __launch_bounds__(128) k_zprolong_fine(ZL F, ZL C, const unsigned long long *__restrict__ mask, T *x,
                                                        const T *xc) {

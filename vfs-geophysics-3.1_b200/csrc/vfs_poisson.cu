@@ -241,9 +241,9 @@ __device__ __forceinline__ int nb_off(const NbOff &o, int t) {
 // (A x)[p] on the grid layout from the first NS stencil slots: NS = 7 when every cross
 // slot of the operator is zero (orthogonal grids), else 19.  A skipped slot is zero, so
 // both forms give the same sums.  Rows of non-unknowns are all zero.
-// Every load is issued before the first coefficient is tested (testing first made each x load
-// wait for its coefficient: 237 us an apply at 256 x 192 x 256); an x under a zero coefficient
-// is loaded and left out.
+// Every load is issued before the first coefficient is tested; an x under a zero coefficient is
+// loaded and left out.  (With neighbour indices formed per slot and the test first, each x load
+// waiting for its coefficient, an apply of 7 slots at 256 x 192 x 256 took 195 us; now 129.)
 template <int NS, typename XT>
 __device__ __forceinline__ double apply_row64(const Grid &g, const double *__restrict__ coef,
                                               const XT *__restrict__ x, long long p) {
@@ -639,9 +639,10 @@ __global__ void __launch_bounds__(256) k_guess(long long n, const uint8_t *__res
 
 // ------------------------------------------------------------------ device-driven FGMRES
 // The same FGMRES as a sequence of kernels that read the iteration state from the device
-// (KryDev): the Gram-Schmidt decisions, the Hessenberg matrix, the Givens rotations and the
-// convergence tests run in one-thread kernels, and every kernel that depends on a
-// decision reads its flag (Guard) and returns at once when it does not apply.  Launched
+// (KryDev): the Gram-Schmidt decisions, the Hessenberg matrix and the Givens rotations are formed
+// by the last block of the basis passes, the start and the end of a restart cycle by one-block
+// kernels, and every kernel that depends on a decision reads its flag (Guard) and returns at once
+// when it does not apply.  Launched
 // from a host loop that reads the two loop flags, or captured into a graph whose two
 // loops are conditional WHILE nodes that the control kernels set, with the same kernels
 // and therefore the same results.
@@ -779,7 +780,8 @@ __device__ __forceinline__ void kry_givens(KryDev *kd, unsigned long long h_inne
 // w = A z_j.  The rows are FP64 sums of FP64 coefficients whatever the vectors' types (precision
 // 2: FP32 coefficients measured 20-40 % more iterations, since iterative refinement converges
 // at the rate of the inner operator's error), rounded to w's type.  Blocks of 64 threads without a
-// register cap: 19 slots at 192 x 128 x 192 215 us against 255 in blocks of 256.
+// register cap: a block's registers are free again as soon as its two warps end (19 slots at
+// 192 x 128 x 192 150 us, 258 in blocks of 256 with the neighbours' indices).
 constexpr int kApplyThreads = 64;
 template <int NS, bool kT, typename B, typename ZT>
 __global__ void __launch_bounds__(kApplyThreads) k_apply_dyn(Grid g, long long ldv, const double *__restrict__ coef,
