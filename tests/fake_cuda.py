@@ -41,8 +41,9 @@ def fake(fake_library):
     vfs._lib = own
 
 
-def context(nx=16, ny=16, nz=16):
+def context(nx=16, ny=16, nz=16, immersed=0):
     case = cases.channel(nx, ny, nz)
+    case.immersed = immersed
     ctx = vfs.Context(case.config())
     ctx.form_metrics(case.X, case.Y, case.Z)
     ctx.set_field(vfs.NVERT, case.nvert)

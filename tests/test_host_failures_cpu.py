@@ -4,6 +4,7 @@ forgets to allocate it."""
 import pytest
 
 import vfs_b200 as vfs
+from vfs_b200 import cases
 from fake_cuda import context, fake, fake_library  # noqa: F401
 
 ERR_CUDA = 2
@@ -160,4 +161,27 @@ def test_precisions_in_turn_where_memory_holds_one(fake):
     n0 = fake.fake_mallocs()
     ctx.poisson_solve(precision=0, allow_unconverged=True)  # nothing is given back while it fits
     assert fake.fake_mallocs() == n0
+    ctx.close()
+
+
+@pytest.mark.parametrize("nth", [2, 3, 4, 5])
+def test_point_lists_after_a_search_that_failed_half_way(fake, nth):
+    """The ray casting has written nvert by then: the lists of boundary and body points that
+    Contra2Cart and the face fluxes run over, and the Poisson operator, are not those any more."""
+    ctx = context(immersed=1)
+    ctx.poisson_lhs()
+    ctx.contra2cart()
+    ctx.formfunction2(1.0)
+    lists, operators = (fake.fake_launches(k) for k in (b"k_collect_points", b"k_poisson_coef"))
+    ctx.formfunction2(1.0)
+    assert fake.fake_launches(b"k_collect_points") == lists
+    fake.fake_fail_malloc(nth)
+    with pytest.raises(vfs.VfsError):
+        ctx.ibm_search(*cases.icosphere((1.5, 1.0, 3.0), 0.4, 1))
+    fake.fake_fail_malloc(0)
+    assert fake.fake_launches(b"k_ibm_cast") == 1
+    ctx.formfunction2(1.0)
+    assert fake.fake_launches(b"k_collect_points") > lists
+    ctx.poisson_rhs()
+    assert fake.fake_launches(b"k_poisson_coef") > operators
     ctx.close()

@@ -549,6 +549,10 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
   S.xmin = xmin; S.xmax = xmax; S.ymin = ymin; S.ymax = ymax; S.zmin = zmin; S.zmax = zmax;
   S.dcx = dcx; S.dcy = dcy; S.dcz = dcz;
   int rc;
+  // from here on nvert is another field, also when the search fails
+  c->nsolid = -1;
+  c->ps.built = false;
+  c->setup_epoch++;
   c->launches++, k_ibm_cast<<<nblocks(g.N, 128), 128, 0, c->stream>>>(g, S, cv(field3(c, VFS_CENT)), c->nv, ibi == 0 ? 1 : 0, err);
   if ((rc = check_launch(c, "k_ibm_cast"))) { cudaFree(buf); return rc; }
   c->launches++, k_ibm_near<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, c->nv, c->bcflag);
@@ -652,9 +656,6 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
   if (herr == -1) return set_err(c, VFS_ERR_INVALID, "vfs_ibm_search: a cell's rays kept hitting coincident crossings");
   if (herr == -2) return set_err(c, VFS_ERR_INVALID, "vfs_ibm_search: a ray crossed too many triangles");
   c->nvert_set = true;
-  c->nsolid = -1;
-  c->ps.built = false;
-  c->setup_epoch++;
   return VFS_OK;
 }
 
