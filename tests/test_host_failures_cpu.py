@@ -185,3 +185,18 @@ def test_point_lists_after_a_search_that_failed_half_way(fake, nth):
     ctx.poisson_rhs()
     assert fake.fake_launches(b"k_poisson_coef") > operators
     ctx.close()
+
+
+@pytest.mark.parametrize("nth", [2, 3, 4, 5])
+def test_marks_after_a_search_that_failed_half_way(fake, nth):
+    """The search marks cells in Contra2Cart's flag buffer: cleared again on every way out."""
+    ctx = context(immersed=1)
+    surface = cases.icosphere((1.5, 1.0, 3.0), 0.4, 1)
+    ctx.ibm_search(*surface)
+    n = ctx.shape[0] * ctx.shape[1] * ctx.shape[2]
+    fake.fake_fail_malloc(nth)
+    n0 = fake.fake_cleared_bytes()
+    with pytest.raises(vfs.VfsError):
+        ctx.ibm_search(*surface)
+    assert fake.fake_cleared_bytes() - n0 >= n
+    ctx.close()

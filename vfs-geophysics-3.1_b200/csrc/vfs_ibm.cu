@@ -553,13 +553,19 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
   c->nsolid = -1;
   c->ps.built = false;
   c->setup_epoch++;
+  // every way out clears the marks in Contra2Cart's flag buffer again
+  auto leave = [&](int code) {
+    cudaMemsetAsync(c->bcflag, 0, (size_t)g.N, c->stream);
+    cudaFree(buf);
+    return code;
+  };
   c->launches++, k_ibm_cast<<<nblocks(g.N, 128), 128, 0, c->stream>>>(g, S, cv(field3(c, VFS_CENT)), c->nv, ibi == 0 ? 1 : 0, err);
-  if ((rc = check_launch(c, "k_ibm_cast"))) { cudaFree(buf); return rc; }
+  if ((rc = check_launch(c, "k_ibm_cast"))) return leave(rc);
   c->launches++, k_ibm_near<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, c->nv, c->bcflag);
-  if ((rc = check_launch(c, "k_ibm_near"))) { cudaFree(buf); return rc; }
+  if ((rc = check_launch(c, "k_ibm_near"))) return leave(rc);
   if (c->nvo && ibi == (int)c->scal[VFS_S_NBODIES] - 1) {
     c->launches++, k_ibm_phase<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, c->nvo, c->bcflag);
-    if ((rc = check_launch(c, "k_ibm_phase"))) { cudaFree(buf); return rc; }
+    if ((rc = check_launch(c, "k_ibm_phase"))) return leave(rc);
   }
   // the IB-node list of this body (ibm.c:347-505): cells marked 2, ascending
   {
@@ -568,14 +574,13 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
     const int cap = 1 << 22;
     long long *cells = nullptr;
     if (cudaMallocAsync((void **)&cells, sizeof(long long) * cap, c->stream) != cudaSuccess) {
-      cudaFree(buf);
-      return set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed");
+      return leave(set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed"));
     }
     c->launches++, k_ibm_collect<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, c->bcflag, cells, cnt, cap);
     int hn = 0;
     cudaMemcpyAsync(&hn, cnt, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
     cudaStreamSynchronize(c->stream);
-    if (hn > cap) { cudaFreeAsync(cells, c->stream); cudaFree(buf); return set_err(c, VFS_ERR_INVALID, "vfs_ibm_search: too many IB nodes"); }
+    if (hn > cap) { cudaFreeAsync(cells, c->stream); return leave(set_err(c, VFS_ERR_INVALID, "vfs_ibm_search: too many IB nodes")); }
     std::vector<long long> hc(hn);
     if (hn) cudaMemcpy(hc.data(), cells, sizeof(long long) * hn, cudaMemcpyDeviceToHost);
     std::sort(hc.begin(), hc.end());
@@ -587,7 +592,7 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
     const int base = (ibi == 0) ? 0 : c->nib;
     bool ok = cudaMalloc(&qd, sizeof(double) * 4 * (size_t)n_elmt) == cudaSuccess;
     ok = ok && cudaMalloc(&nodes, sizeof(IbNode) * (size_t)(base + hn + 1)) == cudaSuccess;
-    if (!ok) { cudaFree(qd); cudaFree(nodes); cudaFreeAsync(cells, c->stream); cudaFree(buf); return set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed"); }
+    if (!ok) { cudaFree(qd); cudaFree(nodes); cudaFreeAsync(cells, c->stream); return leave(set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed")); }
     cudaMemcpyAsync(qd, qx.data(), sizeof(double) * n_elmt, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(qd + n_elmt, qy.data(), sizeof(double) * n_elmt, cudaMemcpyHostToDevice, c->stream);
     cudaMemcpyAsync(qd + 2 * (size_t)n_elmt, qz.data(), sizeof(double) * n_elmt, cudaMemcpyHostToDevice, c->stream);
@@ -609,8 +614,8 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
       double *nvb = nullptr;
       const int ntot = c->nvtx + n_v;
       if (cudaMalloc(&nvb, sizeof(double) * 3 * (size_t)ntot) != cudaSuccess) {
-        cudaFree(qd); cudaFree(nodes); cudaFreeAsync(cells, c->stream); cudaFree(buf);
-        return set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed");
+        cudaFree(qd); cudaFree(nodes); cudaFreeAsync(cells, c->stream);
+        return leave(set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed"));
       }
       cudaMemsetAsync(nvb, 0, sizeof(double) * 3 * (size_t)ntot, c->stream);
       if (c->ibv && c->nvtx)
@@ -623,7 +628,7 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
       c->nvtx = ntot;
     }
     if (hn) c->launches++, k_ibm_nodes<<<nblocks(hn, 64), 64, 0, c->stream>>>(g, G, nodes + base, err);
-    if ((rc = check_launch(c, "k_ibm_nodes"))) { cudaFree(qd); cudaFree(nodes); cudaFree(buf); return rc; }
+    if ((rc = check_launch(c, "k_ibm_nodes"))) { cudaFree(qd); cudaFree(nodes); cudaFreeAsync(cells, c->stream); return leave(rc); }
     cudaFreeAsync(cells, c->stream);
     cudaStreamSynchronize(c->stream);
     cudaFree(qd);
@@ -634,8 +639,8 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
     if (ibi == 0) c->nib_body0 = hn;
     c->ibbuf = nullptr;
     if (c->nib && cudaMalloc(&c->ibbuf, sizeof(double) * kIbOut * (size_t)c->nib) != cudaSuccess) {
-      cudaFree(buf);
-      return set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed");
+      c->nib = 0;  // no nodes without their buffer
+      return leave(set_err(c, VFS_ERR_CUDA, "vfs_ibm_search: allocation failed"));
     }
     std::vector<IbNode> hnodes(hn);
     if (hn) cudaMemcpy(hnodes.data(), nodes + base, sizeof(IbNode) * hn, cudaMemcpyDeviceToHost);
@@ -643,7 +648,7 @@ int ibm_search(Ctx *c, int ibi, int n_v, const double *x, const double *y, const
     for (const IbNode &nd : hnodes) c->nib_unresolved += nd.imode == -2;
   }
   c->launches++, k_ibm_remap<<<nblocks(g.N, 256), 256, 0, c->stream>>>(g, c->bcflag, c->nv, c->f[VFS_NVERT][0]);
-  if ((rc = check_launch(c, "k_ibm_remap"))) { cudaFree(buf); return rc; }
+  if ((rc = check_launch(c, "k_ibm_remap"))) return leave(rc);
   cudaMemsetAsync(c->bcflag, 0, (size_t)g.N, c->stream);  // Contra2Cart's flag buffer, clear again
   int herr = 0;
   cudaMemcpyAsync(&herr, err, sizeof(int), cudaMemcpyDeviceToHost, c->stream);
